@@ -35,7 +35,7 @@ NVCCFLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xco
 HOST_SOURCES = ["host/settings.cpp", "host/vtk_io.cpp", "host/mesh_setup.cpp", "host/host_capi.cpp"]
 CUDA_SOURCES = ["cuda/kernels.cu", "cuda/cluster.cu", "cuda/capi.cu", "cuda/noalloc.cu", "cuda/batch.cu",
                 "cuda/learned.cu", "cuda/tri_tiles.cu", "cuda/node_tiles.cu", "cuda/node_tile_plan.cu",
-                "cuda/node_pipe.cu", "cuda/setup.cu"]
+                "cuda/node_pipe.cu", "cuda/resident.cu", "cuda/setup.cu"]
 # Per-file nvcc flags: the device set-up rounds every operation as the host
 # set-up does (no contraction into fused multiply-adds).
 CUDA_FILE_FLAGS = {"cuda/setup.cu": ["-fmad=false"]}

@@ -94,6 +94,12 @@ struct ms_handle {
     NodeTilePlan ntp{};
     unsigned char* d_nt_rec = nullptr;
     std::vector<int> nt_chunk_tri;  // host copy of NodeTilePlan::chunk_tri
+    // resident step: many steps per launch on small meshes.  It stands in for
+    // the default path until ms_set_step_path asks for one by number.
+    bool have_resident = false;
+    bool default_path = true;
+    ResidentPlan rsp{};
+    unsigned rs_tag = 0;  // tag of the last step published
 };
 
 namespace {
@@ -383,6 +389,57 @@ ms_status build_node_tiles(ms_handle* h, const ms_mesh_desc* d, const std::vecto
     return MS_OK;
 }
 
+// Plan of the resident step, where the mesh is small enough for it.
+ms_status build_resident(ms_handle* h, const ms_mesh_desc* d, const std::vector<int>& off,
+                         const std::vector<int>& ent) {
+    int sms = 0, coop = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device);
+    ResidentLayout L;
+    if (!coop || !resident_layout(d->patch_ids, d->num_nodes, d->num_tris, sms, off, ent, L)) return MS_OK;
+    ResidentPlan q{};
+    q.nodes = L.nodes;
+    q.ntiles = L.ntiles;
+    q.halo = L.halo;
+    q.threads = L.threads;
+    q.width = L.width;
+    int blocks = 0;
+    if (prepare_resident(q, h->precision == MS_PRECISION_MIXED, &blocks) != cudaSuccess || blocks < 1) {
+        cudaGetLastError();
+        return MS_OK;  // the other paths remain
+    }
+    // One buffer: the packets (zeroed: tags start at 1), then the tables.
+    const size_t packets = 6ULL * d->num_nodes * sizeof(ulonglong2);
+    std::vector<unsigned char> blob(packets, 0);
+    auto put = [&](const auto& v) {
+        const size_t at = blob.size(), bytes = v.size() * sizeof(v[0]);
+        blob.resize(at + (bytes + 15) / 16 * 16, 0);
+        std::memcpy(blob.data() + at, v.data(), bytes);
+        return at;
+    };
+    const size_t head = put(L.head), tri = put(L.tri), halo_id = put(L.halo_id), local = put(L.local),
+                 entries = put(L.entries), border = put(L.border), count = put(L.count);
+    unsigned char* base;
+    MS_TRY(upload(h, &base, blob));
+    q.packets = reinterpret_cast<ulonglong2*>(base);
+    q.head = reinterpret_cast<const int4*>(base + head);
+    q.tri = reinterpret_cast<const int*>(base + tri);
+    q.halo_id = reinterpret_cast<const int*>(base + halo_id);
+    q.local = reinterpret_cast<const unsigned short*>(base + local);
+    q.entries = reinterpret_cast<const unsigned short*>(base + entries);
+    q.border = base + border;
+    q.count = base + count;
+    if (L.ntiles > h->s.eq_blocks) {
+        EqPartial* ep;
+        MS_TRY(dalloc(h, &ep, L.ntiles));
+        h->s.eq_part = ep;
+        h->s.eq_blocks = L.ntiles;
+    }
+    h->rsp = q;
+    h->have_resident = true;
+    return MS_OK;
+}
+
 // Tiles of cs * tpc consecutive triangles, one per thread-block cluster; a
 // node is owned by a tile when all its incidences lie in it (see
 // ClusterPlan).  Falls back to the two-kernel step when cluster launches are
@@ -475,7 +532,8 @@ ms_status build_cluster_plan(ms_handle* h, const ms_mesh_desc* d, const std::vec
     }
     h->have_plan = true;
     MS_TRY(build_tiles(h, d));
-    return build_node_tiles(h, d, off, ent);
+    MS_TRY(build_node_tiles(h, d, off, ent));
+    return build_resident(h, d, off, ent);
 }
 
 // Per-triangle director trigonometry for the cluster kernel's protocol-3
@@ -937,10 +995,9 @@ ms_status ms_advance_dynamics(ms_handle* h, double dt, double damping, int gd, i
     return MS_OK;
 }
 
-// Per-step {dial, lambda, lambda^(-2 nu)} triples for the device (the last two
-// are used when lambda_final and nu_ot are uniform; formed as do_dialling.cpp:116-118
-// forms them, in double on the host).
-static ms_status stage_dials(ms_handle* h, const double* dials, int n) {
+// Room for n per-step {dial, lambda, lambda^(-2 nu)} triples, and the last
+// ones no longer being copied.
+static ms_status room_for_dials(ms_handle* h, int n) {
     if (h->dials_cap < 3 * n) {
         if (h->d_dials) {
             cudaFree(h->d_dials);
@@ -959,15 +1016,28 @@ static ms_status stage_dials(ms_handle* h, const double* dials, int n) {
         h->h_dials_cap = cap;
     }
     MS_CUDA(h, cudaStreamSynchronize(h->stream));
-    for (int i = 0; i < n; ++i) {
+    return MS_OK;
+}
+
+// The triples of steps [i0, i1) to the device (the last two values are used
+// when lambda_final and nu_ot are uniform; formed as do_dialling.cpp:116-118
+// forms them, in double on the host).
+static ms_status fill_dials(ms_handle* h, const double* dials, int i0, int i1) {
+    for (int i = i0; i < i1; ++i) {
         const double dial = dials[i];
         const double lam = (1.0 - dial) * 1.0 + dial * h->lce_lam_final;
         h->h_dials[3 * i] = dial;
         h->h_dials[3 * i + 1] = lam;
         h->h_dials[3 * i + 2] = std::pow(lam, -2.0 * h->lce_nu);
     }
-    MS_CUDA(h, cudaMemcpyAsync(h->d_dials, h->h_dials, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    MS_CUDA(h, cudaMemcpyAsync(h->d_dials + 3 * i0, h->h_dials + 3 * i0, 3 * (i1 - i0) * sizeof(double),
+                               cudaMemcpyHostToDevice, h->stream));
     return MS_OK;
+}
+
+static ms_status stage_dials(ms_handle* h, const double* dials, int n) {
+    MS_TRY(room_for_dials(h, n));
+    return fill_dials(h, dials, 0, n);
 }
 
 static cudaError_t launch_step(ms_handle* h, const StepScalars& sc, bool cluster, int dial_mode, cudaStream_t st);
@@ -1032,6 +1102,64 @@ ms_status ms_set_step_path(ms_handle* h, int path) {
     if (path == 3 && !h->have_ntiles) return fail(h, MS_ERR_UNSUPPORTED, "node-tiled kernel unavailable");
     if (path == 4 && !h->have_pipe) return fail(h, MS_ERR_UNSUPPORTED, "warp-specialised node-tiled kernel unavailable");
     h->step_path = path;
+    h->default_path = false;
+    return MS_OK;
+}
+
+// Steps one resident launch takes at most: its time stays in the tens of
+// milliseconds, and so does the stretch that is run again after a guard trip.
+// The first launch of a dialling call is short: the later steps' dial values
+// (a pow each, ~40 ns) are formed while it runs.
+constexpr int kResidentSteps = 8192;
+constexpr int kResidentFirst = 128;
+// Fewest steps of a call worth a resident launch.
+constexpr int kResidentMin = 2;
+
+// The resident step: fused protocol-3 dialling with uniform lambda_final and
+// nu_ot, or metrics from the arrays; uniform material.
+static bool use_resident(const ms_handle* h, int n, bool dialling, bool fuse_lce) {
+    if (!h->have_resident || !h->default_path || n < kResidentMin || !h->m.uniform_hmu) return false;
+    return dialling ? fuse_lce && h->plan.tri_aux && h->plan.lce_uniform : true;
+}
+
+// Runs n steps from h->cur as resident launches and waits for them (the
+// error record is in *h->h_err then, the equilibrium record in *h->h_equil
+// with check_last).  *done receives the steps that stand: n with h->cur
+// holding their state, or, when a launch tripped the guard, the steps before
+// that launch with h->cur holding the state it started from.
+static ms_status run_resident(ms_handle* h, int n, const double* dials, int dial_mode, double dt, double damping,
+                              int gd, int check_last, int* done) {
+    cudaStream_t st = h->stream;
+    const int p0 = h->cur;
+    std::vector<int> starts;
+    for (int at = 0, k = 0; at < n; ++k) {
+        int len = std::min(dials && k == 0 ? kResidentFirst : kResidentSteps, n - at);
+        if (n - at - len < kResidentFirst) len = n - at;
+        if (dials) MS_TRY(fill_dials(h, dials, at, at + len));
+        starts.push_back(at);
+        const bool last = at + len == n;
+        StepScalars sc{at, p0 ^ (k & 1), dt, damping, h->rho_hh, h->force_limit, gd, check_last && last ? 1 : 0};
+        MS_CUDA(h, launch_resident(h->m, h->plan, h->rsp, h->s, sc, dial_mode, h->precision, len, h->rs_tag, st));
+        h->rs_tag += (unsigned)len;
+        at += len;
+    }
+    MS_CUDA(h, cudaMemcpyAsync(h->h_err, h->s.err, sizeof(DevError), cudaMemcpyDeviceToHost, st));
+    if (check_last) MS_CUDA(h, cudaMemcpyAsync(h->h_equil, h->s.equil, sizeof(DevEquil), cudaMemcpyDeviceToHost, st));
+    MS_CUDA(h, cudaStreamSynchronize(st));
+    if (h->h_err->flag == MS_ERR_TIMEOUT) {
+        // Blocks stopped at different steps; the buffer the first launch
+        // read is whole.
+        h->cur = p0;
+        return fail(h, MS_ERR_TIMEOUT, "resident step: a tile waited too long for its neighbours");
+    }
+    int launches = (int)starts.size();
+    *done = n;
+    if (h->h_err->flag) {
+        const int step = (int)(h->h_err->guard_key >> 32);
+        while (launches > 1 && starts[launches - 1] > step) --launches;
+        *done = starts[--launches];
+    }
+    h->cur = p0 ^ (launches & 1);
     return MS_OK;
 }
 
@@ -1053,10 +1181,23 @@ ms_status ms_step_n(ms_handle* h, int n, const double* dials, int dialling, doub
     // Steps that read abar/bbar from the arrays need them current; fused
     // protocol-3 steps dial in the kernel and leave them stale.
     if (!fuse_lce) MS_TRY(materialise_programmed(h));
-    if (dialling) MS_TRY(stage_dials(h, dials, n));
+    const bool resident = use_resident(h, n, dialling != 0, fuse_lce);
+    if (dialling) MS_TRY(resident ? room_for_dials(h, n) : stage_dials(h, dials, n));
     MS_TRY(reset_error(h));
-    const int p0 = h->cur;
     int done = 0;
+    if (resident) {
+        MS_TRY(run_resident(h, n, dialling ? dials : nullptr, dial_mode, dt, damping, gd, check_last, &done));
+        // After a guard trip the rest runs step by step, which stops at the
+        // tripping step with the state it started from.
+        if (done < n) {
+            DevError z{};
+            z.base = done;
+            z.guard_key = ~0ULL;
+            MS_CUDA(h, cudaMemcpyAsync(h->s.err, &z, sizeof(DevError), cudaMemcpyHostToDevice, st));
+        }
+    }
+    const int resident_done = done;
+    const int p0 = h->cur ^ (done & 1);  // parity step 0 would have had
     while (done < n) {
         const int len = std::min(kChunk, n - done);
         const bool last_chunk = done + len == n;
@@ -1090,9 +1231,12 @@ ms_status ms_step_n(ms_handle* h, int n, const double* dials, int dialling, doub
         MS_CUDA(h, cudaGraphLaunch(exec, st));
         done += len;
     }
-    MS_CUDA(h, cudaMemcpyAsync(h->h_err, h->s.err, sizeof(DevError), cudaMemcpyDeviceToHost, st));
-    if (check_last) MS_CUDA(h, cudaMemcpyAsync(h->h_equil, h->s.equil, sizeof(DevEquil), cudaMemcpyDeviceToHost, st));
-    MS_CUDA(h, cudaStreamSynchronize(st));
+    if (resident_done < n) {
+        MS_CUDA(h, cudaMemcpyAsync(h->h_err, h->s.err, sizeof(DevError), cudaMemcpyDeviceToHost, st));
+        if (check_last)
+            MS_CUDA(h, cudaMemcpyAsync(h->h_equil, h->s.equil, sizeof(DevEquil), cudaMemcpyDeviceToHost, st));
+        MS_CUDA(h, cudaStreamSynchronize(st));
+    }
     if (h->h_err->flag) {
         const unsigned long long key = h->h_err->guard_key;
         const int step = (int)(key >> 32);
@@ -1141,6 +1285,7 @@ ms_status ms_prepare_steps(ms_handle* h, int n, int dialling, double dt, double 
         return fail(h, MS_ERR_INVALID_ARGUMENT, "dialling steps need ms_set_programmed");
     const bool fuse_lce = dialling && lce_fusable(h);
     if (dialling && !fuse_lce) return MS_OK;  // launched step by step, no graph to build
+    if (use_resident(h, n, dialling != 0, fuse_lce)) return MS_OK;  // one launch, no graph to build
     const int dial_mode = fuse_lce ? DIAL_LCE : DIAL_ARRAYS;
     const bool cluster = use_cluster(h, dialling != 0);
     if (dialling) {

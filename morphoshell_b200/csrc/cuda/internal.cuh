@@ -227,6 +227,33 @@ void fill_node_tile_records(const NodeTileLayout& L, const int* patch_ids, const
 void fill_node_sections(const NodeTileLayout& L, size_t pitch, std::vector<unsigned char>& sections,
                         std::vector<int>& chunk_tri);
 
+// Resident step (resident.cu): many steps in one cooperative launch, one
+// block per node tile, one thread per triangle of the tile.
+struct ResidentPlan {
+    int nodes, ntiles;             // nodes per tile (consecutive), tiles = blocks
+    int halo;                      // room for a tile's halo nodes
+    int threads;                   // threads per block (triangle slots; at least 3 per node)
+    int width;                     // longest entry list of a node
+    const int4* head;              // [ntiles] triangles, halo nodes of the tile
+    const int* tri;                // [ntiles][threads] triangle of each slot
+    const unsigned short* local;   // [ntiles][6][threads] patch nodes: index in the tile, or nodes + index in the halo
+    const int* halo_id;            // [ntiles][halo] node ids, ascending
+    const unsigned short* entries; // [ntiles][width][nodes] entry k of each node: 3 slot threads + triangle slot
+    const unsigned char* border;   // [N] another tile reads this node
+    const unsigned char* count;    // [N] entries of this node
+    ulonglong2* packets;           // [2][3][N] positions in flight, each half of a double beside its step's tag
+};
+struct ResidentLayout {
+    int nodes = 0, ntiles = 0, halo = 0, threads = 0, width = 0;
+    std::vector<int> head, tri, halo_id;
+    std::vector<unsigned short> local, entries;
+    std::vector<unsigned char> border, count;
+};
+// Host side of the plan for `sms` blocks (off, ent as for node_tile_layout);
+// false when the mesh has too many triangles for one thread each.
+bool resident_layout(const int* patch_ids, int N, int T, int sms, const std::vector<int>& off,
+                     const std::vector<int>& ent, ResidentLayout& L);
+
 // Layout of the per-(triangle, slot) force contributions: x, y, z doubles;
 // for the mixed path x, y, z floats, optionally padded with a zero to 16
 // bytes so that the node kernel loads each with one vector load.
@@ -363,6 +390,14 @@ int node_tile_blocks_target(int mixed);
 cudaError_t prepare_node_tile_kernels(int mixed, size_t smem, int* blocks_per_sm);
 cudaError_t launch_node_tiles(const DevMesh& m, const ClusterPlan& p, const NodeTilePlan& q, const DevState& s,
                               const StepScalars& sc, int dial_mode, int mixed, cudaStream_t st);
+// Resident step (resident.cu): kernel set-up (resident blocks per SM) and the
+// launch of `steps` steps from buffer sc.parity to the other one; the packets
+// carry the tags tag0 + 1 .. tag0 + steps, which no earlier launch on these
+// packets may have used last.
+cudaError_t prepare_resident(const ResidentPlan& q, int mixed, int* blocks_per_sm);
+cudaError_t launch_resident(const DevMesh& m, const ClusterPlan& p, const ResidentPlan& q, const DevState& s,
+                            const StepScalars& sc, int dial_mode, int mixed, int steps, unsigned tag0,
+                            cudaStream_t st);
 // Largest cluster size (8, 4, 2, 1) whose clusters fill the most SMs, and the
 // CTA shape used with it.
 int choose_cluster_size(int tpc, int threads, int mixed);
