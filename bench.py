@@ -707,7 +707,7 @@ def run_mlp(args):
                        "rows_per_s": rows * args.steps / (ms / 1e3), "loss_last": float(losses[-1])},
             "roofline": {"bound": "tensor", "achieved": tflops, "peak": peak, "unit": "TFLOP/s",
                          "frac": tflops / peak, "traffic": None, "peak_kind": peak_kind,
-                         "kernel": "k_gemm (tcgen05, the whole training step incl. transposes, Adam, host loss reads)"},
+                         "kernel": "k_network + k_dweights (tcgen05), the whole training step incl. Adam, host loss reads"},
             "clocks": clk.summary()}
     print(json.dumps(line), flush=True)
     return 0

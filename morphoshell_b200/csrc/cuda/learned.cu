@@ -1,19 +1,19 @@
 // Coordinate network for the learned warm start (ms_mlp_* in
 // include/morphoshell_gpu.h): a SiLU MLP trained and evaluated on the GPU
-// with the tcgen05 BF16 GEMM of tc_gemm.cuh (FP32 accumulation), FP32
-// master weights and Adam.
+// with tcgen05 BF16 MMAs (FP32 accumulation in tensor memory), FP32 master
+// weights and Adam.
 //
 // Layer l maps K_l inputs to N_l outputs: Z_l = H_{l-1} W_l^T + b_l,
 // H_l = SiLU(Z_l) on hidden layers, the last layer linear.  Widths are
-// padded: inputs to a multiple of 16, the output to 16.  Backward for a
-// batch of B rows (padded to a multiple of 128, padding rows carry zero
-// gradient):
-//   dY     = 2 (Y - T) / (rows * out)               (mean squared error)
-//   dW_l   = dZ_l^T H_{l-1}                          GEMM, K = B, split-K
-//   db_l   = column sums of dZ_l
-//   dZ_l-1 = (dZ_l W_l) * SiLU'(Z_l-1)               GEMM with fused epilogue
-// The transposed operands (dZ^T, H^T, W^T) are materialised by a transpose
-// kernel so that every GEMM is A[M x K] * B[N x K]^T with K contiguous.
+// padded: inputs to a multiple of 16, the output to 16.  Z, H and the
+// backward dZ are rounded to BF16.  A training step on B rows (padded to a
+// multiple of 128, padding rows carry zero gradient) is four launches:
+//   k_network   rows -> Y, the loss and dY = 2 (Y - T) / (rows * out), and
+//               dZ_{l-1} = (dZ_l W_l) * SiLU'(Z_{l-1}) down to layer 0
+//   k_dweights  dW_l = dZ_l^T H_{l-1}, every layer, split over the rows
+//   k_colsums   db_l = column sums of dZ_l, every layer, partials
+//   k_update    the partials' sums, Adam, the BF16 weights, the loss
+// and a forward pass is k_network alone.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -30,138 +30,740 @@ namespace {
 
 constexpr int kMaxLayers = 8;
 
-__global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int rows,
-                                 int cols, int ld_in, int ld_out) {
-    __shared__ __nv_bfloat16 tile[32][33];
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int r = r0 + i, c = c0 + threadIdx.x;
-        tile[i][threadIdx.x] = (r < rows && c < cols) ? in[(size_t)r * ld_in + c] : __float2bfloat16(0.0f);
-    }
-    __syncthreads();
-    for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-        const int c = c0 + i, r = r0 + threadIdx.x;
-        if (c < cols && r < rows) out[(size_t)c * ld_out + r] = tile[threadIdx.x][i];
-    }
+// Activations and their gradients lie in HBM as k_network's operands lie in
+// shared memory: tiles of 128 rows, in a tile 8 columns of its 128 rows
+// after another ([tile][column / 8][128][8]).  A row's 8 columns are 16
+// bytes, so 32 rows' stores are 512 contiguous bytes; a tile's columns are
+// one bulk copy; and the same bytes are a K-major operand of the layers and
+// an MN-major one of the weight gradients (8 rows x 16 bytes are a core
+// matrix of both).
+
+// ---- k_network: all layers of 128 rows in one cluster ------------------------------
+//
+// A cluster of width / 128 CTAs takes 128 rows through every layer: each CTA
+// holds the layer's whole input (128 rows x K, BF16) in shared memory and
+// computes 128 of the layer's outputs (one 128 x 128 accumulator in tensor
+// memory); its epilogue writes them, as the next layer's input, into its own
+// shared memory and its peers' (distributed shared memory).  So activations
+// never come back from HBM on the way forward, and dZ never on the way back;
+// what the weight gradients need (every operation's input) and Z, which the
+// backward epilogues read again, leave while the next operation is under way.
+//
+// Warps 0..15 gather the rows and run the epilogues (a warp reads the 32
+// tensor-memory lanes of its rank modulo 4, 32 of the columns), warp 16
+// streams the weights (ready-made core-matrix images, one bulk copy per 64
+// columns of K) through a ring that runs ahead across layers, warp 17 issues
+// the MMAs.  Two barriers order an operation: `ready` (the input is complete:
+// one arrival per epilogue warp of this CTA, and the bytes that the peers send;
+// they are counted as they land, so no warp waits for its own) and `done`
+// (every CTA's MMAs have read their input and this CTA's accumulator is
+// complete: one multicast commit per CTA), after which the input may be
+// overwritten.
+//
+// What bounds it: a chain of 2 layers - 1 operations of about 8,500 SM clocks
+// each at width 256 (16 MMAs 2,250, the commit's way to the epilogue 800, the
+// epilogue 3,000 to 3,700 -- special-function units: one and a half operations
+// per element, 16 per SM and clock -- and the peers' bytes landing 600).
+// Batches of 8,192 rows, width 256, 4 hidden layers, per training step of the
+// four kernels: k_network 43.5, k_update 11.1, k_dweights 10.3, k_colsums 4.8
+// us; the layer-by-layer GEMMs, transposes and reductions before took 375 us
+// in 48 launches.  Epochs of 100,003 rows in batches of 8,192: 6.4 -> 1.4 ms
+// (host permutation included); a forward pass of 9,201 rows from and to host
+// memory 420 -> 126 us.
+constexpr int kEpiWarps = 16;
+constexpr int kNetThreads = (kEpiWarps + 2) * 32;
+constexpr int kRing = 4;               // weight chunks in flight
+constexpr int kChunkK = 64;            // columns of K per chunk
+constexpr int kChunkBytes = 128 * kChunkK * 2;
+
+struct NetLayer {
+    const __nv_bfloat16* Wimg;   // W: [slice of 128 outputs][K / 8][128][8] (the last layer [K / 8][16][8])
+    const __nv_bfloat16* Wtimg;  // W^T: [slice of 128 inputs][Np / 8][128][8]
+    const float* bias;
+    __nv_bfloat16 *Z, *H, *dZ;   // tiles of width columns (hidden layers; training)
+    int K;
+};
+
+struct NetArgs {
+    int nl, width, in_dim, in_pad, out_dim, train;
+    const float* X;              // [n_rows][in_dim]
+    const float* T;              // [n_rows][out_dim] (training)
+    const long long* idx;        // row order, or null
+    long long row0, n_rows;      // rows row0 .. of the order; rows past n_rows are zero
+    __nv_bfloat16* Xb;           // tiles of in_pad columns (training)
+    __nv_bfloat16* dY;           // tiles of 16 columns (training)
+    float* Y;                    // [rows][out_dim] (forward)
+    double scale;                // 1 / (valid rows * out_dim)
+    double* loss_part;           // [B / 32]
+    int* err;
+    NetLayer L[kMaxLayers];
+};
+
+__host__ __device__ inline int net_a_bytes(int width, int in_pad) { return 128 * 2 * (width > in_pad ? width : in_pad); }
+__host__ inline int net_smem_bytes(int width, int in_pad, int nl) {
+    return net_a_bytes(width, in_pad) + kRing * kChunkBytes + nl * 128 * 4;
 }
 
-// Rows idx[row0 .. row0+B) of the data set into a padded bf16 batch; rows
-// past n_rows are zero.
-__global__ void k_gather(const float* __restrict__ X, const float* __restrict__ T, const long long* __restrict__ idx,
-                         long long row0, long long n_rows, int in_dim, int in_pad, int out_dim, int B,
-                         __nv_bfloat16* __restrict__ Xb, float* __restrict__ Tb) {
-    const int r = blockIdx.x;
-    const long long src_row = row0 + r;
-    const bool valid = src_row < n_rows;
-    const long long s = valid ? (idx ? idx[src_row] : src_row) : 0;
-    for (int c = threadIdx.x; c < in_pad; c += blockDim.x)
-        Xb[(size_t)r * in_pad + c] = __float2bfloat16(valid && c < in_dim ? X[s * in_dim + c] : 0.0f);
-    if (T)
-        for (int c = threadIdx.x; c < out_dim; c += blockDim.x) Tb[(size_t)r * out_dim + c] = valid ? T[s * out_dim + c] : 0.0f;
-}
+__global__ void __launch_bounds__(kNetThreads, 1) k_network(const NetArgs g) {
+    extern __shared__ __align__(128) unsigned char net_smem[];
+    __shared__ uint64_t full[kRing], empty[kRing], ready, done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int failed;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cl = g.width / 128;
+    const uint32_t rank = blockIdx.x % cl;
+    const int tile = blockIdx.x / cl;
+    const int a_bytes = net_a_bytes(g.width, g.in_pad);
+    unsigned char* As = net_smem;
+    const uint32_t a_addr = tc::smem_u32(As);
+    const uint32_t ring_addr = a_addr + a_bytes;
+    float* sbias = reinterpret_cast<float*>(net_smem + a_bytes + kRing * kChunkBytes);  // [nl][128]
+    const int nl = g.nl;
+    const int n_ops = g.train ? 2 * nl - 1 : nl;  // forward layers, then backward layers nl - 1 .. 1
 
-// dY (bf16, [B][out_pad]) and per-block partial sums of the squared error.
-__global__ void k_loss_grad(const float* __restrict__ Y, const float* __restrict__ T, int B, int valid_rows, int out_dim,
-                            int out_pad, double scale, __nv_bfloat16* __restrict__ dY, double* __restrict__ part) {
-    __shared__ double red[256];
-    double acc = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B * out_pad; i += gridDim.x * blockDim.x) {
-        const int r = i / out_pad, c = i % out_pad;
-        float g = 0.0f;
-        if (r < valid_rows && c < out_dim) {
-            const float d = Y[(size_t)r * out_pad + c] - T[(size_t)r * out_dim + c];
-            acc += (double)d * (double)d;
-            g = (float)(2.0 * scale * d);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kRing; ++i) {
+            tc::mbar_init(&full[i], 1);
+            tc::mbar_init(&empty[i], 1);
         }
-        dY[i] = __float2bfloat16(g);
+        tc::mbar_init(&ready, kEpiWarps + 1);
+        tc::mbar_init(&done, cl);
+        failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    red[threadIdx.x] = acc;
+    if (warp == kEpiWarps + 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         tc::smem_u32(&tmem_slot)),
+                     "r"(128u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // No CTA touches a peer's barriers or memory before they are set up.
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+
+    // A wait that runs out marks the CTA failed; this thread's later waits are
+    // then skipped and the sequence runs on (its results are reported as
+    // failed), so that peers get their arrivals.
+    bool dead = false;
+    auto give_up = [&]() {
+        dead = true;
+        *(volatile int*)&failed = 1;
+    };
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+        if (!dead && !tc::mbar_wait_bounded(bar, parity)) give_up();
+    };
+    // Operation o: the B operand's image (rows x K, 8-column groups) and K.
+    auto operand = [&](int o, int& K, int& rows) -> const __nv_bfloat16* {
+        rows = 128;
+        if (o < nl - 1) {
+            K = g.L[o].K;
+            return g.L[o].Wimg + (size_t)rank * 128 * K;
+        }
+        if (o == nl - 1) {
+            K = g.width;
+            rows = 16;
+            return g.L[o].Wimg;
+        }
+        const int l = 2 * nl - 1 - o;  // nl - 1 .. 1
+        K = l == nl - 1 ? 16 : g.width;
+        return g.L[l].Wtimg + (size_t)rank * 128 * K;
+    };
+
+    if (warp == kEpiWarps) {
+        if (lane == 0) {
+            int q = 0;
+            for (int o = 0; o < n_ops; ++o) {
+                int K, rows;
+                const __nv_bfloat16* img = operand(o, K, rows);
+                for (int k = 0; k < K; k += kChunkK, ++q) {
+                    const int slot = q % kRing;
+                    if (q >= kRing) wait(&empty[slot], (q / kRing - 1) & 1);
+                    if (dead) continue;
+                    const int kc = min(kChunkK, K - k);
+                    tc::bulk_load(ring_addr + slot * kChunkBytes, img + (size_t)k * rows, (uint32_t)(kc * rows * 2),
+                                  &full[slot]);
+                }
+            }
+        }
+    } else if (warp == kEpiWarps + 1) {
+        // The whole warp walks the sequence, so that descriptors stay in
+        // uniform registers; one elected lane issues.
+        const uint16_t mask = (uint16_t)((1u << cl) - 1u);
+        const uint64_t a_desc = tc::smem_desc(a_addr, 2048, 128);
+        int slot = 0;
+        uint32_t turn = 0;
+        for (int o = 0; o < n_ops; ++o) {
+            // The peers' part of this input; X and dY every CTA makes itself.
+            if (tc::elect_one())
+                tc::mbar_arrive_expect(&ready, o == 0 || o == nl ? 0u : (uint32_t)((cl - 1) * 128 * 128 * 2));
+            __syncwarp();
+            int K, rows;
+            operand(o, K, rows);
+            const uint32_t idesc = tc::instr_desc_bf16(rows);
+            const uint64_t b_step = (uint64_t)(rows * 32 >> 4);  // 16 columns of K
+            if (!dead && !tc::mbar_wait_bounded<true>(&ready, o & 1)) give_up();
+            // The input was written through the generic proxy, by this CTA's
+            // warps and its peers'.
+            asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int k = 0; k < K; k += kChunkK) {
+                wait(&full[slot], turn);
+                const int steps = min(kChunkK, K - k) / 16;
+                const uint64_t ad = a_desc + (uint64_t)(k / 8 * (2048 >> 4));
+                const uint64_t bd = tc::smem_desc(ring_addr + slot * kChunkBytes, rows * 16, 128);
+                if (tc::elect_one()) {
+                    if (!dead) {
+#pragma unroll
+                        for (int j = 0; j < kChunkK / 16; ++j)
+                            if (j < steps)
+                                tc::mma_bf16(tmem, ad + (uint64_t)(j * (2 * 2048 >> 4)), bd + j * b_step, idesc,
+                                             k + j > 0 ? 1u : 0u);
+                    }
+                    tc::mma_commit(&empty[slot]);
+                }
+                if (++slot == kRing) {
+                    slot = 0;
+                    turn ^= 1u;
+                }
+            }
+            if (tc::elect_one()) tc::mma_commit_cluster(&done, mask);
+            __syncwarp();
+        }
+    } else {
+        const int r = (warp & 3) * 32 + lane;      // row in the tile
+        const int c0 = (warp >> 2) * 32;           // this warp's 32 of the CTA's 128 columns
+        const long long src = g.row0 + (long long)tile * 128 + r;
+        const bool valid = src < g.n_rows;
+        const long long row = valid ? (g.idx ? g.idx[src] : src) : 0;
+        // The hand-over of an operation's input: this warp's part is written.
+        auto hand_over = [&]() {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&ready);
+        };
+        for (int i = threadIdx.x; i < (nl - 1) * 128; i += kEpiWarps * 32)
+            sbias[i] = g.L[i / 128].bias[rank * 128 + i % 128];
+        if (threadIdx.x < 16) sbias[(nl - 1) * 128 + threadIdx.x] = g.L[nl - 1].bias[threadIdx.x];
+        // Rows in BF16, 8 columns a step.
+        for (int c = (warp >> 2) * 8; c < g.in_pad; c += 32) {
+            __align__(16) __nv_bfloat16 b[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                b[j] = __float2bfloat16(valid && c + j < g.in_dim ? __ldg(g.X + row * g.in_dim + c + j) : 0.0f);
+            const uint4 v = *reinterpret_cast<const uint4*>(b);
+            *reinterpret_cast<uint4*>(As + c / 8 * 2048 + r * 16) = v;
+            if (g.train && rank == 0)
+                *reinterpret_cast<uint4*>(g.Xb + ((size_t)tile * g.in_pad + c) * 128 + r * 8) = v;
+        }
+        hand_over();
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");  // the biases
+        uint32_t peer[3], peer_ready[3];  // the peers' inputs and barriers (width <= 512: at most 3)
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            peer[p] = p + 1 < cl ? tc::peer_addr(a_addr, (rank + 1 + p) % cl) : 0u;
+            peer_ready[p] = p + 1 < cl ? tc::peer_addr(tc::smem_u32(&ready), (rank + 1 + p) % cl) : 0u;
+        }
+        // 8 values of columns n .. n + 7 (of the whole layer) into the next
+        // operation's input, here and in the peers.
+        auto to_input = [&](int n, const uint4& v) {
+            const uint32_t off = (uint32_t)(n / 8 * 2048 + r * 16);
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+                if (p + 1 < cl) tc::store_async(peer[p] + off, v, peer_ready[p]);
+            *reinterpret_cast<uint4*>(As + off) = v;
+        };
+        const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const int n0 = (int)rank * 128 + c0;       // first column, of the whole layer
+        // This thread's 16 bytes of column group n0 / 8 in a tile of width columns.
+        const size_t at = ((size_t)tile * g.width + n0) * 128 + r * 8;
+        // kGroup columns at a time through the arithmetic.
+        constexpr int kGroup = 16;
+        auto pack2 = [](float lo, float hi) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+            return *reinterpret_cast<const uint32_t*>(&b);
+        };
+        auto half_of = [](uint32_t b, int hi) { return __uint_as_float(hi ? b & 0xffff0000u : b << 16); };
+        uint32_t zb[16];  // 32 columns of Z
+        uint4 kept[4];    // 32 columns of what the next operation takes in
+        for (int o = 0; o < n_ops; ++o) {
+            // A backward operation's Z was written in this launch, by this
+            // thread: it is on its way while the MMAs run.
+            if (o >= nl) {
+                const __nv_bfloat16* z = g.L[2 * nl - 2 - o].Z + at;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(z + j * 1024);
+                    zb[4 * j] = w.x;
+                    zb[4 * j + 1] = w.y;
+                    zb[4 * j + 2] = w.z;
+                    zb[4 * j + 3] = w.w;
+                }
+            }
+            wait(&done, o & 1);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (o < nl - 1) {
+                uint32_t a[32];
+                tc::tmem_ld32(trow + c0, a);
+                tc::tmem_wait();
+#pragma unroll
+                for (int u = 0; u < 32; u += kGroup) {
+                    float z[kGroup], hv[kGroup];
+#pragma unroll
+                    for (int j = 0; j < kGroup; j += 4) {
+                        const float4 b = *reinterpret_cast<const float4*>(&sbias[o * 128 + c0 + u + j]);
+                        const uint32_t* s = a + u + j;
+                        zb[(u + j) / 2] = pack2(__uint_as_float(s[0]) + b.x, __uint_as_float(s[1]) + b.y);
+                        zb[(u + j) / 2 + 1] = pack2(__uint_as_float(s[2]) + b.z, __uint_as_float(s[3]) + b.w);
+                    }
+#pragma unroll
+                    for (int j = 0; j < kGroup; ++j) z[j] = half_of(zb[(u + j) / 2], j & 1);
+                    tc::over_one_plus_exp(z, z, hv);
+#pragma unroll
+                    for (int j = 0; j < kGroup; j += 8) {
+                        kept[(u + j) / 8] = make_uint4(pack2(hv[j], hv[j + 1]), pack2(hv[j + 2], hv[j + 3]),
+                                                       pack2(hv[j + 4], hv[j + 5]), pack2(hv[j + 6], hv[j + 7]));
+                        to_input(n0 + u + j, kept[(u + j) / 8]);
+                    }
+                }
+            } else if (o == nl - 1) {
+                // Every CTA of the cluster has the 16 output columns; each
+                // makes its own dY input, the first writes the results.
+                if (warp < 4) {
+                    uint32_t a[16];
+                    tc::tmem_ld16(trow, a);
+                    float yv[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) yv[j] = __uint_as_float(a[j]) + sbias[(nl - 1) * 128 + j];
+                    if (!g.train) {
+                        if (rank == 0 && valid)
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (j < g.out_dim) g.Y[((size_t)tile * 128 + r) * g.out_dim + j] = yv[j];
+                    } else {
+                        float d[16];
+                        double acc = 0.0;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            d[j] = 0.0f;
+                            if (valid && j < g.out_dim) {
+                                const float e = yv[j] - __ldg(g.T + row * g.out_dim + j);
+                                acc += (double)e * (double)e;
+                                d[j] = (float)(2.0 * g.scale * e);
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < 16; u += 8) {
+                            const uint4 v = make_uint4(pack2(d[u], d[u + 1]), pack2(d[u + 2], d[u + 3]),
+                                                       pack2(d[u + 4], d[u + 5]), pack2(d[u + 6], d[u + 7]));
+                            *reinterpret_cast<uint4*>(As + u / 8 * 2048 + r * 16) = v;
+                            if (rank == 0)
+                                *reinterpret_cast<uint4*>(g.dY + ((size_t)tile * 16 + u) * 128 + r * 8) = v;
+                        }
+#pragma unroll
+                        for (int s = 16; s > 0; s >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, s);
+                        if (rank == 0 && lane == 0) g.loss_part[tile * 4 + warp] = acc;
+                    }
+                }
+            } else {
+                const bool more = o + 1 < n_ops;
+                uint32_t a[32];
+                tc::tmem_ld32(trow + c0, a);
+                tc::tmem_wait();
+#pragma unroll
+                for (int u = 0; u < 32; u += kGroup) {
+                    float one[kGroup], z[kGroup], s[kGroup];
+#pragma unroll
+                    for (int j = 0; j < kGroup; ++j) {
+                        one[j] = 1.0f;
+                        z[j] = half_of(zb[(u + j) / 2], j & 1);
+                    }
+                    tc::over_one_plus_exp(one, z, s);
+                    // SiLU'(z) = s (1 + z (1 - s))
+#pragma unroll
+                    for (int j = 0; j < kGroup; ++j)
+                        s[j] = __uint_as_float(a[u + j]) * (s[j] * (1.0f + z[j] * (1.0f - s[j])));
+#pragma unroll
+                    for (int j = 0; j < kGroup; j += 8) {
+                        kept[(u + j) / 8] = make_uint4(pack2(s[j], s[j + 1]), pack2(s[j + 2], s[j + 3]),
+                                                       pack2(s[j + 4], s[j + 5]), pack2(s[j + 6], s[j + 7]));
+                        if (more) to_input(n0 + u + j, kept[(u + j) / 8]);
+                    }
+                }
+            }
+            if (o + 1 < n_ops) hand_over();
+            // What later kernels and the way back read, once the next
+            // operation is on its way.
+            if (g.train && o != nl - 1) {
+                __nv_bfloat16* h = (o < nl ? g.L[o].H : g.L[2 * nl - 2 - o].dZ) + at;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(h + j * 1024) = kept[j];
+                if (o < nl) {
+                    __nv_bfloat16* z = g.L[o].Z + at;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        *reinterpret_cast<uint4*>(z + j * 1024) =
+                            make_uint4(zb[4 * j], zb[4 * j + 1], zb[4 * j + 2], zb[4 * j + 3]);
+                }
+            }
+        }
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (failed && threadIdx.x == 0) {
+        // Give copies in flight a bounded chance to land before the block ends.
+        for (int i = 0; i < kRing; ++i) tc::mbar_wait_bounded(&full[i], 0);
+        atomicExch(g.err, 1);
+    }
+    __syncthreads();
+    // No CTA leaves while a peer may still write its memory or arrive.
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    if (warp == kEpiWarps + 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128u) : "memory");
 }
 
-// Sum of the split-K partials [S][Mp][ldp] into out[M][N] (+= when accumulate).
-__global__ void k_splitk_sum(const float* __restrict__ part, int S, int Mp, int ldp, int M, int N,
-                             float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M * N) return;
-    const int m = i / N, n = i % N;
-    float s = 0.0f;
-    for (int k = 0; k < S; ++k) s += part[((size_t)k * Mp + m) * ldp + n];
-    out[i] = s;
+// ---- k_dweights: every layer's dW, split over the rows ---------------------------------
+//
+// A job is one layer: D[m][n] = sum over rows of A[row][m] B[row][n], both
+// operands MN-major as they lie in HBM: A = dZ_l (m = output) and B = H_{l-1}
+// (n = input); for the last layer A = H, B = dY, whose 16 columns would leave
+// most of a 128-row accumulator empty the other way round.  One CTA takes 128
+// m, up to 256 n and kSplitRows rows and writes its partial in FP32; k_update
+// adds the partials in row order.  A stage is a tile of 128 rows, two bulk
+// copies of up to 32 and 64 KB; two stages.  What bounds it: those copies
+// (1.5 bytes of L2 per 128 multiply-adds), then the partials' way to L2.
+constexpr int kDwThreads = 256;
+constexpr int kDwStages = 2;
+constexpr int kSplitRows = 512;                      // rows per CTA
+constexpr int kDwA = 128 * 128 * 2, kDwStage = kDwA + 128 * 256 * 2;
+
+struct DwJob {
+    const __nv_bfloat16 *A, *B;  // tiles of lda, ldb columns
+    int lda, ldb;
+    int first_block, m_tiles, n_tiles;
+    float* part;                 // [split][ldb / 4][lda][4]: element (m, n) at ((n / 4) lda + m) 4 + n % 4
+};
+struct DwArgs {
+    int jobs, rows;
+    int* err;
+    DwJob J[kMaxLayers];
+};
+
+__global__ void __launch_bounds__(kDwThreads, 1) k_dweights(const DwArgs g) {
+    extern __shared__ __align__(128) unsigned char dw_smem[];
+    __shared__ uint64_t full[kDwStages], empty[kDwStages], done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int failed;
+    int ji = 0;
+    while (ji + 1 < g.jobs && (int)blockIdx.x >= g.J[ji + 1].first_block) ++ji;
+    const DwJob& J = g.J[ji];
+    int t = (int)blockIdx.x - J.first_block;
+    const int m0 = t % J.m_tiles * 128;
+    t /= J.m_tiles;
+    const int n0 = t % J.n_tiles * 256;
+    const int split = t / J.n_tiles;
+    const int nn = min(256, J.ldb - n0);
+    const int r0 = split * kSplitRows, r1 = min(g.rows, r0 + kSplitRows);
+    const int nk = (r1 - r0) / 128;  // rows is a multiple of 128
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kDwStages; ++i) {
+            tc::mbar_init(&full[i], 1);
+            tc::mbar_init(&empty[i], 1);
+        }
+        tc::mbar_init(&done, 1);
+        failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         tc::smem_u32(&tmem_slot)),
+                     "r"(256u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const uint32_t base = tc::smem_u32(dw_smem);
+    bool dead = false;
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+        if (!dead && !tc::mbar_wait_bounded(bar, parity)) {
+            dead = true;
+            *(volatile int*)&failed = 1;
+        }
+    };
+    if (warp == 0) {
+        if (lane == 0)
+            for (int kt = 0; kt < nk; ++kt) {
+                const int s = kt % kDwStages;
+                if (kt >= kDwStages) wait(&empty[s], (kt / kDwStages - 1) & 1);
+                if (dead) break;
+                const size_t tile = (size_t)r0 / 128 + kt;
+                const uint32_t st = base + s * kDwStage, bytes_b = (uint32_t)nn * 256;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(&full[s])),
+                             "r"((uint32_t)kDwA + bytes_b)
+                             : "memory");
+                tc::bulk_copy(st, J.A + (tile * J.lda + m0) * 128, kDwA, &full[s]);
+                tc::bulk_copy(st + kDwA, J.B + (tile * J.ldb + n0) * 128, bytes_b, &full[s]);
+            }
+    } else if (warp == 1) {
+        const uint32_t idesc = tc::instr_desc_bf16(nn, true);
+        for (int kt = 0; kt < nk; ++kt) {
+            const int s = kt % kDwStages;
+            wait(&full[s], (kt / kDwStages) & 1);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t ad = tc::smem_desc(base + s * kDwStage, 128, 2048);
+            const uint64_t bd = tc::smem_desc(base + s * kDwStage + kDwA, 128, 2048);
+            if (tc::elect_one()) {
+                if (!dead) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        tc::mma_bf16(tmem, ad + (uint64_t)(j * (256 >> 4)), bd + (uint64_t)(j * (256 >> 4)), idesc,
+                                     (kt > 0 || j > 0) ? 1u : 0u);
+                }
+                tc::mma_commit(&empty[s]);
+                if (kt + 1 == nk) tc::mma_commit(&done);
+            }
+            __syncwarp();
+        }
+    }
+    __syncwarp();
+    wait(&done, 0);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (failed) {
+        if (threadIdx.x == 0) {
+            for (int i = 0; i < kDwStages; ++i) tc::mbar_wait_bounded(&full[i], 0);
+            atomicExch(g.err, 1);
+        }
+    } else {
+        const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const int m = m0 + (warp & 3) * 32 + lane;
+        float* out = J.part + (size_t)split * J.ldb * J.lda + ((size_t)(n0 / 4) * J.lda + m) * 4;
+#pragma unroll 1
+        for (int c0 = (warp >> 2) * 16; c0 < nn; c0 += 32) {
+            uint32_t r[16];
+            tc::tmem_ld16(trow + c0, r);
+#pragma unroll
+            for (int j = 0; j < 16; j += 4)
+                *reinterpret_cast<float4*>(out + (size_t)(c0 + j) * J.lda) =
+                    make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
+                                __uint_as_float(r[j + 3]));
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
 }
 
-// Column sums of a bf16 [B][N] matrix (bias gradients) in two fixed-order
-// passes: block (x, y) sums columns 32x .. 32x+31 over rows
-// [y R, (y+1) R) into part[y][c] (8 row lanes, then the lanes in order),
-// then one thread per column adds the partials in order.
+// ---- bias gradients, update ---------------------------------------------------------
+//
+// Column sums of dZ (bias gradients) in two fixed-order passes: block (x, y,
+// layer) sums columns 32x .. 32x+31 over rows [y R, (y+1) R) into part[y][c]
+// (8 row lanes, then the lanes in order), then k_update adds the partials in
+// order.  A thread takes 8 columns (16 bytes) of every 8th row.
 constexpr int kColChunks = 64;
 
-__global__ void k_colsum_part(const __nv_bfloat16* __restrict__ D, int B, int N, float* __restrict__ part) {
+struct ColJob {
+    const __nv_bfloat16* D;  // tiles of N columns
+    int N;
+    float* part;             // [kColChunks][N]
+};
+struct ColArgs {
+    int rows;
+    ColJob J[kMaxLayers];
+};
+
+__global__ void __launch_bounds__(32) k_colsums(const ColArgs g) {
     __shared__ float acc[8][33];
-    const int c = blockIdx.x * 32 + threadIdx.x;
+    const ColJob& J = g.J[blockIdx.z];
+    const int N = J.N, B = g.rows;
+    if ((int)blockIdx.x * 32 >= N) return;  // uniform over the block
+    const int y = threadIdx.x & 7, q = threadIdx.x >> 3;  // row lane, 8-column group
+    const int c = blockIdx.x * 32 + q * 8;
     const int R = (B + kColChunks - 1) / kColChunks;
     const int r0 = blockIdx.y * R, r1 = min(B, r0 + R);
-    float s = 0.0f;
+    float s[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] = 0.0f;
     if (c < N)
-        for (int r = r0 + threadIdx.y; r < r1; r += 8) s += __bfloat162float(D[(size_t)r * N + c]);
-    acc[threadIdx.y][threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.y == 0 && c < N) {
+#pragma unroll 4
+        for (int r = r0 + y; r < r1; r += 8) {
+            const uint4 w = *reinterpret_cast<const uint4*>(J.D + ((size_t)(r / 128) * N + c) * 128 + r % 128 * 8);
+            const uint32_t b[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[j] += __uint_as_float(j & 1 ? b[j / 2] & 0xffff0000u : b[j / 2] << 16);
+        }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[y][q * 8 + j] = s[j];
+    __syncwarp();
+    if ((int)(blockIdx.x * 32 + threadIdx.x) < N) {
         float t = acc[0][threadIdx.x];
         for (int k = 1; k < 8; ++k) t += acc[k][threadIdx.x];
-        part[(size_t)blockIdx.y * N + c] = t;
+        J.part[(size_t)blockIdx.y * N + blockIdx.x * 32 + threadIdx.x] = t;
     }
 }
 
-__global__ void k_colsum_final(const float* __restrict__ part, int N, int n_valid, float* __restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_valid) return;
-    float s = 0.0f;
-    for (int k = 0; k < kColChunks; ++k) s += part[(size_t)k * N + c];
-    out[c] = s;
-}
+struct UpLayer {
+    int first;                     // first parameter (weights [N][K], then biases [Np])
+    int first_block;
+    int N, K, Np;
+    const float* part;             // dW partials (DwJob::part): (output, input), or (input, output) for the last layer
+    const float* colpart;          // [kColChunks][Np]
+    __nv_bfloat16 *Wimg, *Wtimg;
+};
+enum UpMode { UP_ADAM = 0, UP_GRADS = 1, UP_IMAGES = 2 };
+struct UpArgs {
+    int nl, splits, width, mode;
+    float lr, b1, b2, eps, c1, c2;
+    float *p, *g, *m1, *m2;
+    const double* loss_part;
+    int loss_parts;
+    double* loss_acc;
+    UpLayer L[kMaxLayers];
+};
 
-// acc[0] += sum of the loss partials (one thread, fixed order).
-__global__ void k_loss_accumulate(const double* __restrict__ part, int n, double* __restrict__ acc) {
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    acc[0] += s;
-}
+// Blocks of a layer: 32 x 32 weights each (N is 16 or fewer on the last
+// layer), and one for the biases.
+__host__ __device__ inline int up_blocks(int N, int K) { return (N + 31) / 32 * ((K + 31) / 32) + 1; }
 
-__global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m1,
-                       float* __restrict__ m2, long long n, float lr, float b1, float b2, float eps, float c1,
-                       float c2) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float a = b1 * m1[i] + (1.0f - b1) * gi;
-    const float b = b2 * m2[i] + (1.0f - b2) * gi * gi;
-    m1[i] = a;
-    m2[i] = b;
-    p[i] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
-}
-
-// FP32 master weights [N][K] -> bf16 [Np][K] (rows past N zero) and its
-// transpose [K][Np].
-__global__ void k_weights_bf16(const float* __restrict__ W, int N, int K, int Np, __nv_bfloat16* __restrict__ Wb,
-                               __nv_bfloat16* __restrict__ Wt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Np * K) return;
-    const int n = i / K, k = i % K;
-    const __nv_bfloat16 v = __float2bfloat16(n < N ? W[(size_t)n * K + k] : 0.0f);
-    Wb[i] = v;
-    Wt[(size_t)k * Np + n] = v;
+// Partial sums in row order, Adam and the BF16 images of the weights; the last
+// block adds up the loss.  UP_GRADS stops at the gradients, UP_IMAGES only
+// makes the images.  A block's weights change places through shared memory
+// between the partials (neighbouring threads on neighbouring outputs), the
+// parameters (on neighbouring inputs) and the two images.
+__global__ void __launch_bounds__(256) k_update(const UpArgs u) {
+    __shared__ float tile[32][33];
+    __shared__ double red[256];
+    if (blockIdx.x == gridDim.x - 1) {
+        if (u.mode == UP_IMAGES) return;
+        double s = 0.0;
+        for (int i = threadIdx.x; i < u.loss_parts; i += 256) s += u.loss_part[i];
+        red[threadIdx.x] = s;
+        __syncthreads();
+        for (int w = 128; w > 0; w >>= 1) {
+            if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) u.loss_acc[0] += red[0];
+        return;
+    }
+    int l = 0;
+    while (l + 1 < u.nl && (int)blockIdx.x >= u.L[l + 1].first_block) ++l;
+    const UpLayer& y = u.L[l];
+    const bool last = l == u.nl - 1;
+    // A parameter's step; returns its new value.
+    auto step = [&](int i, float gi) -> float {
+        if (u.mode == UP_IMAGES) return u.p[i];
+        u.g[i] = gi;
+        if (u.mode == UP_GRADS) return 0.0f;
+        // Roundings spelled out, so that they do not depend on what the
+        // compiler contracts here.
+        const float a = __fmaf_rn(1.0f - u.b1, gi, __fmul_rn(u.b1, u.m1[i]));
+        const float b = __fmaf_rn(__fmul_rn(1.0f - u.b2, gi), gi, __fmul_rn(u.b2, u.m2[i]));
+        u.m1[i] = a;
+        u.m2[i] = b;
+        const float w = u.p[i] - u.lr * (a / u.c1) / (sqrtf(b / u.c2) + u.eps);
+        u.p[i] = w;
+        return w;
+    };
+    const int kt = (y.K + 31) / 32, bi = (int)blockIdx.x - y.first_block;
+    if (bi == (y.N + 31) / 32 * kt) {  // biases
+        for (int n = threadIdx.x; n < y.Np; n += 256) {
+            float gi = 0.0f;
+            if (u.mode != UP_IMAGES && n < y.N)
+#pragma unroll 8
+                for (int k = 0; k < kColChunks; ++k) gi += y.colpart[(size_t)k * y.Np + n];
+            step(y.first + y.N * y.K + n, gi);
+        }
+        return;
+    }
+    const int n0 = bi / kt * 32, k0 = bi % kt * 32;
+    if (u.mode != UP_IMAGES) {
+        float gr[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (!last) {
+            // Four inputs (k) of one output (n) per thread.
+            const int n = threadIdx.x & 31, k = (int)(threadIdx.x >> 5) * 4;
+            if (k0 + k < y.K) {
+                const float4* s = reinterpret_cast<const float4*>(y.part) + (size_t)((k0 + k) / 4) * u.width + n0 + n;
+                const size_t stride = (size_t)(y.K / 4) * u.width;
+#pragma unroll 8
+                for (int i = 0; i < u.splits; ++i) {
+                    const float4 v = s[i * stride];
+                    gr[0] += v.x;
+                    gr[1] += v.y;
+                    gr[2] += v.z;
+                    gr[3] += v.w;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) tile[n][k + j] = gr[j];
+        } else {
+            // Four outputs of one input per thread.
+            const int k = threadIdx.x & 31, n = (int)(threadIdx.x >> 5) * 4;
+            if (n < 16) {
+                const float4* s = reinterpret_cast<const float4*>(y.part) + (size_t)(n / 4) * u.width + k0 + k;
+                const size_t stride = (size_t)4 * u.width;
+#pragma unroll 8
+                for (int i = 0; i < u.splits; ++i) {
+                    const float4 v = s[i * stride];
+                    gr[0] += v.x;
+                    gr[1] += v.y;
+                    gr[2] += v.z;
+                    gr[3] += v.w;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) tile[n + j][k] = gr[j];
+        }
+        __syncthreads();
+    }
+    // Rows n of the parameters, 32 inputs together.
+    {
+        const int k = threadIdx.x & 31, kk = k0 + k;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = (int)(threadIdx.x >> 5) + 8 * j, nn = n0 + n;
+            if (nn < y.N && kk < y.K) tile[n][k] = step(y.first + nn * y.K + kk, tile[n][k]);
+        }
+    }
+    if (u.mode == UP_GRADS) return;
+    __syncthreads();
+    const int rows = last ? 16 : 128;
+    // W: 8 inputs of one output are 16 bytes; W^T: 8 outputs of one input.
+    // Outputs past N (the last layer's padding) keep their zeros.
+    for (int i = threadIdx.x; i < 2 * 32 * 4; i += 256) {
+        const bool second = i >= 32 * 4;
+        const int r = i & 31, c = (i >> 5 & 3) * 8;
+        const int n = second ? c : r, k = second ? r : c;
+        if (n0 + n >= y.N || k0 + k >= y.K || (second && l == 0)) continue;
+        __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const bool in = !second || n0 + n + j < y.N;
+            v[j] = __float2bfloat16(in ? (second ? tile[n + j][k] : tile[n][k + j]) : 0.0f);
+        }
+        const int nn = n0 + n, kk = k0 + k;
+        __nv_bfloat16* to = second ? y.Wtimg + (((size_t)(kk / 128) * (y.Np / 8) + nn / 8) * 128 + kk % 128) * 8
+                                   : y.Wimg + (((size_t)(nn / rows) * (y.K / 8) + kk / 8) * rows + nn % rows) * 8;
+        *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(v);
+    }
 }
 
 struct Layer {
-    int K, N, Np;            // inputs, outputs, outputs padded (16 for the last layer)
-    size_t w_off, b_off;     // offsets into the flat parameter vector
-    __nv_bfloat16 *Wb, *Wt;  // [Np][K], [K][Np]
+    int K, N, Np;               // inputs, outputs, outputs padded (16 for the last layer)
+    size_t w_off, b_off;        // offsets into the flat parameter vector
+    __nv_bfloat16 *Wimg, *Wtimg;  // BF16 weights and their transpose as k_network's operand images
+    size_t part_off = 0;        // of a split's partials, in floats per split
 };
 
 }  // namespace
@@ -176,15 +778,17 @@ struct ms_mlp {
     long long adam_t = 0;
     // batch work space (rows = cap)
     int cap = 0;
-    __nv_bfloat16 *Xb = nullptr, *XbT = nullptr;
-    __nv_bfloat16 *Z[kMaxLayers] = {}, *H[kMaxLayers] = {}, *HT[kMaxLayers] = {};
-    __nv_bfloat16 *dZ = nullptr, *dZ2 = nullptr, *dZT = nullptr;
-    float *Y = nullptr, *Tb = nullptr, *part = nullptr;
-    double* loss_part = nullptr;
+    __nv_bfloat16 *Xb = nullptr, *dY = nullptr;
+    __nv_bfloat16 *Z[kMaxLayers] = {}, *H[kMaxLayers] = {}, *dZ[kMaxLayers] = {};
+    float *part = nullptr;        // split partials of dW, layer after layer
+    float* colpart = nullptr;     // [nl][kColChunks][width] bias-gradient partials
+    double* loss_part = nullptr;  // [cap / 32]
     double* loss_acc = nullptr;   // [1] running sum over an epoch
-    float* colpart = nullptr;     // [kColChunks][width] bias-gradient partials
-    size_t part_cap = 0;
+    // forward-pass staging (rows = io_cap)
+    int io_cap = 0;
+    float *d_x = nullptr, *d_y = nullptr;
     int* err = nullptr;
+    int* h_err = nullptr;         // pinned
     // data set
     float *dX = nullptr, *dT = nullptr;
     long long n_rows = 0;
@@ -223,192 +827,173 @@ ms_status malloc_dev(ms_mlp* h, T** p, size_t count) {
     return MS_OK;
 }
 
-template <int BN, int EPI>
-cudaError_t launch_gemm(const tc::GemmArgs& a, int splits, cudaStream_t st) {
-    static bool attr_set = false;
-    constexpr int smem = tc::gemm_smem_bytes<BN>();
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(tc::k_gemm<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        attr_set = true;
+void release(ms_mlp* h, std::initializer_list<void*> ps) {
+    for (void* q : ps) {
+        if (!q) continue;
+        cudaFree(q);
+        h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), q), h->allocs.end());
     }
-    dim3 grid(a.M / tc::kBM, a.N / BN, splits);
-    tc::k_gemm<BN, EPI><<<grid, tc::kThreads, smem, st>>>(a);
-    return cudaGetLastError();
 }
 
-// C = A B^T with the widest tile that divides N.
-cudaError_t gemm(const tc::GemmArgs& a, int epi, int splits, cudaStream_t st) {
-    if (a.N % 128 == 0) {
-        if (epi == tc::EPI_F32) return launch_gemm<128, tc::EPI_F32>(a, splits, st);
-        if (epi == tc::EPI_BIAS_SILU) return launch_gemm<128, tc::EPI_BIAS_SILU>(a, splits, st);
-        return launch_gemm<128, tc::EPI_DSILU>(a, splits, st);
-    }
-    if (a.N % 32 == 0) {
-        if (epi == tc::EPI_F32) return launch_gemm<32, tc::EPI_F32>(a, splits, st);
-        if (epi == tc::EPI_BIAS_SILU) return launch_gemm<32, tc::EPI_BIAS_SILU>(a, splits, st);
-        return launch_gemm<32, tc::EPI_DSILU>(a, splits, st);
-    }
-    if (a.N % 16 == 0) {
-        if (epi == tc::EPI_F32) return launch_gemm<16, tc::EPI_F32>(a, splits, st);
-        if (epi == tc::EPI_BIAS_SILU) return launch_gemm<16, tc::EPI_BIAS_SILU>(a, splits, st);
-        return launch_gemm<16, tc::EPI_DSILU>(a, splits, st);
-    }
-    return cudaErrorInvalidValue;
-}
+// Splits of dW over a batch of B rows.
+int dw_splits(int B) { return (B + kSplitRows - 1) / kSplitRows; }
 
+// Training buffers for batches of up to `rows` rows.
 ms_status ensure_batch(ms_mlp* h, int rows) {
     if (rows <= h->cap) return MS_OK;
-    const int B = rows;
-    ML_TRY(malloc_dev(h, &h->Xb, (size_t)B * h->in_pad));
-    ML_TRY(malloc_dev(h, &h->XbT, (size_t)h->in_pad * B));
-    for (int l = 0; l < h->nl; ++l) {
-        const int Np = h->L[l].Np;
-        ML_TRY(malloc_dev(h, &h->Z[l], (size_t)B * Np));
-        ML_TRY(malloc_dev(h, &h->H[l], (size_t)B * Np));
-        ML_TRY(malloc_dev(h, &h->HT[l], (size_t)Np * B));
+    h->cap = 0;
+    release(h, {h->Xb, h->dY, h->part, h->loss_part});
+    h->Xb = h->dY = nullptr;
+    h->part = nullptr;
+    h->loss_part = nullptr;
+    for (int l = 0; l < h->nl - 1; ++l) {
+        release(h, {h->Z[l], h->H[l], h->dZ[l]});
+        h->Z[l] = h->H[l] = h->dZ[l] = nullptr;
     }
-    ML_TRY(malloc_dev(h, &h->dZ, (size_t)B * h->width));
-    ML_TRY(malloc_dev(h, &h->dZ2, (size_t)B * h->width));
-    ML_TRY(malloc_dev(h, &h->dZT, (size_t)std::max(h->width, 128) * B));
-    ML_CUDA(h, cudaMemset(h->dZT, 0, sizeof(__nv_bfloat16) * (size_t)std::max(h->width, 128) * B));
-    ML_TRY(malloc_dev(h, &h->Y, (size_t)B * 16));
-    ML_TRY(malloc_dev(h, &h->Tb, (size_t)B * h->out_dim));
-    ML_TRY(malloc_dev(h, &h->loss_part, 1024));
-    ML_TRY(malloc_dev(h, &h->loss_acc, 1));
-    ML_TRY(malloc_dev(h, &h->colpart, (size_t)kColChunks * std::max(h->width, 16)));
+    const size_t B = rows;
+    ML_TRY(malloc_dev(h, &h->Xb, B * h->in_pad));
+    ML_TRY(malloc_dev(h, &h->dY, B * 16));
+    size_t per_split = 0;
+    for (int l = 0; l < h->nl; ++l) {
+        if (l < h->nl - 1) {
+            ML_TRY(malloc_dev(h, &h->Z[l], B * h->width));
+            ML_TRY(malloc_dev(h, &h->H[l], B * h->width));
+            ML_TRY(malloc_dev(h, &h->dZ[l], B * h->width));
+        }
+        h->L[l].part_off = per_split;
+        per_split += (size_t)h->width * (l == h->nl - 1 ? 16 : h->L[l].K);
+    }
+    ML_TRY(malloc_dev(h, &h->part, per_split * dw_splits(rows)));
+    ML_TRY(malloc_dev(h, &h->loss_part, B / 32));
     h->cap = rows;
     return MS_OK;
 }
 
-ms_status ensure_part(ms_mlp* h, size_t count) {
-    if (count <= h->part_cap) return MS_OK;
-    ML_TRY(malloc_dev(h, &h->part, count));
-    h->part_cap = count;
+// Host rows of a forward pass: staging for up to `rows` rows.
+ms_status ensure_io(ms_mlp* h, int rows) {
+    if (rows <= h->io_cap) return MS_OK;
+    h->io_cap = 0;
+    release(h, {h->d_x, h->d_y});
+    h->d_x = h->d_y = nullptr;
+    ML_TRY(malloc_dev(h, &h->d_x, (size_t)rows * h->in_dim));
+    ML_TRY(malloc_dev(h, &h->d_y, (size_t)rows * h->out_dim));
+    h->io_cap = rows;
     return MS_OK;
 }
 
-ms_status refresh_bf16(ms_mlp* h) {
+NetArgs net_args(const ms_mlp* h) {
+    NetArgs a{};
+    a.nl = h->nl;
+    a.width = h->width;
+    a.in_dim = h->in_dim;
+    a.in_pad = h->in_pad;
+    a.out_dim = h->out_dim;
+    a.err = h->err;
     for (int l = 0; l < h->nl; ++l) {
         const Layer& y = h->L[l];
-        const int n = y.Np * y.K;
-        k_weights_bf16<<<(n + 255) / 256, 256, 0, h->stream>>>(h->p + y.w_off, y.N, y.K, y.Np, y.Wb, y.Wt);
+        a.L[l] = {y.Wimg, y.Wtimg, h->p + y.b_off, h->Z[l], h->H[l], h->dZ[l], y.K};
     }
+    return a;
+}
+
+ms_status launch_network(ms_mlp* h, const NetArgs& a, int B) {
+    const int cl = h->width / 128;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(B / 128 * cl);
+    cfg.blockDim = dim3(kNetThreads);
+    cfg.dynamicSmemBytes = net_smem_bytes(h->width, h->in_pad, h->nl);
+    cfg.stream = h->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cl;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    ML_CUDA(h, cudaLaunchKernelEx(&cfg, k_network, a));
+    return MS_OK;
+}
+
+// Arguments of k_update over the batch's partials (splits of them).
+UpArgs up_args(const ms_mlp* h, int mode, int splits, int B) {
+    UpArgs u{};
+    u.nl = h->nl;
+    u.splits = splits;
+    u.width = h->width;
+    u.mode = mode;
+    u.p = h->p;
+    u.g = h->g;
+    u.m1 = h->m1;
+    u.m2 = h->m2;
+    u.loss_part = h->loss_part;
+    u.loss_parts = B / 32;
+    u.loss_acc = h->loss_acc;
+    int blocks = 0;
+    for (int l = 0; l < h->nl; ++l) {
+        const Layer& y = h->L[l];
+        u.L[l] = {(int)y.w_off, blocks, y.N, y.K, y.Np, h->part + y.part_off * splits,
+                  h->colpart + (size_t)l * kColChunks * h->width, y.Wimg, y.Wtimg};
+        blocks += up_blocks(y.N, y.K);
+    }
+    return u;
+}
+
+ms_status launch_update(ms_mlp* h, const UpArgs& u) {
+    const UpLayer& last = u.L[u.nl - 1];
+    k_update<<<last.first_block + up_blocks(last.N, last.K) + 1, 256, 0, h->stream>>>(u);
     ML_CUDA(h, cudaGetLastError());
     return MS_OK;
 }
 
-// Forward pass over the rows already in h->Xb (B rows, a multiple of 128).
-ms_status forward(ms_mlp* h, int B) {
-    const __nv_bfloat16* in = h->Xb;
-    int K = h->in_pad;
-    for (int l = 0; l < h->nl; ++l) {
-        const Layer& y = h->L[l];
-        tc::GemmArgs a{};
-        a.A = in;
-        a.B = y.Wb;
-        a.M = B;
-        a.N = y.Np;
-        a.K = K;
-        a.lda = K;
-        a.ldb = K;
-        a.k_split = K;
-        a.bias = h->p + y.b_off;
-        a.ldc = y.Np;
-        a.err = h->err;
-        const bool last = l == h->nl - 1;
-        if (last) {
-            a.Cf = h->Y;
-            // bias of the padded output columns: the vector has Np entries
-            ML_CUDA(h, gemm(a, tc::EPI_F32, 1, h->stream));
-        } else {
-            a.Z = h->Z[l];
-            a.H = h->H[l];
-            ML_CUDA(h, gemm(a, tc::EPI_BIAS_SILU, 1, h->stream));
+ms_status refresh_bf16(ms_mlp* h) { return launch_update(h, up_args(h, UP_IMAGES, 0, 0)); }
+
+// Forward and backward pass of the rows that a says, a batch of B (a multiple
+// of 128, at most h->cap), up to the partials of the gradients.
+ms_status gradients(ms_mlp* h, NetArgs a, int B) {
+    a.train = 1;
+    a.Xb = h->Xb;
+    a.dY = h->dY;
+    a.loss_part = h->loss_part;
+    const long long valid = std::max(1LL, std::min<long long>(B, a.n_rows - a.row0));
+    a.scale = 1.0 / ((double)valid * h->out_dim);
+    ML_TRY(launch_network(h, a, B));
+    const int splits = dw_splits(B), nl = h->nl;
+    DwArgs d{};
+    ColArgs c{};
+    d.jobs = nl;
+    d.rows = c.rows = B;
+    d.err = h->err;
+    // The hidden layers' blocks first: the others take a fraction of their
+    // time and fill the last wave.
+    int blocks = 0, jobs = 0;
+    for (int pass = 0; pass < 2; ++pass)
+        for (int l = 0; l < nl; ++l) {
+            const Layer& y = h->L[l];
+            const bool last = l == nl - 1;
+            if ((last || y.K < 256) != (pass == 1)) continue;
+            DwJob& J = d.J[jobs++];
+            J.A = last ? h->H[l - 1] : h->dZ[l];
+            J.B = last ? h->dY : (l > 0 ? h->H[l - 1] : h->Xb);
+            J.lda = h->width;
+            J.ldb = last ? 16 : y.K;
+            J.first_block = blocks;
+            J.m_tiles = h->width / 128;
+            J.n_tiles = (J.ldb + 255) / 256;
+            J.part = h->part + y.part_off * splits;
+            blocks += J.m_tiles * J.n_tiles * splits;
+            c.J[l] = {last ? h->dY : h->dZ[l], y.Np, h->colpart + (size_t)l * kColChunks * h->width};
         }
-        in = h->H[l];
-        K = y.Np;
-    }
-    return MS_OK;
-}
-
-void transpose(const __nv_bfloat16* in, __nv_bfloat16* out, int rows, int cols, int ld_in, int ld_out,
-               cudaStream_t st) {
-    dim3 grid((cols + 31) / 32, (rows + 31) / 32);
-    k_transpose_bf16<<<grid, dim3(32, 8), 0, st>>>(in, out, rows, cols, ld_in, ld_out);
-}
-
-// Backward pass after forward() and the loss gradient in h->dZ (as
-// [B][16]); gradients into h->g.
-ms_status backward(ms_mlp* h, int B) {
-    // Split K = B into chunks of 512 rows.
-    const int chunk = 512;
-    const int S = (B + chunk - 1) / chunk;
-    __nv_bfloat16* dZcur = h->dZ;  // [B][Np_l]
-    __nv_bfloat16* dZnext = h->dZ2;
-    for (int l = h->nl - 1; l >= 0; --l) {
-        const Layer& y = h->L[l];
-        const __nv_bfloat16* Hin = l > 0 ? h->H[l - 1] : h->Xb;
-        const int Kin = y.K;
-        // dW_l = dZ_l^T H_{l-1}
-        const int Mp = std::max(y.Np, 128);
-        transpose(dZcur, h->dZT, B, y.Np, y.Np, B, h->stream);
-        __nv_bfloat16* HinT = l > 0 ? h->HT[l - 1] : h->XbT;
-        transpose(Hin, HinT, B, Kin, Kin, B, h->stream);
-        ML_TRY(ensure_part(h, (size_t)S * Mp * Kin));
-        tc::GemmArgs a{};
-        a.A = h->dZT;
-        a.B = HinT;
-        a.M = Mp;
-        a.N = Kin;
-        a.K = B;
-        a.lda = B;
-        a.ldb = B;
-        a.k_split = chunk;
-        a.Cf = h->part;
-        a.ldc = Kin;
-        a.err = h->err;
-        ML_CUDA(h, gemm(a, tc::EPI_F32, S, h->stream));
-        const int nw = y.N * Kin;
-        k_splitk_sum<<<(nw + 255) / 256, 256, 0, h->stream>>>(h->part, S, Mp, Kin, y.N, Kin, h->g + y.w_off);
-        k_colsum_part<<<dim3((y.Np + 31) / 32, kColChunks), dim3(32, 8), 0, h->stream>>>(dZcur, B, y.Np,
-                                                                                         h->colpart);
-        k_colsum_final<<<(y.N + 127) / 128, 128, 0, h->stream>>>(h->colpart, y.Np, y.N, h->g + y.b_off);
-        ML_CUDA(h, cudaGetLastError());
-        if (l == 0) break;
-        // dZ_{l-1} = (dZ_l W_l) * SiLU'(Z_{l-1})
-        tc::GemmArgs b{};
-        b.A = dZcur;
-        b.B = y.Wt;
-        b.M = B;
-        b.N = Kin;
-        b.K = y.Np;
-        b.lda = y.Np;
-        b.ldb = y.Np;
-        b.k_split = y.Np;
-        b.Z = h->Z[l - 1];
-        b.H = dZnext;
-        b.ldc = Kin;
-        b.err = h->err;
-        ML_CUDA(h, gemm(b, tc::EPI_DSILU, 1, h->stream));
-        std::swap(dZcur, dZnext);
-    }
-    return MS_OK;
-}
-
-// Loss and dY of the rows in h->Tb; returns the sum of squared errors via
-// the partials (read after the stream synchronises).
-ms_status loss_grad(ms_mlp* h, int B, int valid) {
-    const double scale = 1.0 / ((double)std::max(valid, 1) * h->out_dim);
-    k_loss_grad<<<256, 256, 0, h->stream>>>(h->Y, h->Tb, B, valid, h->out_dim, 16, scale, h->dZ, h->loss_part);
+    k_dweights<<<blocks, kDwThreads, kDwStages * kDwStage, h->stream>>>(d);
+    k_colsums<<<dim3(h->width / 32, kColChunks, nl), 32, 0, h->stream>>>(c);
     ML_CUDA(h, cudaGetLastError());
     return MS_OK;
 }
 
+// Waits for the stream and reports a tensor-core wait that ran out.
 ms_status check_err(ms_mlp* h) {
-    int e = 0;
-    ML_CUDA(h, cudaMemcpy(&e, h->err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e) return mfail(h, MS_ERR_TIMEOUT, "tensor-core GEMM wait timed out");
+    ML_CUDA(h, cudaMemcpyAsync(h->h_err, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    ML_CUDA(h, cudaStreamSynchronize(h->stream));
+    if (*h->h_err) return mfail(h, MS_ERR_TIMEOUT, "tensor-core GEMM wait timed out");
     return MS_OK;
 }
 
@@ -455,13 +1040,26 @@ ms_status ms_mlp_create(int32_t in_dim, int32_t width, int32_t hidden_layers, in
     h->n_params = off;
     ms_status st;
     if ((st = malloc_dev(h, &h->p, off)) || (st = malloc_dev(h, &h->g, off)) || (st = malloc_dev(h, &h->m1, off)) ||
-        (st = malloc_dev(h, &h->m2, off)) || (st = malloc_dev(h, &h->err, 1)))
+        (st = malloc_dev(h, &h->m2, off)) || (st = malloc_dev(h, &h->err, 1)) ||
+        (st = malloc_dev(h, &h->loss_acc, 1)) ||
+        (st = malloc_dev(h, &h->colpart, (size_t)h->nl * kColChunks * width)))
         return bail(st);
+    if (cudaMallocHost(&h->h_err, sizeof(int)) != cudaSuccess) return bail(MS_ERR_OUT_OF_MEMORY);
     for (int l = 0; l < h->nl; ++l) {
+        // Rows past N of the last layer stay zero.
         Layer& y = h->L[l];
-        if ((st = malloc_dev(h, &y.Wb, (size_t)y.Np * y.K)) || (st = malloc_dev(h, &y.Wt, (size_t)y.K * y.Np)))
-            return bail(st);
+        const size_t count = (size_t)y.Np * y.K;
+        if ((st = malloc_dev(h, &y.Wimg, count)) || (st = malloc_dev(h, &y.Wtimg, count))) return bail(st);
+        if (cudaMemsetAsync(y.Wimg, 0, 2 * count, h->stream) != cudaSuccess ||
+            cudaMemsetAsync(y.Wtimg, 0, 2 * count, h->stream) != cudaSuccess)
+            return bail(MS_ERR_CUDA);
     }
+    // The kernels' shared memory limits, the same for every network.
+    if (cudaFuncSetAttribute(k_network, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             net_smem_bytes(512, 256, kMaxLayers)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_dweights, cudaFuncAttributeMaxDynamicSharedMemorySize, kDwStages * kDwStage) !=
+            cudaSuccess)
+        return bail(MS_ERR_CUDA);
     // Initial weights: normal with variance 1 / fan_in (inputs past in_dim
     // get zero weights), zero biases.
     std::vector<float> p(off, 0.0f);
@@ -473,11 +1071,14 @@ ms_status ms_mlp_create(int32_t in_dim, int32_t width, int32_t hidden_layers, in
         for (int n = 0; n < y.N; ++n)
             for (int k = 0; k < y.K; ++k) p[y.w_off + (size_t)n * y.K + k] = (l == 0 && k >= in_dim) ? 0.0f : nd(rng);
     }
-    if (cudaMemcpy(h->p, p.data(), off * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(h->g, 0, off * sizeof(float)) != cudaSuccess || cudaMemset(h->m1, 0, off * sizeof(float)) ||
-        cudaMemset(h->m2, 0, off * sizeof(float)) || cudaMemset(h->err, 0, sizeof(int)))
+    if (cudaMemcpyAsync(h->p, p.data(), off * sizeof(float), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+        cudaMemsetAsync(h->g, 0, off * sizeof(float), h->stream) != cudaSuccess ||
+        cudaMemsetAsync(h->m1, 0, off * sizeof(float), h->stream) != cudaSuccess ||
+        cudaMemsetAsync(h->m2, 0, off * sizeof(float), h->stream) != cudaSuccess ||
+        cudaMemsetAsync(h->err, 0, sizeof(int), h->stream) != cudaSuccess)
         return bail(MS_ERR_CUDA);
     if ((st = refresh_bf16(h))) return bail(st);
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bail(MS_ERR_CUDA);
     *out = h;
     return MS_OK;
 }
@@ -487,6 +1088,7 @@ void ms_mlp_destroy(ms_mlp* h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (void* q : h->allocs) cudaFree(q);
+    if (h->h_err) cudaFreeHost(h->h_err);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }
@@ -510,12 +1112,14 @@ ms_status ms_mlp_get_params(ms_mlp* h, float* params) {
 ms_status ms_mlp_set_params(ms_mlp* h, const float* params) {
     if (!h || !params) return MS_ERR_INVALID_ARGUMENT;
     cudaSetDevice(h->device);
-    ML_CUDA(h, cudaStreamSynchronize(h->stream));
-    ML_CUDA(h, cudaMemcpy(h->p, params, h->n_params * sizeof(float), cudaMemcpyHostToDevice));
+    // On the network's stream, which does not wait for the default one: a copy
+    // from pageable memory may return before it has reached the device.
+    ML_CUDA(h, cudaMemcpyAsync(h->p, params, h->n_params * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     h->adam_t = 0;
-    ML_CUDA(h, cudaMemset(h->m1, 0, h->n_params * sizeof(float)));
-    ML_CUDA(h, cudaMemset(h->m2, 0, h->n_params * sizeof(float)));
+    ML_CUDA(h, cudaMemsetAsync(h->m1, 0, h->n_params * sizeof(float), h->stream));
+    ML_CUDA(h, cudaMemsetAsync(h->m2, 0, h->n_params * sizeof(float), h->stream));
     ML_TRY(refresh_bf16(h));
+    ML_CUDA(h, cudaStreamSynchronize(h->stream));
     return MS_OK;
 }
 
@@ -523,31 +1127,20 @@ ms_status ms_mlp_forward(ms_mlp* h, const float* x, int64_t n, float* y) {
     if (!h || !x || !y || n <= 0) return MS_ERR_INVALID_ARGUMENT;
     cudaSetDevice(h->device);
     const int B = round_up(std::min<int64_t>(n, 65536), 128);
-    ML_TRY(ensure_batch(h, B));
-    float* dx;
-    ML_CUDA(h, cudaMalloc(&dx, sizeof(float) * (size_t)n * h->in_dim));
-    std::vector<float> yb((size_t)B * 16);
-    ms_status rc = MS_OK;
-    if (cudaMemcpy(dx, x, sizeof(float) * (size_t)n * h->in_dim, cudaMemcpyHostToDevice) != cudaSuccess)
-        rc = mfail(h, MS_ERR_CUDA, "upload");
-    for (long long r0 = 0; r0 < n && rc == MS_OK; r0 += B) {
+    ML_TRY(ensure_io(h, B));
+    for (long long r0 = 0; r0 < n; r0 += B) {
         const int rows = (int)std::min<long long>(B, n - r0);
-        k_gather<<<B, 64, 0, h->stream>>>(dx, nullptr, nullptr, r0, n, h->in_dim, h->in_pad, h->out_dim, B, h->Xb,
-                                          nullptr);
-        rc = forward(h, B);
-        if (rc != MS_OK) break;
-        if (cudaMemcpyAsync(yb.data(), h->Y, sizeof(float) * (size_t)B * 16, cudaMemcpyDeviceToHost, h->stream) !=
-                cudaSuccess ||
-            cudaStreamSynchronize(h->stream) != cudaSuccess) {
-            rc = mfail(h, MS_ERR_CUDA, "forward");
-            break;
-        }
-        for (int r = 0; r < rows; ++r)
-            for (int c = 0; c < h->out_dim; ++c) y[(r0 + r) * h->out_dim + c] = yb[(size_t)r * 16 + c];
+        ML_CUDA(h, cudaMemcpyAsync(h->d_x, x + r0 * h->in_dim, sizeof(float) * (size_t)rows * h->in_dim,
+                                   cudaMemcpyHostToDevice, h->stream));
+        NetArgs a = net_args(h);
+        a.X = h->d_x;
+        a.n_rows = rows;
+        a.Y = h->d_y;
+        ML_TRY(launch_network(h, a, round_up(rows, 128)));
+        ML_CUDA(h, cudaMemcpyAsync(y + r0 * h->out_dim, h->d_y, sizeof(float) * (size_t)rows * h->out_dim,
+                                   cudaMemcpyDeviceToHost, h->stream));
     }
-    cudaFree(dx);
-    if (rc == MS_OK) rc = check_err(h);
-    return rc;
+    return check_err(h);
 }
 
 ms_status ms_mlp_loss_grad(ms_mlp* h, const float* x, const float* t, int64_t n, double* loss, float* grads) {
@@ -555,36 +1148,22 @@ ms_status ms_mlp_loss_grad(ms_mlp* h, const float* x, const float* t, int64_t n,
     cudaSetDevice(h->device);
     const int B = round_up(n, 128);
     ML_TRY(ensure_batch(h, B));
-    float *dx, *dt;
-    ML_CUDA(h, cudaMalloc(&dx, sizeof(float) * (size_t)n * h->in_dim));
-    if (cudaMalloc(&dt, sizeof(float) * (size_t)n * h->out_dim) != cudaSuccess) {
-        cudaFree(dx);
-        return mfail(h, MS_ERR_OUT_OF_MEMORY, "cudaMalloc");
-    }
-    ms_status rc = MS_OK;
-    if (cudaMemcpy(dx, x, sizeof(float) * (size_t)n * h->in_dim, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(dt, t, sizeof(float) * (size_t)n * h->out_dim, cudaMemcpyHostToDevice) != cudaSuccess)
-        rc = mfail(h, MS_ERR_CUDA, "upload");
-    if (rc == MS_OK) {
-        k_gather<<<B, 64, 0, h->stream>>>(dx, dt, nullptr, 0, n, h->in_dim, h->in_pad, h->out_dim, B, h->Xb, h->Tb);
-        rc = forward(h, B);
-    }
-    if (rc == MS_OK) rc = loss_grad(h, B, (int)n);
-    if (rc == MS_OK) rc = backward(h, B);
-    std::vector<double> part(256);
-    if (rc == MS_OK &&
-        (cudaMemcpyAsync(part.data(), h->loss_part, 256 * sizeof(double), cudaMemcpyDeviceToHost, h->stream) !=
-             cudaSuccess ||
-         cudaStreamSynchronize(h->stream) != cudaSuccess))
-        rc = mfail(h, MS_ERR_CUDA, "loss_grad");
-    cudaFree(dx);
-    cudaFree(dt);
-    if (rc == MS_OK) rc = check_err(h);
-    if (rc != MS_OK) return rc;
+    ML_TRY(ensure_io(h, B));
+    ML_CUDA(h, cudaMemcpyAsync(h->d_x, x, sizeof(float) * (size_t)n * h->in_dim, cudaMemcpyHostToDevice, h->stream));
+    ML_CUDA(h, cudaMemcpyAsync(h->d_y, t, sizeof(float) * (size_t)n * h->out_dim, cudaMemcpyHostToDevice, h->stream));
+    ML_CUDA(h, cudaMemsetAsync(h->loss_acc, 0, sizeof(double), h->stream));
+    NetArgs a = net_args(h);
+    a.X = h->d_x;
+    a.T = h->d_y;
+    a.n_rows = n;
+    ML_TRY(gradients(h, a, B));
+    ML_TRY(launch_update(h, up_args(h, UP_GRADS, dw_splits(B), B)));
     double s = 0.0;
-    for (double v : part) s += v;
+    ML_CUDA(h, cudaMemcpyAsync(&s, h->loss_acc, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    if (grads)
+        ML_CUDA(h, cudaMemcpyAsync(grads, h->g, h->n_params * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+    ML_TRY(check_err(h));
     if (loss) *loss = s / ((double)n * h->out_dim);
-    if (grads) ML_CUDA(h, cudaMemcpy(grads, h->g, h->n_params * sizeof(float), cudaMemcpyDeviceToHost));
     return MS_OK;
 }
 
@@ -605,8 +1184,9 @@ ms_status ms_mlp_set_data(ms_mlp* h, const float* x, const float* t, int64_t n) 
     ML_TRY(malloc_dev(h, &h->dX, (size_t)n * h->in_dim));
     ML_TRY(malloc_dev(h, &h->dT, (size_t)n * h->out_dim));
     ML_TRY(malloc_dev(h, &h->d_idx, (size_t)n));
-    ML_CUDA(h, cudaMemcpy(h->dX, x, sizeof(float) * (size_t)n * h->in_dim, cudaMemcpyHostToDevice));
-    ML_CUDA(h, cudaMemcpy(h->dT, t, sizeof(float) * (size_t)n * h->out_dim, cudaMemcpyHostToDevice));
+    ML_CUDA(h, cudaMemcpyAsync(h->dX, x, sizeof(float) * (size_t)n * h->in_dim, cudaMemcpyHostToDevice, h->stream));
+    ML_CUDA(h, cudaMemcpyAsync(h->dT, t, sizeof(float) * (size_t)n * h->out_dim, cudaMemcpyHostToDevice, h->stream));
+    ML_CUDA(h, cudaStreamSynchronize(h->stream));
     h->n_rows = n;
     return MS_OK;
 }
@@ -627,23 +1207,25 @@ ms_status ms_mlp_train(ms_mlp* h, int32_t epochs, int32_t batch, double lr, uint
         ML_CUDA(h, cudaMemcpyAsync(h->d_idx, perm.data(), sizeof(long long) * n, cudaMemcpyHostToDevice, h->stream));
         ML_CUDA(h, cudaMemsetAsync(h->loss_acc, 0, sizeof(double), h->stream));
         for (long long r0 = 0; r0 < n; r0 += B) {
-            const int rows = (int)std::min<long long>(B, n - r0);
-            k_gather<<<B, 64, 0, h->stream>>>(h->dX, h->dT, h->d_idx, r0, n, h->in_dim, h->in_pad, h->out_dim, B,
-                                              h->Xb, h->Tb);
-            ML_TRY(forward(h, B));
-            ML_TRY(loss_grad(h, B, rows));
-            ML_TRY(backward(h, B));
+            NetArgs a = net_args(h);
+            a.X = h->dX;
+            a.T = h->dT;
+            a.idx = h->d_idx;
+            a.row0 = r0;
+            a.n_rows = n;
+            ML_TRY(gradients(h, a, B));
             h->adam_t += 1;
-            const float c1 = 1.0f - std::pow(b1, (float)h->adam_t), c2 = 1.0f - std::pow(b2, (float)h->adam_t);
-            k_adam<<<(unsigned)((h->n_params + 255) / 256), 256, 0, h->stream>>>(h->p, h->g, h->m1, h->m2,
-                                                                                (long long)h->n_params, (float)lr,
-                                                                                b1, b2, eps, c1, c2);
-            ML_TRY(refresh_bf16(h));
-            k_loss_accumulate<<<1, 1, 0, h->stream>>>(h->loss_part, 256, h->loss_acc);
+            UpArgs u = up_args(h, UP_ADAM, dw_splits(B), B);
+            u.lr = (float)lr;
+            u.b1 = b1;
+            u.b2 = b2;
+            u.eps = eps;
+            u.c1 = 1.0f - std::pow(b1, (float)h->adam_t);
+            u.c2 = 1.0f - std::pow(b2, (float)h->adam_t);
+            ML_TRY(launch_update(h, u));
         }
         double ep_sum = 0.0;
         ML_CUDA(h, cudaMemcpyAsync(&ep_sum, h->loss_acc, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-        ML_CUDA(h, cudaStreamSynchronize(h->stream));
         ML_TRY(check_err(h));
         if (epoch_loss) epoch_loss[ep] = (float)(ep_sum / ((double)n * h->out_dim));
     }

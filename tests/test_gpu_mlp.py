@@ -67,3 +67,38 @@ def test_training_reduces_loss():
     xv, tv = _data(4000, seed=2)
     yv = net.forward(xv)
     assert float(((yv - tv) ** 2).mean()) < 2 * losses[-1] + 1e-3
+
+
+# Edges of the 128-row tiles and the 512-row gradient splits, of the input
+# padding, and every cluster size; tolerances as above (the same rounding
+# points, accumulation in FP32 instead of double).
+@pytest.mark.parametrize("n,in_dim,width,hidden,out_dim", [
+    (1, 1, 128, 1, 1), (127, 16, 128, 7, 3), (129, 17, 256, 2, 16), (512, 22, 384, 3, 3), (513, 256, 128, 2, 3),
+    (1025, 255, 512, 2, 2)])
+def test_network_shapes(n, in_dim, width, hidden, out_dim):
+    from oracle import mlp_ref
+    rng = np.random.default_rng(n)
+    net = _net(in_dim, width, hidden, out_dim)
+    x = rng.standard_normal((n, in_dim)).astype(np.float32)
+    t = rng.standard_normal((n, out_dim)).astype(np.float32)
+    shape = (in_dim, width, hidden, out_dim)
+    assert _rel(net.forward(x), mlp_ref.forward(net.params(), x, *shape, bf16_points=True)) < 1e-2
+    loss, g = net.loss_grad(x, t)
+    lr, gr = mlp_ref.loss_grad(net.params(), x, t, *shape, bf16_points=True)
+    assert abs(loss - lr) / lr < 1e-3
+    for off, N, K, Np in net.layers():
+        assert _rel(g[off:off + N * K], gr[off:off + N * K]) < 2e-2
+        assert _rel(g[off + N * K:off + N * K + N], gr[off + N * K:off + N * K + N]) < 2e-2
+
+
+def test_new_rows_right_after_others():
+    """Rows from pageable memory are in place when the kernels read them: a
+    short call right after another one, and new parameters right before one."""
+    from oracle import mlp_ref
+    net = _net(width=256, hidden=2)
+    p = net.params()
+    for k in range(20):
+        x, t = _data(1000, seed=k)
+        net.loss_grad(x[::-1], t)
+        net.set_params(p * np.float32(1.0 + 0.01 * k))
+        assert _rel(net.forward(x), mlp_ref.forward(net.params(), x, 22, 256, 2, 3, bf16_points=True)) < 1e-2
