@@ -12,17 +12,23 @@
 // device memory.
 //
 // Scratch: one file-scope __device__ array sized for meshes of up to
-// kMaxTris triangles and kMaxNodes nodes (about 11.5 MB, held by every GPU
+// kMaxTris triangles and kMaxNodes nodes (about 13 MB, held by every GPU
 // that loads the library until the process exits).  Larger meshes are
 // rejected.  Every call shares the array and it keeps the last call's
 // contents, so two calls that overlap on the GPU (different streams, or
 // different host threads on the same device) race and corrupt each other;
-// serialise them.  The per-node counters are cleared at the start of every
-// call.
+// serialise them.  The chains' heads are cleared at the start of every call.
 //
-// The node sums are deterministic: each node's incidence list is rebuilt in
-// the scratch (integer counting, then each list sorted by triangle), and its
-// contributions are added in ascending triangle order, as in the main path.
+// The node sums are deterministic: a node's entries are chained as they come
+// (one atomic exchange each), sorted by triangle when the node is summed, and
+// added in ascending triangle order, as in the main path.
+//
+// Two kernels: k_na_tri (chains, and the triangles' contributions) and
+// k_na_gather (sort and sum).  What bounds them: a node's walk along its
+// chain, about 12 dependent trips to L2, and the tables' one trip from HBM.
+// Incidence lists built by counting, a one-block scan, filling and sorting
+// were five more launches; a call for 50,310 triangles took 114 us, now 53.
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 
@@ -36,10 +42,11 @@ constexpr int kMaxNodes = 65536;
 
 struct Scratch {
     double contrib[kMaxTris * 18];  // per (triangle, slot) force contribution
-    int count[kMaxNodes + 1];       // entries per node, then exclusive offsets
-    int cursor[kMaxNodes];          // fill cursors
-    int entries[kMaxTris * 6];      // (6 t + slot) grouped by node
+    int next[kMaxTris * 6];         // entry 6 t + slot: its chain's next entry + 1, or 0
+    int entries[kMaxTris * 6];      // sorted entries of the nodes with long chains
     int bad;                        // patch ids outside [0, num_nodes) seen this call
+    int used;                       // of entries
+    int head[kMaxNodes];            // a node's first entry + 1, or 0 (bad, used and head are cleared every call)
 };
 
 static __device__ __align__(256) unsigned char ms_noalloc_scratch[sizeof(Scratch)];
@@ -55,153 +62,144 @@ cudaError_t scratch_address(Scratch** out) {
     return cudaSuccess;
 }
 
-__global__ void k_na_zero(Scratch* s, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= n) s->count[i] = 0;
-    if (i < n) s->cursor[i] = 0;
-    if (i == 0) s->bad = 0;
-}
+constexpr int kTriBlock = 128;
+constexpr int kNodeBlock = 64;
+constexpr int kListed = 32;  // entries of a node sorted in shared memory
 
-// Ids outside [0, n) are counted as bad and skipped by every later kernel.
-__global__ void k_na_count(Scratch* s, const int* __restrict__ patch, int T, int n) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= 6 * T) return;
-    const int id = patch[k];
-    if (id < 0 || id >= n) {
-        atomicAdd(&s->bad, 1);
-        return;
-    }
-    atomicAdd(&s->count[id + 1], 1);
-}
-
-// Inclusive scan of count[1..n] in place (one block): count[i] becomes the
-// offset of node i's first entry.
-__global__ void k_na_scan(Scratch* s, int n) {
-    __shared__ int partial[1024];
-    const int per = (n + 1 + blockDim.x - 1) / blockDim.x;
-    const int lo = threadIdx.x * per, hi = min(n + 1, lo + per);
-    int acc = 0;
-    for (int i = lo; i < hi; ++i) acc += s->count[i];
-    partial[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int w = 0; w < (int)blockDim.x; ++w) {
-            const int v = partial[w];
-            partial[w] = run;
-            run += v;
-        }
-    }
-    __syncthreads();
-    int run = partial[threadIdx.x];
-    for (int i = lo; i < hi; ++i) {
-        run += s->count[i];
-        s->count[i] = run;
-    }
-}
-
-__global__ void k_na_fill(Scratch* s, const int* __restrict__ patch, int T, int n) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= 6 * T) return;
-    const int node = patch[k];
-    if (node < 0 || node >= n) return;
-    const int pos = s->count[node] + atomicAdd(&s->cursor[node], 1);
-    s->entries[pos] = k;
-}
-
-// The fill order within a node depends on scheduling; sorting each short
-// list makes the summation order the ascending-triangle order.
-__global__ void k_na_sort(Scratch* s, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int* e = s->entries + s->count[i];
-    const int len = s->count[i + 1] - s->count[i];
-    for (int a = 1; a < len; ++a) {
-        const int v = e[a];
-        int b = a - 1;
-        while (b >= 0 && e[b] > v) {
-            e[b + 1] = e[b];
-            --b;
-        }
-        e[b + 1] = v;
-    }
-}
-
-__global__ void k_na_tri(Scratch* s, int N, int T, const int* __restrict__ patch, const double* __restrict__ coef,
-                         const double* __restrict__ area, const double* __restrict__ thick,
-                         const double* __restrict__ shear, const double* __restrict__ abar,
-                         const double* __restrict__ bbar, double nu, double gamma, const double* __restrict__ dofs) {
+__global__ void __launch_bounds__(kTriBlock)
+    k_na_tri(Scratch* s, int N, int T, const int* __restrict__ patch, const double* __restrict__ coef,
+             const double* __restrict__ area, const double* __restrict__ thick, const double* __restrict__ shear,
+             const double* __restrict__ abar, const double* __restrict__ bbar, double nu, double gamma,
+             const double* __restrict__ dofs) {
     using namespace msb::dev;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
-    double c[24], P[6][3];
-    for (int k = 0; k < 24; ++k) c[k] = coef[24 * (size_t)t + k];
-    for (int k = 0; k < 6; ++k) {
-        int id = patch[6 * (size_t)t + k];
-        if (id < 0 || id >= N) id = 0;  // reported through Scratch::bad; never read out of range
-        P[k][0] = dofs[id];
-        P[k][1] = dofs[(size_t)N + id];
-        P[k][2] = dofs[2 * (size_t)N + id];
-    }
-    double rx[3], ry[3], rxx[3], rxy[3], ryy[3];
-    for (int i = 0; i < 3; ++i) {
-        rx[i] = c[0] * P[0][i] + c[1] * P[1][i] + c[2] * P[2][i];
-        ry[i] = c[3] * P[0][i] + c[4] * P[1][i] + c[5] * P[2][i];
-        double sxx = 0, sxy = 0, syy = 0;
+    // The block's weights in one run, then its contributions: rows of 24 and
+    // 18 doubles would be 32 separate lines per warp access.
+    __shared__ double rows[kTriBlock * 24];
+    const int t0 = blockIdx.x * kTriBlock, i = threadIdx.x, t = t0 + i;
+    const int live = min(kTriBlock, T - t0);
+    for (int e = i; e < 24 * live; e += kTriBlock) rows[e] = coef[24 * (size_t)t0 + e];
+    __syncthreads();
+    double c[24], f[18];
+    if (i < live) {
+        double P[6][3];
+#pragma unroll
+        for (int k = 0; k < 24; ++k) c[k] = rows[24 * i + k];
+#pragma unroll
         for (int k = 0; k < 6; ++k) {
-            sxx += c[6 + 3 * k] * P[k][i];
-            sxy += c[7 + 3 * k] * P[k][i];
-            syy += c[8 + 3 * k] * P[k][i];
+            int id = patch[6 * (size_t)t + k];
+            if (id < 0 || id >= N) {
+                // Reported; never read out of range, on no chain.
+                atomicAdd(&s->bad, 1);
+                id = 0;
+            } else {
+                s->next[6 * t + k] = atomicExch(&s->head[id], 6 * t + k + 1);
+            }
+            P[k][0] = dofs[id];
+            P[k][1] = dofs[(size_t)N + id];
+            P[k][2] = dofs[2 * (size_t)N + id];
         }
-        rxx[i] = sxx;
-        rxy[i] = sxy;
-        ryy[i] = syy;
-    }
-    Cq<double> q;
-    q.rx = {rx[0], rx[1], rx[2]};
-    q.ry = {ry[0], ry[1], ry[2]};
-    q.rxx = {rxx[0], rxx[1], rxx[2]};
-    q.rxy = {rxy[0], rxy[1], rxy[2]};
-    q.ryy = {ryy[0], ryy[1], ryy[2]};
-    TriMat<double> m;
-    m.abar0 = abar[3 * (size_t)t];
-    m.abar1 = abar[3 * (size_t)t + 1];
-    m.abar2 = abar[3 * (size_t)t + 2];
-    m.bbar0 = bbar[3 * (size_t)t];
-    m.bbar1 = bbar[3 * (size_t)t + 1];
-    m.bbar2 = bbar[3 * (size_t)t + 2];
-    m.h = thick[t];
-    m.mu = shear[t];
-    material_coefs(m.h, m.mu, nu, gamma, m.ks, m.kb, m.igmh);
-    m.area = area[t];
-    CqGrad<double> g;
-    energy_gradient<double>(q, m, nu, g);
-    double* o = s->contrib + 18 * (size_t)t;
-    for (int k = 0; k < 6; ++k) {
-        const double mxx = c[6 + 3 * k], mxy = c[7 + 3 * k], myy = c[8 + 3 * k];
-        double fx = mxx * g.rxx.x + mxy * g.rxy.x + myy * g.ryy.x;
-        double fy = mxx * g.rxx.y + mxy * g.rxy.y + myy * g.ryy.y;
-        double fz = mxx * g.rxx.z + mxy * g.rxy.z + myy * g.ryy.z;
-        if (k < 3) {
-            fx += c[k] * g.rx.x + c[3 + k] * g.ry.x;
-            fy += c[k] * g.rx.y + c[3 + k] * g.ry.y;
-            fz += c[k] * g.rx.z + c[3 + k] * g.ry.z;
+        double rx[3], ry[3], rxx[3], rxy[3], ryy[3];
+        for (int d = 0; d < 3; ++d) {
+            rx[d] = c[0] * P[0][d] + c[1] * P[1][d] + c[2] * P[2][d];
+            ry[d] = c[3] * P[0][d] + c[4] * P[1][d] + c[5] * P[2][d];
+            double sxx = 0, sxy = 0, syy = 0;
+            for (int k = 0; k < 6; ++k) {
+                sxx += c[6 + 3 * k] * P[k][d];
+                sxy += c[7 + 3 * k] * P[k][d];
+                syy += c[8 + 3 * k] * P[k][d];
+            }
+            rxx[d] = sxx;
+            rxy[d] = sxy;
+            ryy[d] = syy;
         }
-        o[3 * k] = -fx;
-        o[3 * k + 1] = -fy;
-        o[3 * k + 2] = -fz;
+        Cq<double> q;
+        q.rx = {rx[0], rx[1], rx[2]};
+        q.ry = {ry[0], ry[1], ry[2]};
+        q.rxx = {rxx[0], rxx[1], rxx[2]};
+        q.rxy = {rxy[0], rxy[1], rxy[2]};
+        q.ryy = {ryy[0], ryy[1], ryy[2]};
+        TriMat<double> m;
+        m.abar0 = abar[3 * (size_t)t];
+        m.abar1 = abar[3 * (size_t)t + 1];
+        m.abar2 = abar[3 * (size_t)t + 2];
+        m.bbar0 = bbar[3 * (size_t)t];
+        m.bbar1 = bbar[3 * (size_t)t + 1];
+        m.bbar2 = bbar[3 * (size_t)t + 2];
+        m.h = thick[t];
+        m.mu = shear[t];
+        material_coefs(m.h, m.mu, nu, gamma, m.ks, m.kb, m.igmh);
+        m.area = area[t];
+        CqGrad<double> g;
+        energy_gradient<double>(q, m, nu, g);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const double mxx = c[6 + 3 * k], mxy = c[7 + 3 * k], myy = c[8 + 3 * k];
+            double fx = mxx * g.rxx.x + mxy * g.rxy.x + myy * g.ryy.x;
+            double fy = mxx * g.rxx.y + mxy * g.rxy.y + myy * g.ryy.y;
+            double fz = mxx * g.rxx.z + mxy * g.rxy.z + myy * g.ryy.z;
+            if (k < 3) {
+                fx += c[k] * g.rx.x + c[3 + k] * g.ry.x;
+                fy += c[k] * g.rx.y + c[3 + k] * g.ry.y;
+                fz += c[k] * g.rx.z + c[3 + k] * g.ry.z;
+            }
+            f[3 * k] = -fx;
+            f[3 * k + 1] = -fy;
+            f[3 * k + 2] = -fz;
+        }
     }
+    __syncthreads();
+    if (i < live)
+#pragma unroll
+        for (int k = 0; k < 18; ++k) rows[18 * i + k] = f[k];
+    __syncthreads();
+    double* o = s->contrib + 18 * (size_t)t0;
+    for (int e = i; e < 18 * live; e += kTriBlock) o[e] = rows[e];
 }
 
-__global__ void k_na_gather(const Scratch* s, int N, double* __restrict__ forces) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kNodeBlock) k_na_gather(Scratch* s, int N, double* __restrict__ forces) {
+    __shared__ int list[kListed][kNodeBlock];
+    const int n = blockIdx.x * kNodeBlock + threadIdx.x, i = threadIdx.x;
     if (n >= N) return;
+    // The chain in descending order, by insertion while it is walked (a chain
+    // starts with what came last, mostly the highest triangle).
+    int count = 0;
+    for (int e = s->head[n]; e != 0; e = s->next[e - 1]) {
+        if (count < kListed) {
+            int b = count;
+            while (b > 0 && list[b - 1][i] < e) {
+                list[b][i] = list[b - 1][i];
+                --b;
+            }
+            list[b][i] = e;
+        }
+        ++count;
+    }
     double fx = 0.0, fy = 0.0, fz = 0.0;
-    for (int k = s->count[n]; k < s->count[n + 1]; ++k) {
-        const double* c = s->contrib + 3 * (size_t)s->entries[k];
+    auto add = [&](int e) {
+        const double* c = s->contrib + 3 * (size_t)(e - 1);
         fx += c[0];
         fy += c[1];
         fz += c[2];
+    };
+    if (count <= kListed) {
+#pragma unroll 4
+        for (int k = count - 1; k >= 0; --k) add(list[k][i]);
+    } else {
+        // A longer chain: laid out from its end, which is nearly in order
+        // (blocks start in order), then insertion.
+        int* a = s->entries + atomicAdd(&s->used, count);
+        int k = count;
+        for (int e = s->head[n]; e != 0; e = s->next[e - 1]) a[--k] = e;
+        for (k = 1; k < count; ++k) {
+            const int e = a[k];
+            int b = k;
+            while (b > 0 && a[b - 1] > e) {
+                a[b] = a[b - 1];
+                --b;
+            }
+            a[b] = e;
+        }
+        for (k = 0; k < count; ++k) add(a[k]);
     }
     forces[n] = fx;
     forces[(size_t)N + n] = fy;
@@ -267,21 +265,17 @@ extern "C" ms_status ms_deformation_forces_noalloc(int32_t num_nodes, int32_t nu
         set_msg(err, err_len, buf);
         return false;
     };
-    k_na_zero<<<(N + 256) / 256, 256, 0, st>>>(s, N);
-    if (!launched("k_na_zero")) return MS_ERR_CUDA;
-    k_na_count<<<(6 * T + 255) / 256, 256, 0, st>>>(s, patch_ids, T, N);
-    if (!launched("k_na_count")) return MS_ERR_CUDA;
-    k_na_scan<<<1, 1024, 0, st>>>(s, N);
-    if (!launched("k_na_scan")) return MS_ERR_CUDA;
-    k_na_fill<<<(6 * T + 255) / 256, 256, 0, st>>>(s, patch_ids, T, N);
-    if (!launched("k_na_fill")) return MS_ERR_CUDA;
-    k_na_sort<<<(N + 255) / 256, 256, 0, st>>>(s, N);
-    if (!launched("k_na_sort")) return MS_ERR_CUDA;
-    k_na_tri<<<(T + 127) / 128, 128, 0, st>>>(s, N, T, patch_ids, deriv_coeffs, ref_area, ref_thickness,
-                                               ref_shear_modulus, abar, bbar, def_poisson_ratio,
-                                               bend_stiffening_scale_factor, dofs);
+    e = cudaMemsetAsync(&s->bad, 0, offsetof(Scratch, head) - offsetof(Scratch, bad) + sizeof(int) * (size_t)N, st);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_msg(err, err_len, cudaGetErrorString(e));
+        return MS_ERR_CUDA;
+    }
+    k_na_tri<<<(T + kTriBlock - 1) / kTriBlock, kTriBlock, 0, st>>>(
+        s, N, T, patch_ids, deriv_coeffs, ref_area, ref_thickness, ref_shear_modulus, abar, bbar, def_poisson_ratio,
+        bend_stiffening_scale_factor, dofs);
     if (!launched("k_na_tri")) return MS_ERR_CUDA;
-    k_na_gather<<<(N + 255) / 256, 256, 0, st>>>(s, N, forces);
+    k_na_gather<<<(N + kNodeBlock - 1) / kNodeBlock, kNodeBlock, 0, st>>>(s, N, forces);
     if (!launched("k_na_gather")) return MS_ERR_CUDA;
     // Wait for the result and check the ids (a plain host int: no allocation).
     int bad = 0;

@@ -74,6 +74,29 @@ def test_noalloc_matches_handle_path_on_two_calls(workdir):
         assert rel_err(got, ref) < FORCE_RTOL, (m.num_tris, seed, rel_err(got, ref))
 
 
+@pytest.mark.parametrize("shared", [31, 32, 33, 700])
+def test_noalloc_nodes_of_many_triangles(workdir, shared):
+    """A node on more patches than a node's sorted list holds (32): `shared`
+    triangles get it as their last patch node, besides its own."""
+    import types
+
+    m = make_model(workdir, "disk50")
+    ids = m.tables()["patch_ids"].astype(np.int32)
+    own = int((ids == 7).sum())
+    free = [t for t in range(m.num_tris) if 7 not in ids[t]][:: max(1, m.num_tris // 1000)]
+    ids[free[:max(0, shared - own)], 5] = 7
+    assert (ids == 7).sum() == shared
+    desc = type(m.desc)()
+    C.memmove(C.byref(desc), C.byref(m.desc), C.sizeof(desc))
+    desc.patch_ids = ids.ctypes.data_as(C.POINTER(C.c_int32))
+    tables = dict(m.tables(), patch_ids=ids)
+    mm = types.SimpleNamespace(desc=desc, params=m.params, scalars=m.scalars, num_nodes=m.num_nodes,
+                               num_tris=m.num_tris, programmed=m.programmed, tables=lambda: tables)
+    x, v = deformed_state(m, seed=14)
+    ref, abar, bbar = _reference_forces(mm, x, v, 0.5)
+    assert rel_err(_noalloc(mm, x, abar, bbar), ref) < FORCE_RTOL
+
+
 def test_noalloc_rejects_meshes_beyond_its_scratch():
     from morphoshell_b200 import lib
     err = C.create_string_buffer(256)
