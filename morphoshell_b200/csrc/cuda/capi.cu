@@ -67,8 +67,7 @@ struct ms_handle {
     DevError* h_err = nullptr;  // pinned mirror
     DevEquil* h_equil = nullptr;
     double* d_scratch_tri = nullptr;  // [2][T]
-    double* d_scratch_node = nullptr; // [N]
-    double* d_sum_partial = nullptr;  // [512]
+    double* d_sum_partial = nullptr;  // [3][256][2]
     double* d_sums = nullptr;         // [4]
     double* d_out = nullptr;          // generic output staging, sized on demand
     size_t out_cap = 0;
@@ -149,16 +148,25 @@ ms_status upload_transposed(ms_handle* h, T* dst, const T* src, size_t rows, int
     std::vector<T> tmp(rows * cols);
     for (size_t r = 0; r < rows; ++r)
         for (int c = 0; c < cols; ++c) tmp[(size_t)c * rows + r] = src[r * cols + c];
-    MS_CUDA(h, cudaMemcpy(dst, tmp.data(), tmp.size() * sizeof(T), cudaMemcpyHostToDevice));
+    MS_CUDA(h, cudaMemcpyAsync(dst, tmp.data(), tmp.size() * sizeof(T), cudaMemcpyHostToDevice, h->stream));
     return MS_OK;
 }
 
 template <typename T>
 ms_status download_transposed(ms_handle* h, T* dst, const T* src_dev, size_t rows, int cols) {
     std::vector<T> tmp(rows * cols);
-    MS_CUDA(h, cudaMemcpy(tmp.data(), src_dev, tmp.size() * sizeof(T), cudaMemcpyDeviceToHost));
+    MS_CUDA(h, cudaMemcpyAsync(tmp.data(), src_dev, tmp.size() * sizeof(T), cudaMemcpyDeviceToHost, h->stream));
+    MS_CUDA(h, cudaStreamSynchronize(h->stream));
     for (size_t r = 0; r < rows; ++r)
         for (int c = 0; c < cols; ++c) dst[r * cols + c] = tmp[(size_t)c * rows + r];
+    return MS_OK;
+}
+
+// The handle's stream does not wait for the default one, on which tables go
+// up, and a copy from pageable memory may return before it has reached the
+// device: nothing that reads the tables is launched before this.
+ms_status settle_uploads(ms_handle* h) {
+    MS_CUDA(h, cudaStreamSynchronize(cudaStreamLegacy));
     return MS_OK;
 }
 
@@ -774,8 +782,8 @@ ms_status ms_create(const ms_mesh_desc* d, const ms_params* prm, int device, int
     s.eq_blocks = (N + 255) / 256;
     if ((st = dalloc(h, &s.eq_part, s.eq_blocks)) || (st = dalloc(h, &s.eq_counter, 1))) return bail(st);
     cudaMemset(s.eq_counter, 0, sizeof(unsigned int));
-    if ((st = dalloc(h, &h->d_scratch_tri, 2ULL * T)) || (st = dalloc(h, &h->d_scratch_node, N)) ||
-        (st = dalloc(h, &h->d_sum_partial, 1024)) || (st = dalloc(h, &h->d_sums, 4)))
+    if ((st = dalloc(h, &h->d_scratch_tri, 2ULL * T)) || (st = dalloc(h, &h->d_sum_partial, 1536)) ||
+        (st = dalloc(h, &h->d_sums, 4)))
         return bail(st);
     if (precision == MS_PRECISION_MIXED) {
         float* contrib_f;
@@ -788,6 +796,7 @@ ms_status ms_create(const ms_mesh_desc* d, const ms_params* prm, int device, int
         cudaMallocHost(&h->h_equil, sizeof(DevEquil)) != cudaSuccess)
         return bail(MS_ERR_CUDA);
     if (reset_error(h) != MS_OK) return bail(MS_ERR_CUDA);
+    if ((st = settle_uploads(h))) return bail(st);
     cudaError_t le = cudaStreamSynchronize(h->stream);
     if (le != cudaSuccess) {
         cuda_fail(h, le, "ms_create");
@@ -847,6 +856,7 @@ ms_status ms_set_programmed(ms_handle* h, int protocol, const double* abar_info,
         return fail(h, MS_ERR_INVALID_ARGUMENT, "abar_info/bbar_info have too few columns for this protocol");
     if (protocol == 4 && !(spacing > 0)) return fail(h, MS_ERR_INVALID_ARGUMENT, "protocol 4 needs spacing > 0");
     MS_TRY(materialise_programmed(h));
+    MS_CUDA(h, cudaStreamSynchronize(h->stream));  // its kernels read what is replaced here
     const size_t T = h->m.T;
     if (h->m.info_a) {
         cudaFree((void*)h->m.info_a);
@@ -871,7 +881,7 @@ ms_status ms_set_programmed(ms_handle* h, int protocol, const double* abar_info,
     h->programmed = true;
     clear_graphs(h);  // graphs bake the mesh struct
     MS_TRY(prepare_lce_tables(h, abar_info, ka));
-    return MS_OK;
+    return settle_uploads(h);
 }
 
 ms_status ms_set_zero_dial_state(ms_handle* h, const double* a0, const double* b0) {
@@ -884,9 +894,12 @@ ms_status ms_set_zero_dial_state(ms_handle* h, const double* a0, const double* b
         ident[2 * T + t] = 1.0;
     }
     if (a0) MS_TRY(upload_transposed<double>(h, (double*)h->m.a0, a0, T, 3));
-    else MS_CUDA(h, cudaMemcpy((void*)h->m.a0, ident.data(), 3 * T * sizeof(double), cudaMemcpyHostToDevice));
+    else
+        MS_CUDA(h, cudaMemcpyAsync((void*)h->m.a0, ident.data(), 3 * T * sizeof(double), cudaMemcpyHostToDevice,
+                                   h->stream));
     if (b0) MS_TRY(upload_transposed<double>(h, (double*)h->m.b0, b0, T, 3));
-    else MS_CUDA(h, cudaMemset((void*)h->m.b0, 0, 3 * T * sizeof(double)));
+    else MS_CUDA(h, cudaMemsetAsync((void*)h->m.b0, 0, 3 * T * sizeof(double), h->stream));
+    MS_CUDA(h, cudaStreamSynchronize(h->stream));
     return MS_OK;
 }
 
@@ -895,7 +908,6 @@ ms_status ms_do_dialling(ms_handle* h, double dial) {
     if (!h->programmed) return fail(h, MS_ERR_INVALID_ARGUMENT, "ms_set_programmed has not been called");
     MS_CUDA(h, launch_dialling(h->m, h->protocol, dial, h->spacing, h->from_ansatz, h->stream));
     h->ab_stale = false;
-    MS_CUDA(h, cudaStreamSynchronize(h->stream));
     return MS_OK;
 }
 
@@ -910,8 +922,8 @@ ms_status ms_download_programmed(ms_handle* h, double* abar, double* bbar) {
 ms_status ms_surface_derivs(ms_handle* h, double* cq) {
     if (!h) return MS_ERR_INVALID_ARGUMENT;
     MS_CUDA(h, launch_surface_derivs(h->m, h->s, h->cur, h->stream));
-    if (cq)
-        MS_CUDA(h, cudaMemcpyAsync(cq, h->s.cq, 15ULL * h->m.T * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    if (!cq) return MS_OK;
+    MS_CUDA(h, cudaMemcpyAsync(cq, h->s.cq, 15ULL * h->m.T * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     MS_CUDA(h, cudaStreamSynchronize(h->stream));
     return MS_OK;
 }
@@ -939,21 +951,19 @@ ms_status ms_deformation_forces(ms_handle* h, double* forces, double* dE) {
                                    h->stream));
     if (dE)
         MS_CUDA(h, cudaMemcpyAsync(dE, h->s.dEdcq, 15ULL * h->m.T * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    MS_CUDA(h, cudaStreamSynchronize(h->stream));
+    if (forces || dE) MS_CUDA(h, cudaStreamSynchronize(h->stream));
     return MS_OK;
 }
 
 ms_status ms_non_deformation_forces(ms_handle* h, double damping, int gd) {
     if (!h) return MS_ERR_INVALID_ARGUMENT;
     if (!gd) MS_CUDA(h, launch_damping(h->m, h->s, h->cur, damping, h->rho_hh, h->stream));
-    MS_CUDA(h, cudaStreamSynchronize(h->stream));
     return MS_OK;
 }
 
 ms_status ms_impose_constraints(ms_handle* h) {
     if (!h) return MS_ERR_INVALID_ARGUMENT;
     MS_CUDA(h, launch_constraints(h->m, h->s, h->stream));
-    MS_CUDA(h, cudaStreamSynchronize(h->stream));
     return MS_OK;
 }
 
@@ -980,18 +990,19 @@ ms_status ms_advance_dynamics(ms_handle* h, double dt, double damping, int gd, i
     if (bad_dof) *bad_dof = -1;
     MS_TRY(reset_error(h));
     MS_CUDA(h, launch_guard(h->m, h->s, h->force_limit, h->stream));
+    // Updates nothing when the guard tripped.
+    MS_CUDA(h, launch_advance(h->m, h->s, h->cur, dt, damping, h->rho_hh, gd, h->stream));
     MS_CUDA(h, cudaMemcpyAsync(h->h_err, h->s.err, sizeof(DevError), cudaMemcpyDeviceToHost, h->stream));
     MS_CUDA(h, cudaStreamSynchronize(h->stream));
     if (h->h_err->flag) {
         const long long d = (long long)(h->h_err->guard_key & 0xffffffffULL);
         double f = 0;
-        cudaMemcpy(&f, h->s.forces + d, sizeof(double), cudaMemcpyDeviceToHost);
+        MS_CUDA(h, cudaMemcpyAsync(&f, h->s.forces + d, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        MS_CUDA(h, cudaStreamSynchronize(h->stream));
         if (bad_dof) *bad_dof = d;
         if (bad_force) *bad_force = f;
         return fail(h, MS_ERR_IMPLAUSIBLE_FORCE, "implausibly_high_force");
     }
-    MS_CUDA(h, launch_advance(h->m, h->s, h->cur, dt, damping, h->rho_hh, gd, h->stream));
-    MS_CUDA(h, cudaStreamSynchronize(h->stream));
     return MS_OK;
 }
 
@@ -1434,10 +1445,7 @@ ms_status ms_output_quantities(ms_handle* h, double* curv, double* edens, double
     MS_CUDA(h, launch_output_tri(h->m, h->s, dcurv, dedens, dstrain, dstress, h->d_scratch_tri, st));
     if (deficits) MS_CUDA(h, launch_angle_deficits(h->m, h->s, h->cur, ddef, st));
     if (energies) {
-        MS_CUDA(h, launch_kinetic(h->m, h->s, h->cur, h->d_scratch_node, st));
-        MS_CUDA(h, launch_comp_sum(h->d_scratch_tri, (int)T, h->d_sum_partial, h->d_sums + 0, st));
-        MS_CUDA(h, launch_comp_sum(h->d_scratch_tri + T, (int)T, h->d_sum_partial, h->d_sums + 1, st));
-        MS_CUDA(h, launch_comp_sum(h->d_scratch_node, (int)N, h->d_sum_partial, h->d_sums + 2, st));
+        MS_CUDA(h, launch_energies(h->m, h->s, h->cur, h->d_scratch_tri, h->d_sum_partial, h->d_sums, st));
         MS_CUDA(h, cudaMemcpyAsync(energies, h->d_sums, 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
     }
     if (curv) MS_CUDA(h, cudaMemcpyAsync(curv, dcurv, 2 * T * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kHaloBlock)
     }
     if (sc.check) {
         const EqPartial r = eq_block_reduce<kHaloBlock>(fmax, fnode, vmax, vnode);
-        eq_store_and_fold(s, r, part_base + blockIdx.x, gridDim.x, part_base + gridDim.x);
+        eq_store_and_fold<kHaloBlock>(s, r, part_base + blockIdx.x, gridDim.x, part_base + gridDim.x);
     }
 }
 

@@ -355,7 +355,10 @@ cudaError_t launch_a_b_normals(const DevMesh& m, const DevState& s, double* a, d
 cudaError_t launch_output_tri(const DevMesh& m, const DevState& s, double* curv, double* edens, double* strain,
                               double* stress, double* tri_energy /*[2][T]*/, cudaStream_t st);
 cudaError_t launch_angle_deficits(const DevMesh& m, const DevState& s, int parity, double* out, cudaStream_t st);
-cudaError_t launch_kinetic(const DevMesh& m, const DevState& s, int parity, double* ke /*[N]*/, cudaStream_t st);
+// Stretch, bend and kinetic energy (out[3]) as compensated sums in a fixed
+// order, from launch_output_tri's per-triangle energies.
+cudaError_t launch_energies(const DevMesh& m, const DevState& s, int parity, const double* tri_energy /*[2][T]*/,
+                            double* partial /*>= 1536*/, double* out, cudaStream_t st);
 // Advances DevError::base by `len` after a graph chunk of `len` steps.
 cudaError_t launch_chunk_end(const DevState& s, int len, cudaStream_t st);
 
@@ -408,10 +411,8 @@ int cluster_threads();
 // Raise the dynamic shared-memory limit of the cluster kernels (once, outside
 // any stream capture).
 cudaError_t prepare_cluster_kernels(int tpc);
-// Deterministic compensated sum of n doubles into *out (two passes, fixed order).
 // Sliced-ELL copy of the incidence lists (see DevMesh::sell_off): offsets
 // [ceil(N/32) + 1] and entries, built on the host from the CSR lists.
 void build_sell(int N, const int* off, const int* ent, std::vector<int>& sell_off, std::vector<int>& sell_ent);
-cudaError_t launch_comp_sum(const double* x, int n, double* partial /*>= 1024*/, double* out, cudaStream_t st);
 
 }  // namespace msb

@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kTile, MIXED ? MSB_NT_MINB_MIXED : MSB_NT_MINB
         });
     if (sc.check) {
         const EqPartial r = eq_block_reduce<kTile>(fmax, fnode, vmax, vnode);
-        eq_store_and_fold(s, r, blockIdx.x, gridDim.x, gridDim.x);
+        eq_store_and_fold<kTile>(s, r, blockIdx.x, gridDim.x, gridDim.x);
     }
 }
 

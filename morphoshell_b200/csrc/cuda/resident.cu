@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(TH, 1)
             eq_merge(w, wn, sqrt(vx * vx + vy * vy + vz * vz), n0 + i);
         }
         const EqPartial r = eq_block_reduce<TH>(f, fn, w, wn);
-        eq_store_and_fold(s, r, b, gridDim.x, gridDim.x);
+        eq_store_and_fold<TH>(s, r, b, gridDim.x, gridDim.x);
     }
 }
 
