@@ -455,7 +455,8 @@ struct ms_batch {
     int* d_node_inst = nullptr;
     double* d_fnorm = nullptr;
     double* d_vnorm = nullptr;
-    InstState* h_is = nullptr;  // pinned mirror
+    InstState* h_is = nullptr;  // pinned mirror of d_is
+    bool is_stale = true;       // a step has run since the mirror was fetched
     int* d_tri_inst = nullptr;   // [T]
     int* d_err = nullptr;        // copy-wait timeouts of the tile kernels
     int tile_grid = 0;           // 0: tile kernel unavailable
@@ -630,6 +631,7 @@ ms_status plan_from_layout(ms_batch* b, const NodeTileLayout& L, int NT, int blo
     MB_CUDA(b, cudaMemcpy(d_ctri, ctri.data(), sizeof(int) * ctri.size(), cudaMemcpyHostToDevice));
     MB_CUDA(b, cudaMemcpy2D(d_rec + L.fixed, L.stride, sections.data(), pitch, pitch, (size_t)L.C,
                             cudaMemcpyHostToDevice));
+    MB_CUDA(b, cudaStreamSynchronize(cudaStreamLegacy));
     if (L.C > 0) {
         if (b->precision == MS_PRECISION_MIXED)
             k_fill_node_tile_tables<true><<<L.C, kTile, 0, b->stream>>>(d_rec, L.stride, d_ctri, b->p.tri_idx,
@@ -680,11 +682,20 @@ bool all_frozen(const ms_batch* b) {
 }
 
 ms_status fetch_states(ms_batch* b) {
+    if (!b->is_stale) return MS_OK;
     MB_CUDA(b, cudaMemcpyAsync(b->h_is, b->d_is, sizeof(InstState) * b->n_inst, cudaMemcpyDeviceToHost, b->stream));
     int e = 0;
     if (b->d_err) MB_CUDA(b, cudaMemcpyAsync(&e, b->d_err, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
     MB_CUDA(b, cudaStreamSynchronize(b->stream));
     if (e) return bfail(b, MS_ERR_TIMEOUT, "a tile copy did not land within its bounded wait");
+    b->is_stale = false;
+    return MS_OK;
+}
+
+// Instance i's state, on the device and in the mirror.
+ms_status put_state(ms_batch* b, int i) {
+    MB_CUDA(b, cudaMemcpyAsync(b->d_is + i, &b->init_state[i], sizeof(InstState), cudaMemcpyHostToDevice, b->stream));
+    if (!b->is_stale) b->h_is[i] = b->init_state[i];
     return MS_OK;
 }
 
@@ -997,6 +1008,9 @@ ms_status ms_batch_create(const ms_batch_instance* inst, int32_t n, int32_t devi
         return bail(st);
     if (cudaMallocHost(&b->h_is, sizeof(InstState) * n) != cudaSuccess) return bail(MS_ERR_OUT_OF_MEMORY);
     std::memcpy(b->h_is, b->init_state.data(), sizeof(InstState) * n);
+    // Tables went up on the default stream, which the batch's own does not
+    // wait for; a copy from pageable memory may return before it has landed.
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) return bail(MS_ERR_CUDA);
     *out = b;
     return MS_OK;
 }
@@ -1022,6 +1036,7 @@ ms_status ms_batch_run(ms_batch* b, int64_t max_steps, int64_t* steps_done) {
     MB_TRY(fetch_states(b));
     while (done < max_steps && !all_frozen(b)) {
         const int len = (int)std::min<int64_t>(b->chunk, max_steps - done);
+        b->is_stale = true;
         MB_TRY(run_graph(b, len, b->parity, b->sched));
         b->parity ^= len & 1;
         done += len;
@@ -1059,39 +1074,40 @@ ms_status ms_batch_download_dofs(ms_batch* b, int32_t i, double* dofs, double* v
     const int buf = st.frozen_parity >= 0 ? st.frozen_parity : b->parity;
     const InstParams& q = b->ip[i];
     const size_t Ni = (size_t)(q.node_end - q.node_begin), N = (size_t)b->m.N;
-    for (int c = 0; c < 3; ++c) {
-        if (dofs)
-            MB_CUDA(b, cudaMemcpy(dofs + c * Ni, b->s.pos[buf] + c * N + q.node_begin, Ni * sizeof(double),
-                                  cudaMemcpyDeviceToHost));
-        if (vel)
-            MB_CUDA(b, cudaMemcpy(vel + c * Ni, b->s.vel[buf] + c * N + q.node_begin, Ni * sizeof(double),
-                                  cudaMemcpyDeviceToHost));
-    }
+    // The three components in one copy each.
+    const size_t row = Ni * sizeof(double), pitch = N * sizeof(double);
+    if (dofs)
+        MB_CUDA(b, cudaMemcpy2DAsync(dofs, row, b->s.pos[buf] + q.node_begin, pitch, row, 3, cudaMemcpyDeviceToHost,
+                                     b->stream));
+    if (vel)
+        MB_CUDA(b, cudaMemcpy2DAsync(vel, row, b->s.vel[buf] + q.node_begin, pitch, row, 3, cudaMemcpyDeviceToHost,
+                                     b->stream));
+    MB_CUDA(b, cudaStreamSynchronize(b->stream));
     return MS_OK;
 }
 
 ms_status ms_batch_upload_dofs(ms_batch* b, int32_t i, const double* dofs, const double* vel) {
     if (!b || !dofs || i < 0 || i >= b->n_inst) return MS_ERR_INVALID_ARGUMENT;
     cudaSetDevice(b->device);
-    MB_CUDA(b, cudaStreamSynchronize(b->stream));
+    // On the batch's stream, in order with its steps: one copy per array from
+    // the host, one more on the device for the other buffer.
     const InstParams& q = b->ip[i];
-    const size_t Ni = (size_t)(q.node_end - q.node_begin), N = (size_t)b->m.N;
-    std::vector<double> zero(vel ? 0 : Ni, 0.0);
-    for (int k = 0; k < 2; ++k)
-        for (int c = 0; c < 3; ++c) {
-            MB_CUDA(b, cudaMemcpy(b->s.pos[k] + c * N + q.node_begin, dofs + c * Ni, Ni * sizeof(double),
-                                  cudaMemcpyHostToDevice));
-            MB_CUDA(b, cudaMemcpy(b->s.vel[k] + c * N + q.node_begin, vel ? vel + c * Ni : zero.data(),
-                                  Ni * sizeof(double), cudaMemcpyHostToDevice));
-        }
-    MB_CUDA(b, cudaMemcpy(b->d_is + i, &b->init_state[i], sizeof(InstState), cudaMemcpyHostToDevice));
-    return MS_OK;
+    const size_t row = (size_t)(q.node_end - q.node_begin) * sizeof(double), pitch = (size_t)b->m.N * sizeof(double);
+    const int nb = q.node_begin;
+    cudaStream_t st = b->stream;
+    MB_CUDA(b, cudaMemcpy2DAsync(b->s.pos[0] + nb, pitch, dofs, row, row, 3, cudaMemcpyHostToDevice, st));
+    if (vel) MB_CUDA(b, cudaMemcpy2DAsync(b->s.vel[0] + nb, pitch, vel, row, row, 3, cudaMemcpyHostToDevice, st));
+    else MB_CUDA(b, cudaMemset2DAsync(b->s.vel[0] + nb, pitch, 0, row, 3, st));
+    MB_CUDA(b, cudaMemcpy2DAsync(b->s.pos[1] + nb, pitch, b->s.pos[0] + nb, pitch, row, 3, cudaMemcpyDeviceToDevice,
+                                 st));
+    MB_CUDA(b, cudaMemcpy2DAsync(b->s.vel[1] + nb, pitch, b->s.vel[0] + nb, pitch, row, 3, cudaMemcpyDeviceToDevice,
+                                 st));
+    return put_state(b, i);
 }
 
 ms_status ms_batch_set_start(ms_batch* b, int32_t i, double dial_factor, int32_t waiting) {
     if (!b || i < 0 || i >= b->n_inst || !(dial_factor >= 0.0) || dial_factor > 1.0) return MS_ERR_INVALID_ARGUMENT;
     cudaSetDevice(b->device);
-    MB_CUDA(b, cudaStreamSynchronize(b->stream));
     const InstParams& q = b->ip[i];
     InstState st = b->init_state[i];
     st.dial_factor = st.last_equil_dial = dial_factor;
@@ -1110,8 +1126,7 @@ ms_status ms_batch_set_start(ms_batch* b, int32_t i, double dial_factor, int32_t
         st.k_phase = static_cast<long long>(std::fmod(dial_factor, q.spacing) * static_cast<double>(q.steps_per_phase));
     }
     b->init_state[i] = st;
-    MB_CUDA(b, cudaMemcpy(b->d_is + i, &st, sizeof(InstState), cudaMemcpyHostToDevice));
-    return MS_OK;
+    return put_state(b, i);
 }
 
 ms_status ms_batch_set_schedule(ms_batch* b, const ms_batch_schedule* s) {
@@ -1297,6 +1312,7 @@ ms_status ms_batch_autotune(ms_batch* b, int32_t steps, ms_batch_schedule* chose
     cudaEventDestroy(ev1);
     release();
     b->parity = p0;
+    b->is_stale = true;
     clear_graphs(b);
     if (rc != MS_OK) {
         b->sched = keep_sched;
