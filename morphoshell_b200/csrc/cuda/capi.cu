@@ -93,12 +93,15 @@ struct ms_handle {
     NodeTilePlan ntp{};
     unsigned char* d_nt_rec = nullptr;
     std::vector<int> nt_chunk_tri;  // host copy of NodeTilePlan::chunk_tri
-    // resident step: many steps per launch on small meshes.  It stands in for
-    // the default path until ms_set_step_path asks for one by number.
+    // Many steps per launch: the resident step on small meshes, the streamed
+    // step (over ntp) on mid-size ones.  They stand in for the default path
+    // until ms_set_step_path asks for one by number.
     bool have_resident = false;
+    bool have_stream = false;
     bool default_path = true;
     ResidentPlan rsp{};
-    unsigned rs_tag = 0;  // tag of the last step published
+    StreamPlan stp{};
+    unsigned pk_tag = 0;  // tag of the last step published in packets
 };
 
 namespace {
@@ -279,6 +282,11 @@ ms_status build_tiles(ms_handle* h, const ms_mesh_desc* d) {
 #define MSB_NT_NODES_MIXED 1008
 #endif
 constexpr int kNtNodesMin = 256;
+// Largest tables of the streamed step.  Per step against the default path's
+// graphs: FP64 147,922 triangles (38 MB) 14.6 us against 19.0, 290,073 (74 MB)
+// 27.3 against 28.7, 358,048 33.2 against 33.3; mixed 358,048 (57 MB) 22.9
+// against 28.8.
+constexpr double kStreamBytes = 60e6;
 // Largest nodes per tile of the warp-specialised step (one block per SM): its
 // shared memory holds two table buffers, two staging areas, eight node
 // sections and the prefetched node state besides the accumulators, and tiles
@@ -294,6 +302,10 @@ constexpr int kNtNodesMin = 256;
 // tile count is a multiple of the resident blocks (SMs x blocks per SM), at
 // the largest size that keeps those blocks resident.  Leaves the other paths
 // in place when the kernel cannot be set up.
+// (forward: the streamed step's part of that plan)
+bool stream_range(const ms_handle* h, int N, int T);
+ms_status build_streamed(ms_handle* h, const StreamLayout& S);
+
 ms_status build_node_tiles(ms_handle* h, const ms_mesh_desc* d, const std::vector<int>& off,
                            const std::vector<int>& ent) {
     const int mixed = h->precision == MS_PRECISION_MIXED;
@@ -339,7 +351,29 @@ ms_status build_node_tiles(ms_handle* h, const ms_mesh_desc* d, const std::vecto
             return fail(h, MS_ERR_INVALID_ARGUMENT, err);
         if (pipe_blocks > 0) blocks = tile_blocks(tile_smem(L, NT));
     }
-    if (pipe_blocks <= 0) {
+    // The streamed step's plan, where the mesh is in its range: a tile per
+    // resident block, all in one wave.  The node-tiled step runs on it too.
+    StreamLayout S;
+    bool stream = false;
+    if (!plan4 && !h->have_resident && stream_range(h, N, T)) {
+        const int target = stream_blocks_target(mixed);
+        NT = (N + sms * target - 1) / (sms * target);
+        if (!node_tile_layout(d->patch_ids, N, T, NT, mixed, off, ent, L, err))
+            return fail(h, MS_ERR_INVALID_ARGUMENT, err);
+        stream_layout(L, d->patch_ids, N, NT, S);
+        int b = 0;
+        NodeTilePlan q{};
+        StreamPlan sp{};
+        q.stride = L.stride;
+        q.nodes = NT;
+        sp.halo = S.halo;
+        stream = stream_smem(L.stride, NT, S.halo, mixed) <= 227 * 1024 &&
+                 prepare_streamed(q, sp, mixed, &b) == cudaSuccess && (long long)b * sms >= L.K;
+        cudaGetLastError();
+        blocks = stream ? tile_blocks(tile_smem(L, NT)) : 0;
+        stream = stream && blocks > 0;
+    }
+    if (pipe_blocks <= 0 && !stream) {
         // MSB_NT_NODES in the environment overrides the largest tile (a
         // tuning knob; the plan still picks a tile count that is a multiple
         // of the resident blocks).
@@ -389,11 +423,42 @@ ms_status build_node_tiles(ms_handle* h, const ms_mesh_desc* d, const std::vecto
     }
     h->have_ntiles = q.grid > 0;
     h->have_pipe = q.grid_pipe > 0;
+    if (stream) MS_TRY(build_streamed(h, S));
     // The node-tiled kernels once every block has a tile of its own (same
     // bits as paths 1 and 2); the warp-specialised one when its plan was
     // asked for.
     if (h->have_pipe && K >= q.grid_pipe) h->step_path = 4;
-    else if (h->have_ntiles && K >= q.grid) h->step_path = 3;
+    else if (h->have_ntiles && (stream ? (N + kNtNodesMin - 1) / kNtNodesMin : K) >= q.grid) h->step_path = 3;
+    return MS_OK;
+}
+
+// Tables of one plan, gathered for one upload, each on a 16-byte boundary.
+struct TableBlob {
+    std::vector<unsigned char> bytes;
+    template <typename V>
+    size_t put(const V& v) {
+        const size_t at = bytes.size(), n = v.size() * sizeof(v[0]);
+        bytes.resize(at + (n + 15) / 16 * 16, 0);
+        std::memcpy(bytes.data() + at, v.data(), n);
+        return at;
+    }
+};
+
+// Packets of the many-step kernels, zeroed: tags start at 1.
+ms_status make_packets(ms_handle* h, ulonglong2** p) {
+    const size_t n = 6ULL * h->m.N;
+    MS_TRY(dalloc(h, p, n));
+    MS_CUDA(h, cudaMemsetAsync(*p, 0, n * sizeof(ulonglong2), h->stream));
+    return MS_OK;
+}
+
+// Equilibrium partials for n blocks.
+ms_status room_for_partials(ms_handle* h, int n) {
+    if (n <= h->s.eq_blocks) return MS_OK;
+    EqPartial* ep;
+    MS_TRY(dalloc(h, &ep, n));
+    h->s.eq_part = ep;
+    h->s.eq_blocks = n;
     return MS_OK;
 }
 
@@ -416,20 +481,13 @@ ms_status build_resident(ms_handle* h, const ms_mesh_desc* d, const std::vector<
         cudaGetLastError();
         return MS_OK;  // the other paths remain
     }
-    // One buffer: the packets (zeroed: tags start at 1), then the tables.
-    const size_t packets = 6ULL * d->num_nodes * sizeof(ulonglong2);
-    std::vector<unsigned char> blob(packets, 0);
-    auto put = [&](const auto& v) {
-        const size_t at = blob.size(), bytes = v.size() * sizeof(v[0]);
-        blob.resize(at + (bytes + 15) / 16 * 16, 0);
-        std::memcpy(blob.data() + at, v.data(), bytes);
-        return at;
-    };
-    const size_t head = put(L.head), tri = put(L.tri), halo_id = put(L.halo_id), local = put(L.local),
-                 entries = put(L.entries), border = put(L.border), count = put(L.count);
+    TableBlob blob;
+    const size_t head = blob.put(L.head), tri = blob.put(L.tri), halo_id = blob.put(L.halo_id),
+                 local = blob.put(L.local), entries = blob.put(L.entries), border = blob.put(L.border),
+                 count = blob.put(L.count);
     unsigned char* base;
-    MS_TRY(upload(h, &base, blob));
-    q.packets = reinterpret_cast<ulonglong2*>(base);
+    MS_TRY(upload(h, &base, blob.bytes));
+    MS_TRY(make_packets(h, &q.packets));
     q.head = reinterpret_cast<const int4*>(base + head);
     q.tri = reinterpret_cast<const int*>(base + tri);
     q.halo_id = reinterpret_cast<const int*>(base + halo_id);
@@ -437,14 +495,37 @@ ms_status build_resident(ms_handle* h, const ms_mesh_desc* d, const std::vector<
     q.entries = reinterpret_cast<const unsigned short*>(base + entries);
     q.border = base + border;
     q.count = base + count;
-    if (L.ntiles > h->s.eq_blocks) {
-        EqPartial* ep;
-        MS_TRY(dalloc(h, &ep, L.ntiles));
-        h->s.eq_part = ep;
-        h->s.eq_blocks = L.ntiles;
-    }
+    MS_TRY(room_for_partials(h, L.ntiles));
     h->rsp = q;
     h->have_resident = true;
+    return MS_OK;
+}
+
+// Meshes the streamed step is for: tables (of the mesh's triangles; border
+// ones come once per tile, about a quarter more) that stay in L2.
+bool stream_range(const ms_handle* h, int N, int T) {
+    int coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device);
+    const double per_tri = h->precision == MS_PRECISION_MIXED ? 160.0 : 256.0;
+    return coop && N >= 8192 && per_tri * T <= kStreamBytes;
+}
+
+ms_status build_streamed(ms_handle* h, const StreamLayout& S) {
+    TableBlob blob;
+    const size_t count = blob.put(S.halo_count), ids = blob.put(S.halo_id), local = blob.put(S.local),
+                 border = blob.put(S.border);
+    unsigned char* base;
+    MS_TRY(upload(h, &base, blob.bytes));
+    StreamPlan& q = h->stp;
+    MS_TRY(dalloc(h, &q.metric, 6ULL * kTile * h->ntp.nchunks));
+    MS_TRY(make_packets(h, &q.packets));
+    q.halo = S.halo;
+    q.halo_count = reinterpret_cast<const int*>(base + count);
+    q.halo_id = reinterpret_cast<const int*>(base + ids);
+    q.local = reinterpret_cast<const unsigned*>(base + local);
+    q.border = base + border;
+    MS_TRY(room_for_partials(h, h->ntp.ntiles));
+    h->have_stream = true;
     return MS_OK;
 }
 
@@ -540,8 +621,8 @@ ms_status build_cluster_plan(ms_handle* h, const ms_mesh_desc* d, const std::vec
     }
     h->have_plan = true;
     MS_TRY(build_tiles(h, d));
-    MS_TRY(build_node_tiles(h, d, off, ent));
-    return build_resident(h, d, off, ent);
+    MS_TRY(build_resident(h, d, off, ent));
+    return build_node_tiles(h, d, off, ent);
 }
 
 // Per-triangle director trigonometry for the cluster kernel's protocol-3
@@ -1126,14 +1207,15 @@ constexpr int kResidentFirst = 128;
 // Fewest steps of a call worth a resident launch.
 constexpr int kResidentMin = 2;
 
-// The resident step: fused protocol-3 dialling with uniform lambda_final and
-// nu_ot, or metrics from the arrays; uniform material.
+// The resident and streamed steps: fused protocol-3 dialling with uniform
+// lambda_final and nu_ot, or metrics from the arrays; uniform material.
 static bool use_resident(const ms_handle* h, int n, bool dialling, bool fuse_lce) {
-    if (!h->have_resident || !h->default_path || n < kResidentMin || !h->m.uniform_hmu) return false;
+    if (!(h->have_resident || h->have_stream) || !h->default_path || n < kResidentMin || !h->m.uniform_hmu)
+        return false;
     return dialling ? fuse_lce && h->plan.tri_aux && h->plan.lce_uniform : true;
 }
 
-// Runs n steps from h->cur as resident launches and waits for them (the
+// Runs n steps from h->cur as resident or streamed launches and waits for them (the
 // error record is in *h->h_err then, the equilibrium record in *h->h_equil
 // with check_last).  *done receives the steps that stand: n with h->cur
 // holding their state, or, when a launch tripped the guard, the steps before
@@ -1150,8 +1232,11 @@ static ms_status run_resident(ms_handle* h, int n, const double* dials, int dial
         starts.push_back(at);
         const bool last = at + len == n;
         StepScalars sc{at, p0 ^ (k & 1), dt, damping, h->rho_hh, h->force_limit, gd, check_last && last ? 1 : 0};
-        MS_CUDA(h, launch_resident(h->m, h->plan, h->rsp, h->s, sc, dial_mode, h->precision, len, h->rs_tag, st));
-        h->rs_tag += (unsigned)len;
+        if (h->have_resident)
+            MS_CUDA(h, launch_resident(h->m, h->plan, h->rsp, h->s, sc, dial_mode, h->precision, len, h->pk_tag, st));
+        else
+            MS_CUDA(h, launch_streamed(h->m, h->ntp, h->stp, h->s, sc, dial_mode, h->precision, len, h->pk_tag, st));
+        h->pk_tag += (unsigned)len;
         at += len;
     }
     MS_CUDA(h, cudaMemcpyAsync(h->h_err, h->s.err, sizeof(DevError), cudaMemcpyDeviceToHost, st));
@@ -1161,7 +1246,7 @@ static ms_status run_resident(ms_handle* h, int n, const double* dials, int dial
         // Blocks stopped at different steps; the buffer the first launch
         // read is whole.
         h->cur = p0;
-        return fail(h, MS_ERR_TIMEOUT, "resident step: a tile waited too long for its neighbours");
+        return fail(h, MS_ERR_TIMEOUT, "a tile waited too long for its neighbours' positions");
     }
     int launches = (int)starts.size();
     *done = n;
@@ -1412,7 +1497,7 @@ ms_status ms_node_tile_layout(int num_nodes, int num_tris, const int* patch_ids,
         for (int k = 0; k < 6; ++k) ent[fill[patch_ids[6LL * t + k]]++] = 6 * t + k;
     NodeTileLayout L;
     std::string err;
-    if (!node_tile_layout(patch_ids, N, T, nodes_per_tile, precision == MS_PRECISION_MIXED, off, ent, L, err))
+    if (!node_tile_layout(patch_ids, N, T, nodes_per_tile, precision == MS_PRECISION_MIXED, off, ent, L, err, -1))
         return MS_ERR_INVALID_ARGUMENT;
     out->tiles = L.K;
     out->chunks = L.C;

@@ -194,9 +194,9 @@ struct NodeTileLayout {
     size_t stride_sliced = 0;       // the record stride with them
 };
 // off/ent: each node's (6t + slot) entries in ascending order (CSR).
-// sliced: the records carry the sliced order (slice_off, dst) that the
-// warp-specialised step reads; the node-tiled step and the batch do not
-// need it.
+// sliced: 1, the records carry the sliced order (slice_off, dst) that the
+// warp-specialised step reads; -1, it is only measured; 0, the node-tiled and
+// streamed steps and the batch do not need it.
 bool node_tile_layout(const int* patch_ids, int N, int T, int NT, int mixed, const std::vector<int>& off,
                       const std::vector<int>& ent, NodeTileLayout& L, std::string& err, int sliced = 0);
 // A block walks its tiles in turn, so a step takes as long as the block with
@@ -253,6 +253,27 @@ struct ResidentLayout {
 // false when the mesh has too many triangles for one thread each.
 bool resident_layout(const int* patch_ids, int N, int T, int sms, const std::vector<int>& off,
                      const std::vector<int>& ent, ResidentLayout& L);
+
+// Streamed step (streamed.cu): many steps in one cooperative launch over a
+// node-tile plan whose tiles are all resident, one block each.
+struct StreamPlan {
+    int halo;                      // room for a tile's halo nodes
+    const int* halo_count;         // [ntiles]
+    const int* halo_id;            // [ntiles][halo] node ids, ascending
+    const unsigned* local;         // [nchunks][3][kTile] patch nodes, two to a word: index in the tile, or
+                                   // nodes + index in the halo
+    const unsigned char* border;   // [N] another tile reads this node
+    double* metric;                // [nchunks][6][kTile] abar, bbar of a launch that reads them from the arrays
+    ulonglong2* packets;           // as ResidentPlan::packets
+};
+struct StreamLayout {
+    int halo = 0;
+    std::vector<int> halo_count, halo_id;
+    std::vector<unsigned> local;
+    std::vector<unsigned char> border;
+};
+struct NodeTileLayout;
+void stream_layout(const NodeTileLayout& L, const int* patch_ids, int N, int NT, StreamLayout& S);
 
 // Layout of the per-(triangle, slot) force contributions: x, y, z doubles;
 // for the mixed path x, y, z floats, optionally padded with a zero to 16
@@ -399,6 +420,14 @@ cudaError_t launch_node_tiles(const DevMesh& m, const ClusterPlan& p, const Node
 // packets may have used last.
 cudaError_t prepare_resident(const ResidentPlan& q, int mixed, int* blocks_per_sm);
 cudaError_t launch_resident(const DevMesh& m, const ClusterPlan& p, const ResidentPlan& q, const DevState& s,
+                            const StepScalars& sc, int dial_mode, int mixed, int steps, unsigned tag0,
+                            cudaStream_t st);
+// Streamed step (streamed.cu): shared memory per block, blocks per SM it is
+// built for, kernel set-up, and the launch (as launch_resident).
+size_t stream_smem(size_t stride, int nodes, int halo, int mixed);
+int stream_blocks_target(int mixed);
+cudaError_t prepare_streamed(const NodeTilePlan& q, const StreamPlan& sp, int mixed, int* blocks_per_sm);
+cudaError_t launch_streamed(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp, const DevState& s,
                             const StepScalars& sc, int dial_mode, int mixed, int steps, unsigned tag0,
                             cudaStream_t st);
 // Largest cluster size (8, 4, 2, 1) whose clusters fill the most SMs, and the

@@ -179,7 +179,7 @@ bool node_tile_layout(const int* patch_ids, int N, int T, int NT, int mixed, con
     L.dst.assign(C, {});
     std::vector<int> slc_w(threads, 32);
     std::fill(bad.begin(), bad.end(), 0);
-    parallel_ranges(C, threads, [&](int c0, int c1, int w) {
+    if (sliced) parallel_ranges(C, threads, [&](int c0, int c1, int w) {
         std::vector<unsigned char> used;
         for (int c = c0; c < c1 && !bad[w]; ++c) {
             const auto& re = L.run_end[c];
@@ -228,7 +228,7 @@ bool node_tile_layout(const int* patch_ids, int N, int T, int NT, int mixed, con
         }
     L.slc_max = *std::max_element(slc_w.begin(), slc_w.end());
     L.fixed = tile_record_bytes(mixed);
-    L.sliced = sliced != 0;
+    L.sliced = sliced > 0;
     size_t ns_max_sliced = 16;
     L.bytes.assign(C, 0);
     std::vector<size_t> ns_w(threads, 16), nss_w(threads, 16);

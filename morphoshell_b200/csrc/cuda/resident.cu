@@ -45,12 +45,14 @@
 #include <climits>
 
 #include "internal.cuh"
+#include "packets.cuh"
 #include "step_common.cuh"
 #include "tri_contrib.cuh"
 
 namespace msb {
 namespace {
 
+using namespace packets;
 using namespace stepdev;
 using namespace tridev;
 
@@ -68,25 +70,6 @@ constexpr int kBatch = 8;      // of which this many are loaded together
 // 2.49 / 2.48 / 2.46 us, 32,219 triangles 3.57 / 3.49 / 3.40 / 3.38 / 3.35 /
 // 3.36 us.
 constexpr unsigned kFirstPoll = 500;
-
-__device__ __forceinline__ void put_packet(ulonglong2* p, double v, unsigned tag) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    const unsigned long long t = (unsigned long long)tag << 32;
-    const unsigned long long lo = (b & 0xffffffffULL) | t, hi = (b >> 32) | t;
-    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(lo), "l"(hi) : "memory");
-}
-
-__device__ __forceinline__ void get_packet(const ulonglong2* p, unsigned long long& lo, unsigned long long& hi) {
-    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
-}
-
-__device__ __forceinline__ bool packet_is(unsigned long long lo, unsigned long long hi, unsigned tag) {
-    return (unsigned)(lo >> 32) == tag && (unsigned)(hi >> 32) == tag;
-}
-
-__device__ __forceinline__ double packet_value(unsigned long long lo, unsigned long long hi) {
-    return __longlong_as_double((long long)((lo & 0xffffffffULL) | (hi << 32)));
-}
 
 template <int DIAL, bool MIXED, int TH>
 __global__ void __launch_bounds__(TH, 1)

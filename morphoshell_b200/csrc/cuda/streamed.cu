@@ -1,0 +1,452 @@
+// Streamed step: many fused steps in one launch, for meshes too large for the
+// resident step (resident.cu) whose tables still fit in L2.
+//
+// One block per node tile, three (FP64) or four (mixed) blocks per SM, every
+// tile's block resident for the whole launch.  A tile's positions and its
+// halo's, its velocities, mass terms and force accumulators stay in shared
+// memory; the triangles' tables stream from L2 in the node-tiled step's chunk
+// records (NodeTilePlan), the next chunk's -- across the step's end too -- while
+// the block adds up the current one's runs.  Positions are gathered from
+// shared memory by 16-bit local ids, and tiles exchange them as the resident
+// step does (packets.cuh; the same argument that no packet is overwritten
+// early holds, tile adjacency being the same).  Every node's contributions are
+// added in ascending triangle order from zero, with the arithmetic of the
+// other paths: the same bits.
+//
+// What bounds it: the SM, at 12 (FP64) or 16 warps: 2,100 clocks per chunk of
+// 128 triangles, of which FP64 takes half and shared-memory accesses two
+// thirds, plus a node phase and one exchange per step.  Per step, FP64 (mixed),
+// against the two-kernel step in graphs: 50,310 triangles 6.7 (6.3) us against
+// 11.1 (10.0), 72,364 8.8 (6.8) against 13.2 (11.0), 147,922 14.6 (11.7)
+// against 19.0 (15.9).  A component of a run per thread, four values ahead of
+// the adds, was slower (15.9 us): three times the entries' loads.
+//
+// The launch is cooperative; every wait is bounded; the state a launch starts
+// from stays untouched, and a step that trips the force guard is found by
+// running the launch's steps again one by one, as for the resident step.
+#include <algorithm>
+#include <climits>
+
+#include "internal.cuh"
+#include "node_tile_walk.cuh"
+#include "packets.cuh"
+#include "step_common.cuh"
+#include "tile_copy.cuh"
+#include "tri_contrib.cuh"
+
+namespace msb {
+namespace {
+
+using namespace packets;
+using namespace stepdev;
+using namespace tiles;
+using namespace tridev;
+
+constexpr int kPolls = 4;  // halo components a thread has under way together
+
+// Shared memory of a block: staging area, two node sections, then per node of
+// the tile accumulator, velocity (3 doubles each), dt / m and the damping
+// term, positions of the tile and its halo, flags.
+template <bool MIXED>
+struct StSmem {
+    static constexpr size_t stage = NtSmem<MIXED>::stage;
+    __host__ __device__ static size_t bytes(size_t stride, int nodes, int halo) {
+        return stage + 2 * NtSmem<MIXED>::ns_cap(stride) + 8 * (8 * (size_t)nodes + 3 * ((size_t)nodes + halo)) +
+               ((size_t)nodes + 15) / 16 * 16;
+    }
+};
+
+// Loads that pass L1 by (tables are read once per step) and stay in L2.
+__device__ __forceinline__ unsigned ld_l2(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_l2(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld_l2(const double* p) {
+    double v;
+    asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
+// Slot i's tables of chunk c: local patch ids (two to a word), weights, area,
+// and the director trigonometry or the metric in force (abar, bbar).
+template <int DIAL, bool MIXED>
+struct StTables {
+    using R = typename Real<MIXED>::T;
+    static constexpr int kMet = DIAL == DIAL_LCE ? 3 : 6;
+    unsigned lid[3];
+    R cf[24];
+    double area, met[kMet];
+
+    __device__ __forceinline__ void load(const NodeTilePlan& q, const StreamPlan& sp, int c, int i) {
+        using L = TileLayout<MIXED>;
+        const unsigned char* rec = q.rec + (size_t)c * q.stride;
+        const R* coef = reinterpret_cast<const R*>(rec + L::ids);
+        const double* aux = reinterpret_cast<const double*>(rec + L::ids + L::coef);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) lid[k] = ld_l2(sp.local + ((size_t)c * 3 + k) * kTile + i);
+#pragma unroll
+        for (int k = 0; k < 24; ++k) cf[k] = ld_l2(coef + k * kTile + i);
+        area = ld_l2(aux + i);
+#pragma unroll
+        for (int k = 0; k < kMet; ++k)
+            met[k] = DIAL == DIAL_LCE ? ld_l2(aux + (k + 1) * kTile + i)
+                                      : ld_l2(sp.metric + ((size_t)c * 6 + k) * kTile + i);
+    }
+};
+
+// The metric in force of every slot, field-major per chunk, for a launch that
+// reads abar and bbar from the arrays (they do not change while it runs).
+__global__ void k_stream_metric(const DevMesh m, const NodeTilePlan q, double* __restrict__ out) {
+    const int c = blockIdx.x, i = threadIdx.x;
+    const int t = q.chunk_tri[(size_t)c * kTile + i];
+    const size_t T = m.T;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        out[((size_t)c * 6 + k) * kTile + i] = t >= 0 ? m.abar[k * T + t] : 0.0;
+        out[((size_t)c * 6 + 3 + k) * kTile + i] = t >= 0 ? m.bbar[k * T + t] : 0.0;
+    }
+}
+
+template <int DIAL, bool MIXED>
+__global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
+    k_streamed(const DevMesh m, const NodeTilePlan q, const StreamPlan sp, const DevState s, const StepScalars sc,
+               int steps, unsigned tag0) {
+    using R = typename Real<MIXED>::T;
+    const int g0 = global_step(s.err, sc.step);
+    // An earlier launch tripped the guard or timed out: uniform over the grid.
+    if (stale(s.err, g0) || *((volatile const int*)&s.err->flag) == 5) return;
+    extern __shared__ __align__(128) unsigned char st_smem[];
+    __shared__ uint64_t bar;
+    const int NT = q.nodes, N = m.N, ld = NT + sp.halo;
+    const size_t ns_cap = NtSmem<MIXED>::ns_cap(q.stride);
+    R* stage = reinterpret_cast<R*>(st_smem);
+    unsigned char* nsec = st_smem + StSmem<MIXED>::stage;
+    double* acc = reinterpret_cast<double*>(nsec + 2 * ns_cap);  // [NT][3]
+    double* svel = acc + 3 * NT;                                 // [3][NT]
+    double* sk2 = svel + 3 * NT;
+    double* sdm = sk2 + NT;
+    double* spos = sdm + NT;                                     // [3][ld]: own nodes, then the halo
+    unsigned char* sflag = reinterpret_cast<unsigned char*>(spos + 3 * ld);  // 1: constrained, 2: others read it
+
+    const int b = blockIdx.x, i = threadIdx.x;
+    const int n0 = b * NT, nn = min(NT, N - n0), nh = __ldg(sp.halo_count + b);
+    const int* halo_id = sp.halo_id + (size_t)b * sp.halo;
+    const int c0 = __ldg(q.tile_chunk + b), c1 = __ldg(q.tile_chunk + b + 1);
+    const double* pos = pos_buf(s, sc.parity);
+    const double* vel = vel_buf(s, sc.parity);
+    if (i == 0) {
+        bar_init(&bar);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int j = i; j < nn; j += kTile) {
+        const double mass = __ldg(m.mass + n0 + j);
+        sk2[j] = sc.dt / mass;
+        // Gradient descent divides by damping m instead.
+        sdm[j] = sc.gd ? sc.damping * mass : -sc.damping * mass / sc.rho_hh;
+        sflag[j] = (__ldg(m.fixed + n0 + j) ? 1 : 0) | (__ldg(sp.border + n0 + j) ? 2 : 0);
+        for (int c = 0; c < 3; ++c) {
+            spos[c * ld + j] = pos[(size_t)c * N + n0 + j];
+            svel[c * NT + j] = vel[(size_t)c * N + n0 + j];
+            acc[3 * j + c] = 0.0;
+        }
+    }
+    for (int j = i; j < nh; j += kTile) {
+        const int n = __ldg(halo_id + j);
+        for (int c = 0; c < 3; ++c) spos[c * ld + NT + j] = pos[(size_t)c * N + n];
+    }
+    __syncthreads();
+    auto fetch = [&](int c, int slot) {
+        bulk_load(nsec + slot * ns_cap, q.rec + (size_t)c * q.stride + NtSmem<MIXED>::fixed,
+                  __ldg(q.chunk_bytes + c) - (uint32_t)NtSmem<MIXED>::fixed, &bar);
+    };
+    if (i == 0) fetch(c0, 0);
+    StTables<DIAL, MIXED> tb;
+    tb.load(q, sp, c0, i);
+    TriMat<double> mt;
+    mt.h = m.h_uniform;
+    mt.mu = m.mu_uniform;
+    mt.ks = m.ks_uniform;
+    mt.kb = m.kb_uniform;
+    mt.igmh = m.igmh_uniform;
+    double lam = 0.0, pw = 0.0;
+    if (DIAL == DIAL_LCE) {
+        lam = __ldg(s.dials + 3 * (size_t)g0 + 1);
+        pw = __ldg(s.dials + 3 * (size_t)g0 + 2);
+    }
+    uint32_t phase = 0u;
+    int slot = 0;
+    bool tripped = false;
+    double fmax = -1.0, vmax = -1.0;
+    int fnode = INT_MAX, vnode = INT_MAX;
+
+    for (int it = 0; it < steps; ++it) {
+        const bool last = it + 1 == steps;
+        for (int c = c0; c < c1; ++c) {
+            const int nc = c + 1 < c1 ? c + 1 : last ? -1 : c0;
+            // This barrier also ends the previous chunk's runs.
+            const int ok = __syncthreads_and(bar_wait(&bar, phase) ? 1 : 0);
+            phase ^= 1u;
+            if (!ok) {
+                if (i == 0) atomicCAS(&s.err->flag, 0, 5);  // MS_ERR_TIMEOUT; no other copy is in flight
+                return;
+            }
+            if (i == 0 && nc >= 0) fetch(nc, slot ^ 1);
+            const unsigned char* ns = nsec + slot * ns_cap;
+            const int4 hd = *reinterpret_cast<const int4*>(ns);  // R, E, ntri
+            if (i < hd.z) {
+                mt.area = tb.area;
+                if (DIAL == DIAL_LCE) {
+                    lce_metric(tb.met[0], tb.met[1], tb.met[2], __dmul_rn(lam, lam), pw, mt);
+                } else {
+                    constexpr int k = StTables<DIAL, MIXED>::kMet;  // 6
+                    mt.abar0 = tb.met[0];
+                    mt.abar1 = tb.met[1];
+                    mt.abar2 = tb.met[2];
+                    mt.bbar0 = tb.met[k - 3];
+                    mt.bbar1 = tb.met[k - 2];
+                    mt.bbar2 = tb.met[k - 1];
+                }
+                double P[6][3];
+#pragma unroll
+                for (int sl = 0; sl < 6; ++sl) {
+                    const unsigned id = sl & 1 ? tb.lid[sl / 2] >> 16 : tb.lid[sl / 2] & 0xffffu;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) P[sl][k] = spos[k * ld + id];
+                }
+                R f[18];
+                tri_forces<MIXED>(P, tb.cf, mt, m.nu, f);
+#pragma unroll
+                for (int k = 0; k < 18; ++k) stage[k * kTile + i] = f[k];
+            }
+            __syncthreads();
+            if (nc >= 0) tb.load(q, sp, nc, i);
+            // Runs, as in node_tile_walk.
+            const unsigned short* rn = reinterpret_cast<const unsigned short*>(ns + 16);
+            const unsigned short* re = rn + hd.x;
+            const unsigned short* en = re + hd.x;
+            for (int r = i; r < hd.x; r += kTile) {
+                const int j = rn[r] & ~kRunFinal;
+                int e = r ? re[r - 1] : 0;
+                const int e1 = re[r];
+                double a0 = acc[3 * j], a1 = acc[3 * j + 1], a2 = acc[3 * j + 2];
+                for (; e < e1; ++e) {
+                    const R* v = stage + en[e];
+                    a0 += (double)v[0];
+                    a1 += (double)v[kTile];
+                    a2 += (double)v[2 * kTile];
+                }
+                acc[3 * j] = a0;
+                acc[3 * j + 1] = a1;
+                acc[3 * j + 2] = a2;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            slot ^= 1;
+        }
+        __syncthreads();
+        if (DIAL == DIAL_LCE && !last) {
+            lam = __ldg(s.dials + 3 * (size_t)(g0 + it + 1) + 1);
+            pw = __ldg(s.dials + 3 * (size_t)(g0 + it + 1) + 2);
+        }
+        // The tile's nodes.
+        const unsigned tag = tag0 + (unsigned)it + 1u;
+        ulonglong2* pk = sp.packets + (tag & 1u) * 3 * (size_t)N;
+        for (int j = i; j < nn; j += kTile) {
+            const int flag = sflag[j];
+            double F[3], v[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                F[c] = acc[3 * j + c];
+                acc[3 * j + c] = 0.0;
+                v[c] = svel[c * NT + j];
+                if (!sc.gd) F[c] += sdm[j] * v[c];
+                if (flag & 1) F[c] = 0.0;
+                if (!(fabs(F[c]) < sc.force_limit) && !tripped) {
+                    tripped = true;
+                    record_guard(s, g0 + it, (long long)c * N + n0 + j);
+                }
+                double nv;
+                if (!sc.gd) nv = v[c] + sk2[j] * F[c];
+                else nv = sc.rho_hh * F[c] / sdm[j];
+                const double x = spos[c * ld + j] + sc.dt * nv;
+                if (last) {
+                    pos_buf(s, sc.parity ^ 1)[(size_t)c * N + n0 + j] = x;
+                    vel_buf(s, sc.parity ^ 1)[(size_t)c * N + n0 + j] = nv;
+                } else {
+                    svel[c * NT + j] = nv;
+                    spos[c * ld + j] = x;
+                    if (flag & 2) put_packet(pk + (size_t)c * N + n0 + j, x, tag);
+                }
+            }
+            if (sc.check && last) {
+                eq_merge(fmax, fnode, sqrt(F[0] * F[0] + F[1] * F[1] + F[2] * F[2]), n0 + j);
+                eq_merge(vmax, vnode, sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]), n0 + j);
+            }
+        }
+        if (last) break;
+        // Halo positions of the next step.
+        int ok = 1;
+        long long t0 = 0;
+        int spin = 0;
+        for (int k0 = i; ok && k0 < 3 * nh; k0 += kPolls * kTile) {
+            int src[kPolls], dst[kPolls];
+#pragma unroll
+            for (int u = 0; u < kPolls; ++u) {
+                const int k = k0 + u * kTile;
+                src[u] = -1;
+                dst[u] = 0;
+                if (k < 3 * nh) {
+                    const int c = k / nh, j = k - c * nh;
+                    src[u] = c * N + __ldg(halo_id + j);
+                    dst[u] = c * ld + NT + j;
+                }
+            }
+            for (;;) {
+                unsigned long long lo[kPolls], hi[kPolls];
+                bool wait = false;
+#pragma unroll
+                for (int u = 0; u < kPolls; ++u)
+                    if (src[u] >= 0) get_packet(pk + src[u], lo[u], hi[u]);
+#pragma unroll
+                for (int u = 0; u < kPolls; ++u)
+                    if (src[u] >= 0) {
+                        if (packet_is(lo[u], hi[u], tag)) {
+                            spos[dst[u]] = packet_value(lo[u], hi[u]);
+                            src[u] = -1;
+                        } else {
+                            wait = true;
+                        }
+                    }
+                if (!wait) break;
+                if (++spin == 64) t0 = clock64();
+                if (spin > 64 && clock64() - t0 > 2000000000LL) {
+                    ok = 0;
+                    break;
+                }
+            }
+        }
+        if (!__syncthreads_and(ok)) {
+            if (i == 0) {
+                atomicCAS(&s.err->flag, 0, 5);  // MS_ERR_TIMEOUT
+                bar_wait(&bar, phase);          // the next step's first node section is on its way
+            }
+            return;
+        }
+    }
+    if (sc.check) {
+        const EqPartial r = eq_block_reduce<kTile>(fmax, fnode, vmax, vnode);
+        eq_store_and_fold<kTile>(s, r, b, gridDim.x, gridDim.x);
+    }
+}
+
+template <int DIAL, bool MIXED>
+cudaError_t prepare_one(const NodeTilePlan& q, const StreamPlan& sp, int& blocks) {
+    const size_t smem = StSmem<MIXED>::bytes(q.stride, q.nodes, sp.halo);
+    cudaError_t e =
+        cudaFuncSetAttribute(k_streamed<DIAL, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int b = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_streamed<DIAL, MIXED>, kTile, smem);
+    blocks = std::min(blocks, b);
+    return e;
+}
+
+template <int DIAL, bool MIXED>
+cudaError_t launch_one(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp, const DevState& s,
+                       const StepScalars& sc, int steps, unsigned tag0, cudaStream_t st) {
+    if (DIAL != DIAL_LCE) {
+        k_stream_metric<<<q.nchunks, kTile, 0, st>>>(m, q, sp.metric);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    const size_t smem = StSmem<MIXED>::bytes(q.stride, q.nodes, sp.halo);
+    // The limit belongs to the function, not to a handle.
+    cudaError_t e =
+        cudaFuncSetAttribute(k_streamed<DIAL, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(q.ntiles);
+    cfg.blockDim = dim3(kTile);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_streamed<DIAL, MIXED>, m, q, sp, s, sc, steps, tag0);
+}
+
+}  // namespace
+
+void stream_layout(const NodeTileLayout& L, const int* patch, int N, int NT, StreamLayout& S) {
+    S = StreamLayout();
+    S.halo_count.assign(L.K, 0);
+    S.border.assign(N, 0);
+    S.local.assign((size_t)L.C * 3 * kTile, 0);
+    std::vector<std::vector<int>> halo(L.K);
+    std::vector<int> seen(N, -1), place(N, 0);
+    for (int k = 0; k < L.K; ++k) {
+        const int n0 = k * NT, n1 = std::min(N, n0 + NT);
+        std::vector<int>& h = halo[k];
+        for (long long x = L.start[k]; x < L.start[k + 1]; ++x)
+            for (int j = 0; j < 6; ++j) {
+                const int n = patch[6LL * L.lst[x] + j];
+                if ((n < n0 || n >= n1) && seen[n] != k) {
+                    seen[n] = k;
+                    h.push_back(n);
+                }
+            }
+        std::sort(h.begin(), h.end());
+        for (size_t j = 0; j < h.size(); ++j) {
+            place[h[j]] = NT + (int)j;
+            S.border[h[j]] = 1;
+        }
+        S.halo_count[k] = (int)h.size();
+        S.halo = std::max(S.halo, (int)h.size());
+        for (long long x = L.start[k]; x < L.start[k + 1]; ++x) {
+            const long long at = x - L.start[k];
+            const size_t c = (size_t)L.tile_chunk[k] + at / kTile, i = at % kTile;
+            for (int j = 0; j < 6; ++j) {
+                const int n = patch[6LL * L.lst[x] + j];
+                const unsigned id = (unsigned)(n >= n0 && n < n1 ? n - n0 : place[n]);
+                S.local[(c * 3 + j / 2) * kTile + i] |= id << (16 * (j & 1));
+            }
+        }
+    }
+    S.halo = std::max(S.halo, 1);
+    S.halo_id.assign((size_t)L.K * S.halo, 0);
+    for (int k = 0; k < L.K; ++k) std::copy(halo[k].begin(), halo[k].end(), S.halo_id.begin() + (size_t)k * S.halo);
+}
+
+size_t stream_smem(size_t stride, int nodes, int halo, int mixed) {
+    return mixed ? StSmem<true>::bytes(stride, nodes, halo) : StSmem<false>::bytes(stride, nodes, halo);
+}
+
+int stream_blocks_target(int mixed) { return mixed ? 4 : 3; }
+
+cudaError_t prepare_streamed(const NodeTilePlan& q, const StreamPlan& sp, int mixed, int* blocks_per_sm) {
+    int b = INT_MAX;
+    cudaError_t e = mixed ? prepare_one<DIAL_LCE, true>(q, sp, b) : prepare_one<DIAL_LCE, false>(q, sp, b);
+    if (e == cudaSuccess)
+        e = mixed ? prepare_one<DIAL_ARRAYS, true>(q, sp, b) : prepare_one<DIAL_ARRAYS, false>(q, sp, b);
+    *blocks_per_sm = e == cudaSuccess ? b : 0;
+    return e;
+}
+
+cudaError_t launch_streamed(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp, const DevState& s,
+                            const StepScalars& sc, int dial_mode, int mixed, int steps, unsigned tag0,
+                            cudaStream_t st) {
+    if (dial_mode == DIAL_LCE)
+        return mixed ? launch_one<DIAL_LCE, true>(m, q, sp, s, sc, steps, tag0, st)
+                     : launch_one<DIAL_LCE, false>(m, q, sp, s, sc, steps, tag0, st);
+    return mixed ? launch_one<DIAL_ARRAYS, true>(m, q, sp, s, sc, steps, tag0, st)
+                 : launch_one<DIAL_ARRAYS, false>(m, q, sp, s, sc, steps, tag0, st);
+}
+
+}  // namespace msb

@@ -1,5 +1,5 @@
-"""The resident step (many steps in one cooperative launch, the default on
-small meshes) against the two-kernel step -- GPU.
+"""The many-step kernels (resident on small meshes, streamed on mid-size
+ones; the default there) against the two-kernel step -- GPU.
 
 Both compute each triangle with the same arithmetic and sum every node's
 contributions in ascending triangle order from zero
@@ -40,10 +40,11 @@ def _equil(r):
     return e.max_force, e.max_speed, e.max_force_node, e.max_speed_node, e.at_equilibrium
 
 
-# disk250: a handful of tiles; disk100, disk50: 128 threads; disk18k: 256;
-# disk15: 384; disk14: near the largest mesh, disk11: too large for it.
+# Resident: disk250, a handful of tiles; disk100, disk50, 128 threads; disk18k,
+# 256; disk15, 384.  Streamed: disk14, the smallest; disk7; disk6, near the
+# largest in FP64; disk5, mixed only; disk4, too large for both.
 @pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("name", ["disk250", "disk100", "disk50", "disk18k", "disk15", "disk14", "disk11"])
+@pytest.mark.parametrize("name", ["disk250", "disk100", "disk50", "disk18k", "disk15", "disk14", "disk7", "disk6", "disk5", "disk4"])
 def test_resident_equals_two_kernel_bitwise(workdir, name, precision):
     m = make_model(workdir, name)
     s = m.scalars
@@ -62,14 +63,15 @@ def test_resident_equals_two_kernel_bitwise(workdir, name, precision):
     assert _same(ga, gb)
 
 
-def test_resident_more_than_one_launch_and_gradient_descent(workdir):
-    m = make_model(workdir, "disk100")
+@pytest.mark.parametrize("name,steps", [("disk100", 20001), ("disk12", 300)])
+def test_resident_more_than_one_launch_and_gradient_descent(workdir, name, steps):
+    m = make_model(workdir, name)
     s = m.scalars
     x, v = deformed_state(m, seed=42, amp=0.02)
     ga, gb = _pair(m)
     for g in (ga, gb):
         g.upload(x, v)
-        g.step_n(20001, 0.2 + 1e-7 * np.arange(20001), s.timestep, s.damping_factor_1)
+        g.step_n(steps, 0.2 + 1e-7 * np.arange(steps), s.timestep, s.damping_factor_1)
         g.do_dialling(0.2)
         g.step_n(7, None, 1e-3 * s.timestep, s.damping_factor_1, gd=True)
     assert _same(ga, gb)
@@ -105,13 +107,14 @@ def test_resident_other_metrics_and_constraints(workdir, tmp_path):
         assert _same(ga, gb)
 
 
+@pytest.mark.parametrize("name", ["disk18k", "disk10"])
 @pytest.mark.parametrize("at", [0, 3])
-def test_resident_guard(workdir, at):
+def test_resident_guard(workdir, at, name):
     """A trip of the force guard: the same step, dof, force and surviving
     state as the two-kernel step, at the first step and later (a node whose
     speed carries it away)."""
     from morphoshell_b200 import MsError
-    m = make_model(workdir, "disk18k")
+    m = make_model(workdir, name)
     s = m.scalars
     x, v = deformed_state(m, seed=44, amp=0.02)
     node = 2 * m.num_nodes + 4321
