@@ -321,6 +321,55 @@ __global__ void __launch_bounds__(kTile)
     }
 }
 
+// A stretch of steps in which nothing happens to any instance but steps
+// (streamed.cu): the protocol-3 values of step k of the stretch, as k_batch_pre
+// would form them, ...
+__global__ void k_batch_dials(const InstParams* __restrict__ ip, const InstState* __restrict__ is, int n, int steps,
+                              double2* __restrict__ out) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n * steps) return;
+    const int k = j / n, i = j - k * n;
+    const InstState& st = is[i];
+    const InstParams& p = ip[i];
+    double2 o = make_double2(st.cur_lam, st.cur_pw);
+    if (st.status == INST_DIALLING) {
+        double d = k == 0 ? st.dial_factor
+                          : st.last_equil_dial + p.spacing * ((double)(st.k_phase + k) / (double)p.steps_per_phase);
+        if (d >= 1.0) d = 1.0;
+        const double lam = (1.0 - d) * 1.0 + d * p.lam_final;
+        o = make_double2(lam, pow(lam, -2.0 * p.nu_ot));
+    }
+    out[j] = o;
+}
+
+// ... and the instances' counters after it, unless a node tripped the guard.
+__global__ void k_batch_advance(const InstParams* __restrict__ ip, InstState* __restrict__ is, int n, int steps,
+                                const double2* __restrict__ dials, const int* __restrict__ trip) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || *trip) return;
+    InstState st = is[i];
+    if (is_frozen(st.status)) return;
+    const InstParams& p = ip[i];
+    st.check_now = 0;
+    if (st.status == INST_DIALLING) {
+        const long long k = st.k_phase + steps - 1;
+        double d = steps == 1 ? st.dial_factor
+                              : st.last_equil_dial + p.spacing * ((double)k / (double)p.steps_per_phase);
+        if (d >= 1.0) d = 1.0;
+        const double2 o = dials[(size_t)(steps - 1) * n + i];
+        st.cur_dial = d;
+        st.cur_lam = o.x;
+        st.cur_pw = o.y;
+        st.k_phase += steps;
+    } else {
+        st.tsc += steps;
+    }
+    for (int k = 0; k < steps; ++k) st.time += p.dt;  // step by step: the same roundings
+    st.stepcount += steps;
+    st.dial_factor = st.last_equil_dial + p.spacing * ((double)st.k_phase / (double)p.steps_per_phase);
+    is[i] = st;
+}
+
 constexpr int kPostBlock = 256;
 
 __global__ void __launch_bounds__(kPostBlock) k_batch_post(const InstParams* __restrict__ ip,
@@ -433,6 +482,10 @@ using namespace msb;
 
 namespace {
 
+// Largest union tables of streamed stretches: a step there also saves two
+// launches around the force kernel.
+constexpr double kBatchStreamBytes = 80e6;
+
 struct BatchGraph {
     int len, parity, sched;
     cudaGraphExec_t exec;
@@ -465,6 +518,16 @@ struct ms_batch {
     int nt_blocks = 0;           // resident blocks per SM the node-tiled plan runs at
     std::string tune_report;     // the last autotune's trials, one per line
     std::vector<void*> nt_allocs;  // the node-tiled plan's device buffers (replaced by the autotuner)
+    // Streamed stretches (streamed.cu), on a plan of their own; until a
+    // schedule is asked for by number.
+    bool have_stream = false;
+    bool stream_on = true;
+    NodeTilePlan st_ntp{};
+    StreamPlan stp{};
+    BatchStream bst{};
+    double2* d_dials = nullptr;    // [kStretchDials]
+    int* d_trip = nullptr;
+    unsigned pk_tag = 0;           // tag of the last step published in packets
     int parity = 0;
     int sched = 0;
     int chunk = 64;
@@ -592,7 +655,7 @@ ms_status run_graph(ms_batch* b, int len, int parity, int sched) {
     e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     MB_CUDA(b, e);
-    if (b->graphs.size() >= 16) clear_graphs(b);
+    if (b->graphs.size() >= 32) clear_graphs(b);
     b->graphs.push_back({len, parity, sched, exec});
     MB_CUDA(b, cudaGraphLaunch(exec, b->stream));
     return MS_OK;
@@ -675,12 +738,6 @@ int batch_node_tile_blocks(int mixed, size_t smem) {
     return nb;
 }
 
-bool all_frozen(const ms_batch* b) {
-    for (int i = 0; i < b->n_inst; ++i)
-        if (b->h_is[i].status < INST_DONE) return false;
-    return true;
-}
-
 ms_status fetch_states(ms_batch* b) {
     if (!b->is_stale) return MS_OK;
     MB_CUDA(b, cudaMemcpyAsync(b->h_is, b->d_is, sizeof(InstState) * b->n_inst, cudaMemcpyDeviceToHost, b->stream));
@@ -690,6 +747,113 @@ ms_status fetch_states(ms_batch* b) {
     if (e) return bfail(b, MS_ERR_TIMEOUT, "a tile copy did not land within its bounded wait");
     b->is_stale = false;
     return MS_OK;
+}
+
+// Steps of a streamed stretch at most, and fewest worth one.
+constexpr int kStretchSteps = 4096;
+constexpr int kStretchMin = 8;
+constexpr int kStretchDials = 1 << 18;  // dial table entries (instances x steps)
+
+// The streamed plan of the union, where it is in that kernel's range.
+ms_status build_stream(ms_batch* b, const std::vector<int>& patch6, const std::vector<int>& node_inst,
+                       const std::vector<int>& off, const std::vector<int>& ent, int sms) {
+    const int N = b->m.N, T = b->m.T, mixed = b->precision == MS_PRECISION_MIXED;
+    int coop = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, b->device);
+    for (const InstParams& p : b->ip)
+        if (!p.uniform_hmu) return MS_OK;  // per-triangle materials take the general path
+    if (!coop || b->n_inst > kStretchDials / kStretchMin || stream_bytes(mixed, T) > kBatchStreamBytes) return MS_OK;
+    const int target = stream_blocks_target(mixed);
+    // Small unions: tiles of at least 32 nodes, on fewer SMs.
+    const int NT = std::max(32, (N + sms * target - 1) / (sms * target));
+    NodeTileLayout L;
+    std::string err;
+    if (!node_tile_layout(patch6.data(), N, T, NT, mixed, off, ent, L, err)) return bfail(b, MS_ERR_INVALID_ARGUMENT, err);
+    StreamLayout S;
+    stream_layout(L, patch6.data(), N, NT, S);
+    int insts = 1;
+    for (int k = 0; k < L.K; ++k)
+        insts = std::max(insts, node_inst[std::min(N, (k + 1) * NT) - 1] - node_inst[k * NT] + 1);
+    NodeTilePlan q{};
+    StreamPlan sp{};
+    q.stride = L.stride;
+    q.nodes = NT;
+    sp.halo = S.halo;
+    int blocks = 0;
+    if (stream_smem(L.stride, NT, S.halo, insts, mixed) > 227 * 1024 ||
+        prepare_streamed(q, sp, insts, mixed, &blocks) != cudaSuccess || (long long)blocks * sms < L.K) {
+        cudaGetLastError();
+        return MS_OK;
+    }
+    MB_TRY(plan_from_layout(b, L, NT, blocks, b->st_ntp, b->allocs));
+    int *d_count, *d_ids;
+    unsigned* d_local;
+    unsigned char* d_border;
+    MB_TRY(bupload(b, &d_count, S.halo_count));
+    MB_TRY(bupload(b, &d_ids, S.halo_id));
+    MB_TRY(bupload(b, &d_local, S.local));
+    MB_TRY(bupload(b, &d_border, S.border));
+    MB_TRY(balloc(b, &sp.packets, 6ULL * N));
+    MB_TRY(balloc(b, &b->d_dials, kStretchDials));
+    MB_TRY(balloc(b, &b->d_trip, 1));
+    MB_CUDA(b, cudaMemsetAsync(sp.packets, 0, 6ULL * N * sizeof(ulonglong2), b->stream));
+    sp.halo_count = d_count;
+    sp.halo_id = d_ids;
+    sp.local = d_local;
+    sp.border = d_border;
+    b->stp = sp;
+    b->bst.n_inst = b->n_inst;
+    b->bst.insts = insts;
+    b->bst.node_inst = b->d_node_inst;
+    b->bst.dials = b->d_dials;
+    b->bst.err = b->d_err;
+    b->bst.trip = b->d_trip;
+    b->have_stream = true;
+    return MS_OK;
+}
+
+// Steps from the mirrored states in which no instance reaches the end of its
+// dial phase or a check (k_batch_pre's conditions): at most `most`.
+int64_t quiet_steps(const ms_batch* b, int64_t most) {
+    for (int i = 0; i < b->n_inst; ++i) {
+        const InstState& st = b->h_is[i];
+        const InstParams& p = b->ip[i];
+        if (st.status == INST_DIALLING) most = std::min<int64_t>(most, p.steps_per_phase - st.k_phase);
+        else if (st.status == INST_WAITING) most = std::min<int64_t>(most, p.steps_between_checks - st.tsc + 1);
+        else if (st.status < INST_DONE) most = 0;
+    }
+    return std::max<int64_t>(most, 0);
+}
+
+// One streamed stretch of `steps` steps; *stood says whether it counts (no
+// node tripped the guard).
+ms_status run_stretch(ms_batch* b, int steps, bool* stood) {
+    const int n = b->n_inst;
+    cudaStream_t st = b->stream;
+    MB_CUDA(b, cudaMemsetAsync(b->d_trip, 0, sizeof(int), st));
+    k_batch_dials<<<(n * steps + 127) / 128, 128, 0, st>>>(b->d_ip, b->d_is, n, steps, b->d_dials);
+    MB_CUDA(b, cudaGetLastError());
+    BatchStream bs = b->bst;
+    bs.ip = b->d_ip;
+    bs.is = b->d_is;
+    MB_CUDA(b, launch_batch_streamed(b->m, b->st_ntp, b->stp, bs, b->s, b->parity, b->precision, steps, b->pk_tag,
+                                     st));
+    b->pk_tag += (unsigned)steps;
+    k_batch_advance<<<(n + 127) / 128, 128, 0, st>>>(b->d_ip, b->d_is, n, steps, b->d_dials, b->d_trip);
+    MB_CUDA(b, cudaGetLastError());
+    int trip = 0;
+    MB_CUDA(b, cudaMemcpyAsync(&trip, b->d_trip, sizeof(int), cudaMemcpyDeviceToHost, st));
+    b->is_stale = true;
+    MB_TRY(fetch_states(b));
+    *stood = trip == 0;
+    if (*stood) b->parity ^= 1;
+    return MS_OK;
+}
+
+bool all_frozen(const ms_batch* b) {
+    for (int i = 0; i < b->n_inst; ++i)
+        if (b->h_is[i].status < INST_DONE) return false;
+    return true;
 }
 
 // Instance i's state, on the device and in the mirror.
@@ -988,6 +1152,7 @@ ms_status ms_batch_create(const ms_batch_instance* inst, int32_t n, int32_t devi
         b->sched = (b->have_nt && b->ntp.ntiles >= b->ntp.grid) ? kSchedNodeTiles
                    : b->tile_grid > 0                         ? kSchedTiles
                                                               : kSchedAos;
+        if ((st = build_stream(b, patch6, node_inst, off, ent, sms))) return bail(st);
     }
     m.mass = d_mass;
     m.fixed = d_fixed;
@@ -1034,14 +1199,33 @@ ms_status ms_batch_run(ms_batch* b, int64_t max_steps, int64_t* steps_done) {
     cudaSetDevice(b->device);
     int64_t done = 0;
     MB_TRY(fetch_states(b));
+    const bool stream = b->have_stream && b->stream_on;
+    const int64_t stretch = std::min<int64_t>(kStretchSteps, kStretchDials / b->n_inst);
+    int64_t by_step = 0;  // steps to take one by one: a stretch whose guard tripped
     while (done < max_steps && !all_frozen(b)) {
-        const int len = (int)std::min<int64_t>(b->chunk, max_steps - done);
+        int64_t most = b->chunk;
+        if (stream) {
+            const int64_t quiet = quiet_steps(b, std::min(stretch, max_steps - done));
+            if (by_step <= 0 && quiet >= kStretchMin) {
+                bool stood = false;
+                MB_TRY(run_stretch(b, (int)quiet, &stood));
+                if (stood) done += quiet;
+                else by_step = quiet;
+                continue;
+            }
+            // Up to and including the step in which something happens.
+            if (by_step <= 0) most = std::min<int64_t>(most, quiet + 1);
+        }
+        const int len = (int)std::min<int64_t>(most, max_steps - done);
+        by_step -= len;
         b->is_stale = true;
         MB_TRY(run_graph(b, len, b->parity, b->sched));
         b->parity ^= len & 1;
         done += len;
         MB_TRY(fetch_states(b));
     }
+    // Steps go in chunks: those after the last instance stopped change nothing.
+    if (stream && all_frozen(b)) done = std::min(max_steps, (done + b->chunk - 1) / b->chunk * b->chunk);
     if (steps_done) *steps_done = done;
     return MS_OK;
 }
@@ -1139,6 +1323,7 @@ ms_status ms_batch_set_schedule(ms_batch* b, const ms_batch_schedule* s) {
             (s->tri_block >= 0 || b->have_nt)) {
             b->sched = k;
             b->chunk = s->chunk_steps;
+            b->stream_on = false;
             return MS_OK;
         }
     return bfail(b, MS_ERR_UNSUPPORTED, "no built-in schedule with these block sizes");

@@ -282,11 +282,6 @@ ms_status build_tiles(ms_handle* h, const ms_mesh_desc* d) {
 #define MSB_NT_NODES_MIXED 1008
 #endif
 constexpr int kNtNodesMin = 256;
-// Largest tables of the streamed step.  Per step against the default path's
-// graphs: FP64 147,922 triangles (38 MB) 14.6 us against 19.0, 290,073 (74 MB)
-// 27.3 against 28.7, 358,048 33.2 against 33.3; mixed 358,048 (57 MB) 22.9
-// against 28.8.
-constexpr double kStreamBytes = 60e6;
 // Largest nodes per tile of the warp-specialised step (one block per SM): its
 // shared memory holds two table buffers, two staging areas, eight node
 // sections and the prefetched node state besides the accumulators, and tiles
@@ -367,8 +362,8 @@ ms_status build_node_tiles(ms_handle* h, const ms_mesh_desc* d, const std::vecto
         q.stride = L.stride;
         q.nodes = NT;
         sp.halo = S.halo;
-        stream = stream_smem(L.stride, NT, S.halo, mixed) <= 227 * 1024 &&
-                 prepare_streamed(q, sp, mixed, &b) == cudaSuccess && (long long)b * sms >= L.K;
+        stream = stream_smem(L.stride, NT, S.halo, 0, mixed) <= 227 * 1024 &&
+                 prepare_streamed(q, sp, 0, mixed, &b) == cudaSuccess && (long long)b * sms >= L.K;
         cudaGetLastError();
         blocks = stream ? tile_blocks(tile_smem(L, NT)) : 0;
         stream = stream && blocks > 0;
@@ -506,8 +501,7 @@ ms_status build_resident(ms_handle* h, const ms_mesh_desc* d, const std::vector<
 bool stream_range(const ms_handle* h, int N, int T) {
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device);
-    const double per_tri = h->precision == MS_PRECISION_MIXED ? 160.0 : 256.0;
-    return coop && N >= 8192 && per_tri * T <= kStreamBytes;
+    return coop && N >= 8192 && stream_bytes(h->precision == MS_PRECISION_MIXED, T) <= kStreamBytes;
 }
 
 ms_status build_streamed(ms_handle* h, const StreamLayout& S) {

@@ -326,6 +326,19 @@ struct InstState {
     unsigned long long guard_key;      // smallest tripping dof (within the instance) of this step, ~0 if none
 };
 
+// A stretch of batch steps in the streamed kernel: steps in which no instance
+// changes its status or checks.
+struct BatchStream {
+    int n_inst;
+    int insts;                  // most instances of a tile
+    const int* node_inst;       // [N]
+    const InstParams* ip;
+    const InstState* is;
+    const double2* dials;       // [steps][n_inst] lambda, lambda^(-2 nu_ot)
+    int* err;                   // 5 (MS_ERR_TIMEOUT) when a wait ran out
+    int* trip;                  // 1 when a node tripped the force guard: the stretch does not count
+};
+
 struct DevState {
     double* pos[2];
     double* vel[2];
@@ -423,13 +436,23 @@ cudaError_t launch_resident(const DevMesh& m, const ClusterPlan& p, const Reside
                             const StepScalars& sc, int dial_mode, int mixed, int steps, unsigned tag0,
                             cudaStream_t st);
 // Streamed step (streamed.cu): shared memory per block, blocks per SM it is
-// built for, kernel set-up, and the launch (as launch_resident).
-size_t stream_smem(size_t stride, int nodes, int halo, int mixed);
+// built for, kernel set-up, and the launch (as launch_resident).  insts: the
+// most instances a tile's nodes belong to (batch), 0 for a single mesh.
+size_t stream_smem(size_t stride, int nodes, int halo, int insts, int mixed);
 int stream_blocks_target(int mixed);
-cudaError_t prepare_streamed(const NodeTilePlan& q, const StreamPlan& sp, int mixed, int* blocks_per_sm);
+cudaError_t prepare_streamed(const NodeTilePlan& q, const StreamPlan& sp, int insts, int mixed, int* blocks_per_sm);
 cudaError_t launch_streamed(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp, const DevState& s,
                             const StepScalars& sc, int dial_mode, int mixed, int steps, unsigned tag0,
                             cudaStream_t st);
+cudaError_t launch_batch_streamed(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp,
+                                  const BatchStream& bs, const DevState& s, int parity, int mixed, int steps,
+                                  unsigned tag0, cudaStream_t st);
+// Largest tables of the streamed step.  Per step against the default path's
+// graphs: FP64 147,922 triangles (38 MB) 14.6 us against 19.0, 290,073 (74 MB)
+// 27.3 against 28.7, 358,048 33.2 against 33.3; mixed 358,048 (57 MB) 22.9
+// against 28.8.
+constexpr double kStreamBytes = 60e6;
+constexpr double stream_bytes(int mixed, double tris) { return (mixed ? 160.0 : 256.0) * tris; }
 // Largest cluster size (8, 4, 2, 1) whose clusters fill the most SMs, and the
 // CTA shape used with it.
 int choose_cluster_size(int tpc, int threads, int mixed);

@@ -24,6 +24,12 @@
 // The launch is cooperative; every wait is bounded; the state a launch starts
 // from stays untouched, and a step that trips the force guard is found by
 // running the launch's steps again one by one, as for the resident step.
+//
+// The batch runs stretches of steps in which no instance changes its status or
+// checks for equilibrium the same way (BATCH): the union is the mesh, a tile
+// keeps its instances' scalars in shared memory, and their dial values of
+// every step come from a table.  Done and failed instances' triangles and
+// nodes are left alone, except that their nodes keep publishing.
 #include <algorithm>
 #include <climits>
 
@@ -47,12 +53,19 @@ constexpr int kPolls = 4;  // halo components a thread has under way together
 // Shared memory of a block: staging area, two node sections, then per node of
 // the tile accumulator, velocity (3 doubles each), dt / m and the damping
 // term, positions of the tile and its halo, flags.
+// For the batch: its instances' scalars, and each node's instance.
+struct StInst {
+    double ks, kb, igmh, nu, dt, force_limit;
+    double lam[2], pw[2];  // of this step and the next, by the step's parity
+    int frozen;
+};
 template <bool MIXED>
 struct StSmem {
     static constexpr size_t stage = NtSmem<MIXED>::stage;
-    __host__ __device__ static size_t bytes(size_t stride, int nodes, int halo) {
+    __host__ __device__ static size_t bytes(size_t stride, int nodes, int halo, int insts) {
         return stage + 2 * NtSmem<MIXED>::ns_cap(stride) + 8 * (8 * (size_t)nodes + 3 * ((size_t)nodes + halo)) +
-               ((size_t)nodes + 15) / 16 * 16;
+               ((size_t)nodes + 15) / 16 * 16 +
+               (insts ? sizeof(StInst) * (size_t)insts + ((size_t)nodes * 2 + 15) / 16 * 16 : 0);
     }
 };
 
@@ -82,6 +95,7 @@ struct StTables {
     unsigned lid[3];
     R cf[24];
     double area, met[kMet];
+    int tag;  // the slot's instance (batch)
 
     __device__ __forceinline__ void load(const NodeTilePlan& q, const StreamPlan& sp, int c, int i) {
         using L = TileLayout<MIXED>;
@@ -97,6 +111,7 @@ struct StTables {
         for (int k = 0; k < kMet; ++k)
             met[k] = DIAL == DIAL_LCE ? ld_l2(aux + (k + 1) * kTile + i)
                                       : ld_l2(sp.metric + ((size_t)c * 6 + k) * kTile + i);
+        tag = q.chunk_tag ? __ldg(q.chunk_tag + (size_t)c * kTile + i) : 0;
     }
 };
 
@@ -113,14 +128,18 @@ __global__ void k_stream_metric(const DevMesh m, const NodeTilePlan q, double* _
     }
 }
 
-template <int DIAL, bool MIXED>
+template <int DIAL, bool MIXED, bool BATCH>
 __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
-    k_streamed(const DevMesh m, const NodeTilePlan q, const StreamPlan sp, const DevState s, const StepScalars sc,
-               int steps, unsigned tag0) {
+    k_streamed(const DevMesh m, const NodeTilePlan q, const StreamPlan sp, const BatchStream bs, const DevState s,
+               const StepScalars sc, int steps, unsigned tag0) {
     using R = typename Real<MIXED>::T;
-    const int g0 = global_step(s.err, sc.step);
-    // An earlier launch tripped the guard or timed out: uniform over the grid.
-    if (stale(s.err, g0) || *((volatile const int*)&s.err->flag) == 5) return;
+    int g0 = 0;
+    if constexpr (!BATCH) {
+        g0 = global_step(s.err, sc.step);
+        // An earlier launch tripped the guard or timed out: uniform over the grid.
+        if (stale(s.err, g0) || *((volatile const int*)&s.err->flag) == 5) return;
+    }
+    int* err_flag = BATCH ? bs.err : &s.err->flag;
     extern __shared__ __align__(128) unsigned char st_smem[];
     __shared__ uint64_t bar;
     const int NT = q.nodes, N = m.N, ld = NT + sp.halo;
@@ -132,7 +151,10 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
     double* sk2 = svel + 3 * NT;
     double* sdm = sk2 + NT;
     double* spos = sdm + NT;                                     // [3][ld]: own nodes, then the halo
-    unsigned char* sflag = reinterpret_cast<unsigned char*>(spos + 3 * ld);  // 1: constrained, 2: others read it
+    // 1: constrained, 2: others read it, 4: its instance is done or failed.
+    unsigned char* sflag = reinterpret_cast<unsigned char*>(spos + 3 * ld);
+    StInst* sinst = reinterpret_cast<StInst*>(sflag + (NT + 15) / 16 * 16);
+    unsigned short* sni = reinterpret_cast<unsigned short*>(sinst + bs.insts);  // [NT] node's instance in sinst
 
     const int b = blockIdx.x, i = threadIdx.x;
     const int n0 = b * NT, nn = min(NT, N - n0), nh = __ldg(sp.halo_count + b);
@@ -144,12 +166,42 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
         bar_init(&bar);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    int i_lo = 0, i_n = 0;
+    if constexpr (BATCH) {
+        i_lo = __ldg(bs.node_inst + n0);
+        i_n = __ldg(bs.node_inst + n0 + nn - 1) - i_lo + 1;
+        for (int k = i; k < i_n; k += kTile) {
+            const InstParams& p = bs.ip[i_lo + k];
+            StInst& o = sinst[k];
+            o.ks = p.ks;
+            o.kb = p.kb;
+            o.igmh = p.igmh;
+            o.nu = p.nu;
+            o.dt = p.dt;
+            o.force_limit = p.force_limit;
+            o.frozen = bs.is[i_lo + k].status >= INST_DONE;
+            const double2 d = __ldg(bs.dials + i_lo + k);
+            o.lam[0] = d.x;
+            o.pw[0] = d.y;
+        }
+    }
     for (int j = i; j < nn; j += kTile) {
         const double mass = __ldg(m.mass + n0 + j);
-        sk2[j] = sc.dt / mass;
-        // Gradient descent divides by damping m instead.
-        sdm[j] = sc.gd ? sc.damping * mass : -sc.damping * mass / sc.rho_hh;
-        sflag[j] = (__ldg(m.fixed + n0 + j) ? 1 : 0) | (__ldg(sp.border + n0 + j) ? 2 : 0);
+        int frozen = 0;
+        if constexpr (BATCH) {
+            const int inst = __ldg(bs.node_inst + n0 + j);
+            const InstParams& p = bs.ip[inst];
+            const double damping = bs.is[inst].damping;
+            sni[j] = (unsigned short)(inst - i_lo);
+            sk2[j] = p.dt / mass;
+            sdm[j] = -damping * mass / p.rho_hh;
+            frozen = bs.is[inst].status >= INST_DONE ? 4 : 0;
+        } else {
+            sk2[j] = sc.dt / mass;
+            // Gradient descent divides by damping m instead.
+            sdm[j] = sc.gd ? sc.damping * mass : -sc.damping * mass / sc.rho_hh;
+        }
+        sflag[j] = (__ldg(m.fixed + n0 + j) ? 1 : 0) | (__ldg(sp.border + n0 + j) ? 2 : 0) | frozen;
         for (int c = 0; c < 3; ++c) {
             spos[c * ld + j] = pos[(size_t)c * N + n0 + j];
             svel[c * NT + j] = vel[(size_t)c * N + n0 + j];
@@ -174,8 +226,8 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
     mt.ks = m.ks_uniform;
     mt.kb = m.kb_uniform;
     mt.igmh = m.igmh_uniform;
-    double lam = 0.0, pw = 0.0;
-    if (DIAL == DIAL_LCE) {
+    double lam = 0.0, pw = 0.0, nu = m.nu;
+    if (DIAL == DIAL_LCE && !BATCH) {
         lam = __ldg(s.dials + 3 * (size_t)g0 + 1);
         pw = __ldg(s.dials + 3 * (size_t)g0 + 2);
     }
@@ -193,13 +245,26 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
             const int ok = __syncthreads_and(bar_wait(&bar, phase) ? 1 : 0);
             phase ^= 1u;
             if (!ok) {
-                if (i == 0) atomicCAS(&s.err->flag, 0, 5);  // MS_ERR_TIMEOUT; no other copy is in flight
+                if (i == 0) atomicCAS(err_flag, 0, 5);  // MS_ERR_TIMEOUT; no other copy is in flight
                 return;
             }
             if (i == 0 && nc >= 0) fetch(nc, slot ^ 1);
             const unsigned char* ns = nsec + slot * ns_cap;
             const int4 hd = *reinterpret_cast<const int4*>(ns);  // R, E, ntri
-            if (i < hd.z) {
+            bool live = i < hd.z;
+            if constexpr (BATCH) {
+                // The chunk's triangles are of the tile's instances: each
+                // touches one of its nodes.
+                const StInst& o = sinst[live ? tb.tag - i_lo : 0];
+                live = live && !o.frozen;
+                mt.ks = o.ks;
+                mt.kb = o.kb;
+                mt.igmh = o.igmh;
+                nu = o.nu;
+                lam = o.lam[it & 1];
+                pw = o.pw[it & 1];
+            }
+            if (live) {
                 mt.area = tb.area;
                 if (DIAL == DIAL_LCE) {
                     lce_metric(tb.met[0], tb.met[1], tb.met[2], __dmul_rn(lam, lam), pw, mt);
@@ -220,7 +285,7 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
                     for (int k = 0; k < 3; ++k) P[sl][k] = spos[k * ld + id];
                 }
                 R f[18];
-                tri_forces<MIXED>(P, tb.cf, mt, m.nu, f);
+                tri_forces<MIXED>(P, tb.cf, mt, nu, f);
 #pragma unroll
                 for (int k = 0; k < 18; ++k) stage[k * kTile + i] = f[k];
             }
@@ -249,7 +314,15 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
             slot ^= 1;
         }
         __syncthreads();
-        if (DIAL == DIAL_LCE && !last) {
+        if constexpr (BATCH) {
+            if (!last)
+                for (int k = i; k < i_n; k += kTile) {
+                    const double2 d = __ldg(bs.dials + (size_t)(it + 1) * bs.n_inst + i_lo + k);
+                    sinst[k].lam[(it + 1) & 1] = d.x;
+                    sinst[k].pw[(it + 1) & 1] = d.y;
+                }
+        }
+        if (DIAL == DIAL_LCE && !BATCH && !last) {
             lam = __ldg(s.dials + 3 * (size_t)(g0 + it + 1) + 1);
             pw = __ldg(s.dials + 3 * (size_t)(g0 + it + 1) + 2);
         }
@@ -258,6 +331,12 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
         ulonglong2* pk = sp.packets + (tag & 1u) * 3 * (size_t)N;
         for (int j = i; j < nn; j += kTile) {
             const int flag = sflag[j];
+            double dt = sc.dt, limit = sc.force_limit;
+            if constexpr (BATCH) {
+                const StInst& o = sinst[sni[j]];
+                dt = o.dt;
+                limit = o.force_limit;
+            }
             double F[3], v[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
@@ -266,22 +345,26 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
                 v[c] = svel[c * NT + j];
                 if (!sc.gd) F[c] += sdm[j] * v[c];
                 if (flag & 1) F[c] = 0.0;
-                if (!(fabs(F[c]) < sc.force_limit) && !tripped) {
-                    tripped = true;
-                    record_guard(s, g0 + it, (long long)c * N + n0 + j);
+                double x = spos[c * ld + j];
+                if (!BATCH || !(flag & 4)) {
+                    if (!(fabs(F[c]) < limit) && !tripped) {
+                        tripped = true;
+                        if constexpr (BATCH) atomicExch(bs.trip, 1);
+                        else record_guard(s, g0 + it, (long long)c * N + n0 + j);
+                    }
+                    double nv;
+                    if (!sc.gd) nv = v[c] + sk2[j] * F[c];
+                    else nv = sc.rho_hh * F[c] / sdm[j];
+                    x += dt * nv;
+                    if (last) {
+                        pos_buf(s, sc.parity ^ 1)[(size_t)c * N + n0 + j] = x;
+                        vel_buf(s, sc.parity ^ 1)[(size_t)c * N + n0 + j] = nv;
+                    } else {
+                        svel[c * NT + j] = nv;
+                        spos[c * ld + j] = x;
+                    }
                 }
-                double nv;
-                if (!sc.gd) nv = v[c] + sk2[j] * F[c];
-                else nv = sc.rho_hh * F[c] / sdm[j];
-                const double x = spos[c * ld + j] + sc.dt * nv;
-                if (last) {
-                    pos_buf(s, sc.parity ^ 1)[(size_t)c * N + n0 + j] = x;
-                    vel_buf(s, sc.parity ^ 1)[(size_t)c * N + n0 + j] = nv;
-                } else {
-                    svel[c * NT + j] = nv;
-                    spos[c * ld + j] = x;
-                    if (flag & 2) put_packet(pk + (size_t)c * N + n0 + j, x, tag);
-                }
+                if (!last && (flag & 2)) put_packet(pk + (size_t)c * N + n0 + j, x, tag);
             }
             if (sc.check && last) {
                 eq_merge(fmax, fnode, sqrt(F[0] * F[0] + F[1] * F[1] + F[2] * F[2]), n0 + j);
@@ -332,7 +415,7 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
         }
         if (!__syncthreads_and(ok)) {
             if (i == 0) {
-                atomicCAS(&s.err->flag, 0, 5);  // MS_ERR_TIMEOUT
+                atomicCAS(err_flag, 0, 5);  // MS_ERR_TIMEOUT
                 bar_wait(&bar, phase);          // the next step's first node section is on its way
             }
             return;
@@ -344,30 +427,30 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
     }
 }
 
-template <int DIAL, bool MIXED>
-cudaError_t prepare_one(const NodeTilePlan& q, const StreamPlan& sp, int& blocks) {
-    const size_t smem = StSmem<MIXED>::bytes(q.stride, q.nodes, sp.halo);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_streamed<DIAL, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int DIAL, bool MIXED, bool BATCH>
+cudaError_t prepare_one(const NodeTilePlan& q, const StreamPlan& sp, int insts, int& blocks) {
+    const size_t smem = StSmem<MIXED>::bytes(q.stride, q.nodes, sp.halo, insts);
+    cudaError_t e = cudaFuncSetAttribute(k_streamed<DIAL, MIXED, BATCH>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int b = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_streamed<DIAL, MIXED>, kTile, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_streamed<DIAL, MIXED, BATCH>, kTile, smem);
     blocks = std::min(blocks, b);
     return e;
 }
 
-template <int DIAL, bool MIXED>
-cudaError_t launch_one(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp, const DevState& s,
-                       const StepScalars& sc, int steps, unsigned tag0, cudaStream_t st) {
+template <int DIAL, bool MIXED, bool BATCH>
+cudaError_t launch_one(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp, const BatchStream& bs,
+                       const DevState& s, const StepScalars& sc, int steps, unsigned tag0, cudaStream_t st) {
     if (DIAL != DIAL_LCE) {
         k_stream_metric<<<q.nchunks, kTile, 0, st>>>(m, q, sp.metric);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    const size_t smem = StSmem<MIXED>::bytes(q.stride, q.nodes, sp.halo);
+    const size_t smem = StSmem<MIXED>::bytes(q.stride, q.nodes, sp.halo, bs.insts);
     // The limit belongs to the function, not to a handle.
-    cudaError_t e =
-        cudaFuncSetAttribute(k_streamed<DIAL, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_streamed<DIAL, MIXED, BATCH>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(q.ntiles);
@@ -379,7 +462,7 @@ cudaError_t launch_one(const DevMesh& m, const NodeTilePlan& q, const StreamPlan
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_streamed<DIAL, MIXED>, m, q, sp, s, sc, steps, tag0);
+    return cudaLaunchKernelEx(&cfg, k_streamed<DIAL, MIXED, BATCH>, m, q, sp, bs, s, sc, steps, tag0);
 }
 
 }  // namespace
@@ -424,17 +507,24 @@ void stream_layout(const NodeTileLayout& L, const int* patch, int N, int NT, Str
     for (int k = 0; k < L.K; ++k) std::copy(halo[k].begin(), halo[k].end(), S.halo_id.begin() + (size_t)k * S.halo);
 }
 
-size_t stream_smem(size_t stride, int nodes, int halo, int mixed) {
-    return mixed ? StSmem<true>::bytes(stride, nodes, halo) : StSmem<false>::bytes(stride, nodes, halo);
+size_t stream_smem(size_t stride, int nodes, int halo, int insts, int mixed) {
+    return mixed ? StSmem<true>::bytes(stride, nodes, halo, insts) : StSmem<false>::bytes(stride, nodes, halo, insts);
 }
 
 int stream_blocks_target(int mixed) { return mixed ? 4 : 3; }
 
-cudaError_t prepare_streamed(const NodeTilePlan& q, const StreamPlan& sp, int mixed, int* blocks_per_sm) {
+cudaError_t prepare_streamed(const NodeTilePlan& q, const StreamPlan& sp, int insts, int mixed, int* blocks_per_sm) {
     int b = INT_MAX;
-    cudaError_t e = mixed ? prepare_one<DIAL_LCE, true>(q, sp, b) : prepare_one<DIAL_LCE, false>(q, sp, b);
-    if (e == cudaSuccess)
-        e = mixed ? prepare_one<DIAL_ARRAYS, true>(q, sp, b) : prepare_one<DIAL_ARRAYS, false>(q, sp, b);
+    cudaError_t e;
+    if (insts > 0) {
+        e = mixed ? prepare_one<DIAL_LCE, true, true>(q, sp, insts, b)
+                  : prepare_one<DIAL_LCE, false, true>(q, sp, insts, b);
+    } else {
+        e = mixed ? prepare_one<DIAL_LCE, true, false>(q, sp, 0, b) : prepare_one<DIAL_LCE, false, false>(q, sp, 0, b);
+        if (e == cudaSuccess)
+            e = mixed ? prepare_one<DIAL_ARRAYS, true, false>(q, sp, 0, b)
+                      : prepare_one<DIAL_ARRAYS, false, false>(q, sp, 0, b);
+    }
     *blocks_per_sm = e == cudaSuccess ? b : 0;
     return e;
 }
@@ -442,11 +532,21 @@ cudaError_t prepare_streamed(const NodeTilePlan& q, const StreamPlan& sp, int mi
 cudaError_t launch_streamed(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp, const DevState& s,
                             const StepScalars& sc, int dial_mode, int mixed, int steps, unsigned tag0,
                             cudaStream_t st) {
+    const BatchStream no{};
     if (dial_mode == DIAL_LCE)
-        return mixed ? launch_one<DIAL_LCE, true>(m, q, sp, s, sc, steps, tag0, st)
-                     : launch_one<DIAL_LCE, false>(m, q, sp, s, sc, steps, tag0, st);
-    return mixed ? launch_one<DIAL_ARRAYS, true>(m, q, sp, s, sc, steps, tag0, st)
-                 : launch_one<DIAL_ARRAYS, false>(m, q, sp, s, sc, steps, tag0, st);
+        return mixed ? launch_one<DIAL_LCE, true, false>(m, q, sp, no, s, sc, steps, tag0, st)
+                     : launch_one<DIAL_LCE, false, false>(m, q, sp, no, s, sc, steps, tag0, st);
+    return mixed ? launch_one<DIAL_ARRAYS, true, false>(m, q, sp, no, s, sc, steps, tag0, st)
+                 : launch_one<DIAL_ARRAYS, false, false>(m, q, sp, no, s, sc, steps, tag0, st);
+}
+
+cudaError_t launch_batch_streamed(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp,
+                                  const BatchStream& bs, const DevState& s, int parity, int mixed, int steps,
+                                  unsigned tag0, cudaStream_t st) {
+    StepScalars sc{};
+    sc.parity = parity;
+    return mixed ? launch_one<DIAL_LCE, true, true>(m, q, sp, bs, s, sc, steps, tag0, st)
+                 : launch_one<DIAL_LCE, false, true>(m, q, sp, bs, s, sc, steps, tag0, st);
 }
 
 }  // namespace msb

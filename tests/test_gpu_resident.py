@@ -131,3 +131,60 @@ def test_resident_guard(workdir, at, name):
         got.append((r.error_step, r.offending_dof, r.offending_force, r.steps_done) + tuple(map(bytes, g.download())))
     assert got[0] == got[1]
     assert (got[0][0] == 0) == (at == 0)
+
+
+def _batch_members(tmp_path, ks, **kw):
+    from morphoshell_b200 import ensemble
+    # Short dial phases and loose thresholds: whole runs in a few thousand steps.
+    fast = dict(dial_factors_to_hold_at_spacing=0.5, dial_phase_time_prefactor=0.02,
+                force_to_char_force_ratio_equil_threshold=1e-5, speed_to_char_speed_ratio_equil_threshold=1e-4)
+    return ensemble.build_members(ks, str(tmp_path), threads=4, **dict(fast, **kw))[0]
+
+
+def _batch_state(b):
+    out = []
+    for i in range(b.n):
+        s = b.status(i)
+        out.append((s.status, s.equilibria, s.stepcount, s.dial_factor, s.last_equil_dial, s.sim_time, s.max_force_ratio,
+                    s.max_speed_ratio, s.max_force_node, s.max_speed_node, s.offending_dof)
+                   + tuple(map(bytes, b.download(i))))
+    return out
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batch_stretches_equal_step_by_step(tmp_path, precision):
+    """Streamed stretches of a batch against its two-kernel schedule: from the
+    start through dial phases, checks, one instance reaching its final
+    equilibrium and one failing on the guard; the same states and step
+    counts at every stop."""
+    from morphoshell_b200 import MS_INST_DONE, MS_INST_FAILED, Batch
+    models = _batch_members(tmp_path, [12, 13, 14], spacing_range=(0.07, 0.1))
+    bad = models[2].dofs(1).copy()
+    vel = np.zeros_like(bad)
+    vel[2 * models[2].num_nodes + 5] = 10.0 / models[2].scalars.timestep
+    a, b = Batch(models, precision=precision), Batch(models, precision=precision)
+    b.set_schedule(0, 256, 64)
+    for g in (a, b):
+        g.upload(2, bad, vel)
+    for steps in (1, 7, 100, 1001, 20_000, 400_000):
+        assert a.run(steps) == b.run(steps)
+        assert _batch_state(a) == _batch_state(b)
+    assert a.status(2).status == MS_INST_FAILED
+    assert a.status(0).status == MS_INST_DONE and a.status(1).status == MS_INST_DONE
+
+
+@pytest.mark.parametrize("ks,lo,hi", [([3], 0.02, 0.021), ([3, 4, 5, 6, 7, 8], 0.012, 0.02), (list(range(40)), 0.08, 0.1)])
+def test_batch_stretches_many_sizes(tmp_path, ks, lo, hi):
+    """One instance, several per SM, and tiles of several instances; from the
+    start and from warm starts in both kinds of phase."""
+    from morphoshell_b200 import Batch
+    models = _batch_members(tmp_path, ks, spacing_range=(lo, hi))
+    a, b = Batch(models), Batch(models)
+    b.set_schedule(0, 256, 64)
+    for g in (a, b):
+        for i, m in enumerate(models):
+            if i % 3:
+                g.upload(i, *deformed_state(m, seed=50 + i, amp=0.02))
+                g.set_start(i, 0.52 if i % 3 == 1 else 1.0, i % 3 == 2)
+    assert a.run(700) == b.run(700)
+    assert _batch_state(a) == _batch_state(b)
