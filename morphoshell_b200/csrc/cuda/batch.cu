@@ -518,8 +518,8 @@ struct ms_batch {
     int nt_blocks = 0;           // resident blocks per SM the node-tiled plan runs at
     std::string tune_report;     // the last autotune's trials, one per line
     std::vector<void*> nt_allocs;  // the node-tiled plan's device buffers (replaced by the autotuner)
-    // Streamed stretches (streamed.cu), on a plan of their own; until a
-    // schedule is asked for by number.
+    // Streamed stretches (streamed.cu), on a plan that the autotuner leaves in
+    // place; until a schedule is asked for by number.
     bool have_stream = false;
     bool stream_on = true;
     NodeTilePlan st_ntp{};
@@ -1138,21 +1138,31 @@ ms_status ms_batch_create(const ms_batch_instance* inst, int32_t n, int32_t devi
         std::string err;
         int NT = 0, blocks = 0;
         auto smem_for = [&](const NodeTileLayout& lay, int nodes) { return node_tile_smem(lay.stride, nodes, mixed); };
-        if (!choose_node_tiles(patch6.data(), (int)N, (int)T, mixed, sms, mixed ? MSB_NT_MINB_MIXED : MSB_NT_MINB,
-                               mixed ? 1008 : 1100, 256, off, ent, smem_for, blocks_for, L, NT, blocks, err))
-            return bail(bfail(b, MS_ERR_INVALID_ARGUMENT, err));
-        if (blocks > 0) {
-            if ((st = plan_from_layout(b, L, NT, blocks, b->ntp, b->nt_allocs))) return bail(st);
-            b->nt_blocks = blocks;
-            b->have_nt = true;
+        // One plan serves streamed stretches and the node-tiled schedule where
+        // the union is in the former's range.
+        if ((st = build_stream(b, patch6, node_inst, off, ent, sms))) return bail(st);
+        int tiles_of_own = 0;  // node tiles of at least 256 nodes
+        if (b->have_stream) {
+            b->ntp = b->st_ntp;
+            blocks = blocks_for(node_tile_smem(b->ntp.stride, b->ntp.nodes, mixed));
+            b->ntp.grid = sms * blocks;
+            tiles_of_own = ((int)N + 255) / 256;
+        } else {
+            if (!choose_node_tiles(patch6.data(), (int)N, (int)T, mixed, sms,
+                                   mixed ? MSB_NT_MINB_MIXED : MSB_NT_MINB, mixed ? 1008 : 1100, 256, off, ent, smem_for,
+                                   blocks_for, L, NT, blocks, err))
+                return bail(bfail(b, MS_ERR_INVALID_ARGUMENT, err));
+            if (blocks > 0 && (st = plan_from_layout(b, L, NT, blocks, b->ntp, b->nt_allocs))) return bail(st);
+            tiles_of_own = b->ntp.ntiles;
         }
+        b->nt_blocks = blocks;
+        b->have_nt = blocks > 0;
         // The one-kernel step once every block has a tile of its own
         // (measured fastest on B200 for the single-mesh step), else the
         // tile kernel, else the per-triangle kernel.
-        b->sched = (b->have_nt && b->ntp.ntiles >= b->ntp.grid) ? kSchedNodeTiles
+        b->sched = (b->have_nt && tiles_of_own >= b->ntp.grid) ? kSchedNodeTiles
                    : b->tile_grid > 0                         ? kSchedTiles
                                                               : kSchedAos;
-        if ((st = build_stream(b, patch6, node_inst, off, ent, sms))) return bail(st);
     }
     m.mass = d_mass;
     m.fixed = d_fixed;
