@@ -1157,12 +1157,11 @@ ms_status ms_batch_create(const ms_batch_instance* inst, int32_t n, int32_t devi
         }
         b->nt_blocks = blocks;
         b->have_nt = blocks > 0;
-        // The one-kernel step once every block has a tile of its own
-        // (measured fastest on B200 for the single-mesh step), else the
+        // The one-kernel step once the blocks have a tile each, else the
         // tile kernel, else the per-triangle kernel.
-        b->sched = (b->have_nt && tiles_of_own >= b->ntp.grid) ? kSchedNodeTiles
-                   : b->tile_grid > 0                         ? kSchedTiles
-                                                              : kSchedAos;
+        b->sched = (b->have_nt && tiles_fill_grid(tiles_of_own, b->ntp.grid)) ? kSchedNodeTiles
+                   : b->tile_grid > 0                                        ? kSchedTiles
+                                                                             : kSchedAos;
     }
     m.mass = d_mass;
     m.fixed = d_fixed;

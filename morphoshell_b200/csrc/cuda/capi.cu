@@ -419,11 +419,11 @@ ms_status build_node_tiles(ms_handle* h, const ms_mesh_desc* d, const std::vecto
     h->have_ntiles = q.grid > 0;
     h->have_pipe = q.grid_pipe > 0;
     if (stream) MS_TRY(build_streamed(h, S));
-    // The node-tiled kernels once every block has a tile of its own (same
-    // bits as paths 1 and 2); the warp-specialised one when its plan was
-    // asked for.
+    // The node-tiled kernels once the blocks have a tile each (same bits as
+    // paths 1 and 2); the warp-specialised one when its plan was asked for.
     if (h->have_pipe && K >= q.grid_pipe) h->step_path = 4;
-    else if (h->have_ntiles && (stream ? (N + kNtNodesMin - 1) / kNtNodesMin : K) >= q.grid) h->step_path = 3;
+    else if (h->have_ntiles && tiles_fill_grid(stream ? (N + kNtNodesMin - 1) / kNtNodesMin : K, q.grid))
+        h->step_path = 3;
     return MS_OK;
 }
 

@@ -213,6 +213,15 @@ bool choose_node_tiles(const int* patch_ids, int N, int T, int mixed, int sms, i
                        const std::function<size_t(const NodeTileLayout&, int)>& smem_for,
                        const std::function<int(size_t)>& blocks_for, NodeTileLayout& L, int& NT, int& blocks,
                        std::string& err, int sliced = 0);
+// Whether a plan's tiles fill the grid, one tile to a block: the node-tiled
+// kernel is then the fastest of the one-step kernels.  A tile count chosen for
+// one tile a block comes out a few short of the grid, since the tiles are of
+// whole nodes (443 of 444, 739 of 740), so the line lies at nine tenths; asked
+// for all of the grid, half of the meshes between one and two tiles a block
+// took the two-kernel step.  Two kernels against this one, us per step
+// dialling: 290k triangles FP64 43.0 against 28.4; mixed, 453k 42.9 against
+// 32.9, 754k 62.4 against 48.5.
+inline bool tiles_fill_grid(int tiles, int grid) { return 10LL * tiles >= 9LL * grid; }
 // The chunk records of a layout (ids from patch_ids [T][6]; weights from
 // coef_d [T][24] double, or coef_f float for the mixed path when given; the
 // trigonometry block from aux4 [T][4] = area, cos^2, sin^2, cos sin, or

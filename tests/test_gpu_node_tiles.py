@@ -161,6 +161,14 @@ def test_node_tile_plan_balances_blocks(workdir):
         assert nt == 256 or tiles % blocks == 0 or tiles % blocks > 0.9 * blocks
 
 
+@pytest.mark.parametrize("name,precision", [("disk5", 0), ("disk4", 1)])
+def test_one_tile_a_block_takes_the_node_tiled_step(workdir, name, precision):
+    """A plan of one tile a block whose count is a tile or two short of the
+    resident blocks (tiles are of whole nodes) is the default step."""
+    from morphoshell_b200 import GpuLoop
+    assert GpuLoop(make_model(workdir, name), precision=precision).plan_info()["path"] == 3
+
+
 def test_prepared_graphs_give_the_same_steps(workdir):
     """ms_prepare_steps builds the graphs of a later ms_step_n call and runs
     nothing: the state is untouched, and the prepared call gives the bits of
