@@ -188,3 +188,54 @@ def test_batch_stretches_many_sizes(tmp_path, ks, lo, hi):
                 g.set_start(i, 0.52 if i % 3 == 1 else 1.0, i % 3 == 2)
     assert a.run(700) == b.run(700)
     assert _batch_state(a) == _batch_state(b)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batch_node_tiled_stretches_equal_step_by_step(tmp_path, precision):
+    """Quiet stretches of the node-tiled schedule (one launch a step) against
+    the two-kernel schedule: lengths around the shortest stretch and the
+    longest, dial phases, checks, an instance that fails inside a stretch while
+    the others go on, one that failed before, and a warm start in each kind of
+    phase."""
+    from morphoshell_b200 import MS_INST_DONE, MS_INST_FAILED, Batch
+    models = _batch_members(tmp_path, [12, 13, 14, 15], spacing_range=(0.07, 0.1))
+    bad = models[2].dofs(1).copy()
+    vel = np.zeros_like(bad)
+    vel[2 * models[2].num_nodes + 5] = 10.0 / models[2].scalars.timestep
+    warm = deformed_state(models[3], seed=53, amp=0.02)
+    a, b = Batch(models, precision=precision), Batch(models, precision=precision)
+    a.set_schedule(-1, 0, 64)
+    b.set_schedule(0, 256, 64)
+    for g in (a, b):
+        g.upload(3, *warm)
+        g.set_start(3, 0.52, True)
+    for steps in (1, 7, 8, 9, 300, 1001):
+        assert a.run(steps) == b.run(steps)
+        assert _batch_state(a) == _batch_state(b)
+    for g in (a, b):
+        g.upload(2, bad, vel)
+    for steps in (100, 20_000, 400_000):
+        assert a.run(steps) == b.run(steps)
+        assert _batch_state(a) == _batch_state(b)
+    assert a.status(2).status == MS_INST_FAILED
+    assert a.status(0).status == MS_INST_DONE and a.status(1).status == MS_INST_DONE
+
+
+@pytest.mark.parametrize("sched", [None, (-1, 0)])
+def test_batch_steps_reported_when_the_last_instance_fails(tmp_path, sched):
+    """A run ends with the chunk of the step at which its last instance fails,
+    with and without a stretch before that step."""
+    from morphoshell_b200 import MS_INST_FAILED, Batch
+    # An unstable timestep: both fail, one sooner.
+    models = _batch_members(tmp_path, [12, 13], spacing_range=(0.07, 0.1), timestep_prefactor=1.7)
+    out = []
+    for choice in (sched, (0, 256)):
+        g = Batch(models)
+        if choice is not None:
+            g.set_schedule(*choice, 64)
+        for i, m in enumerate(models):
+            g.upload(i, *deformed_state(m, seed=50 + i, amp=(1e-6, 1e-2)[i]))
+        done = [g.run(10), g.run(3000)]
+        assert all(g.status(i).status == MS_INST_FAILED for i in range(2))
+        out.append((done, _batch_state(g)))
+    assert out[0] == out[1]
