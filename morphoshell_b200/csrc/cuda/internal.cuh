@@ -456,11 +456,14 @@ cudaError_t launch_streamed(const DevMesh& m, const NodeTilePlan& q, const Strea
 cudaError_t launch_batch_streamed(const DevMesh& m, const NodeTilePlan& q, const StreamPlan& sp,
                                   const BatchStream& bs, const DevState& s, int parity, int mixed, int steps,
                                   unsigned tag0, cudaStream_t st);
-// Largest tables of the streamed step.  Per step against the default path's
-// graphs: FP64 147,922 triangles (38 MB) 14.6 us against 19.0, 290,073 (74 MB)
-// 27.3 against 28.7, 358,048 33.2 against 33.3; mixed 358,048 (57 MB) 22.9
-// against 28.8.
-constexpr double kStreamBytes = 60e6;
+// Largest tables of the streamed step; above, they no longer stay in L2 from
+// one step to the next.  us per step, dialling (waiting), against the
+// node-tiled step in graphs: FP64 268,146 triangles (69 MB) 24.8 (23.7) against
+// 26.9 (26.6), 342,658 (88 MB) 30.4 (28.9) against 32.7 (32.6), but 374,412
+// (96 MB) 42.0 against 33.7; mixed 342,658 (55 MB) 22.6 against 28.6, 411,150
+// (66 MB) 29.6 (30.6) against 31.2 (32.4); the mixed blocks of larger meshes do
+// not fit.
+constexpr double kStreamBytes = 88e6;
 constexpr double stream_bytes(int mixed, double tris) { return (mixed ? 160.0 : 256.0) * tris; }
 // Largest cluster size (8, 4, 2, 1) whose clusters fill the most SMs, and the
 // CTA shape used with it.

@@ -304,6 +304,48 @@ bool choose_node_tiles(const int* patch_ids, int N, int T, int mixed, int sms, i
     return true;
 }
 
+void stream_layout(const NodeTileLayout& L, const int* patch, int N, int NT, StreamLayout& S) {
+    S = StreamLayout();
+    S.halo_count.assign(L.K, 0);
+    S.border.assign(N, 0);
+    S.local.assign((size_t)L.C * 3 * kTile, 0);
+    std::vector<std::vector<int>> halo(L.K);
+    parallel_ranges(L.K, plan_threads(L.C), [&](int k0, int k1, int) {
+        std::vector<int> seen(N, -1), place(N, 0);
+        for (int k = k0; k < k1; ++k) {
+            const int n0 = k * NT, n1 = std::min(N, n0 + NT);
+            std::vector<int>& h = halo[k];
+            for (long long x = L.start[k]; x < L.start[k + 1]; ++x)
+                for (int j = 0; j < 6; ++j) {
+                    const int n = patch[6LL * L.lst[x] + j];
+                    if ((n < n0 || n >= n1) && seen[n] != k) {
+                        seen[n] = k;
+                        h.push_back(n);
+                    }
+                }
+            std::sort(h.begin(), h.end());
+            for (size_t j = 0; j < h.size(); ++j) place[h[j]] = NT + (int)j;
+            for (long long x = L.start[k]; x < L.start[k + 1]; ++x) {
+                const long long at = x - L.start[k];
+                const size_t c = (size_t)L.tile_chunk[k] + at / kTile, i = at % kTile;
+                for (int j = 0; j < 6; ++j) {
+                    const int n = patch[6LL * L.lst[x] + j];
+                    const unsigned id = (unsigned)(n >= n0 && n < n1 ? n - n0 : place[n]);
+                    S.local[(c * 3 + j / 2) * kTile + i] |= id << (16 * (j & 1));
+                }
+            }
+        }
+    });
+    for (int k = 0; k < L.K; ++k) S.halo = std::max(S.halo, (int)halo[k].size());
+    S.halo = std::max(S.halo, 1);
+    S.halo_id.assign((size_t)L.K * S.halo, 0);
+    for (int k = 0; k < L.K; ++k) {
+        S.halo_count[k] = (int)halo[k].size();
+        std::copy(halo[k].begin(), halo[k].end(), S.halo_id.begin() + (size_t)k * S.halo);
+        for (int n : halo[k]) S.border[n] = 1;
+    }
+}
+
 // Chunk c's node section (header, runs, entries and, for a sliced layout,
 // the sliced order) at dst, which holds zeros.
 void write_node_section(const NodeTileLayout& L, int c, int ntri, unsigned char* dst) {

@@ -467,46 +467,6 @@ cudaError_t launch_one(const DevMesh& m, const NodeTilePlan& q, const StreamPlan
 
 }  // namespace
 
-void stream_layout(const NodeTileLayout& L, const int* patch, int N, int NT, StreamLayout& S) {
-    S = StreamLayout();
-    S.halo_count.assign(L.K, 0);
-    S.border.assign(N, 0);
-    S.local.assign((size_t)L.C * 3 * kTile, 0);
-    std::vector<std::vector<int>> halo(L.K);
-    std::vector<int> seen(N, -1), place(N, 0);
-    for (int k = 0; k < L.K; ++k) {
-        const int n0 = k * NT, n1 = std::min(N, n0 + NT);
-        std::vector<int>& h = halo[k];
-        for (long long x = L.start[k]; x < L.start[k + 1]; ++x)
-            for (int j = 0; j < 6; ++j) {
-                const int n = patch[6LL * L.lst[x] + j];
-                if ((n < n0 || n >= n1) && seen[n] != k) {
-                    seen[n] = k;
-                    h.push_back(n);
-                }
-            }
-        std::sort(h.begin(), h.end());
-        for (size_t j = 0; j < h.size(); ++j) {
-            place[h[j]] = NT + (int)j;
-            S.border[h[j]] = 1;
-        }
-        S.halo_count[k] = (int)h.size();
-        S.halo = std::max(S.halo, (int)h.size());
-        for (long long x = L.start[k]; x < L.start[k + 1]; ++x) {
-            const long long at = x - L.start[k];
-            const size_t c = (size_t)L.tile_chunk[k] + at / kTile, i = at % kTile;
-            for (int j = 0; j < 6; ++j) {
-                const int n = patch[6LL * L.lst[x] + j];
-                const unsigned id = (unsigned)(n >= n0 && n < n1 ? n - n0 : place[n]);
-                S.local[(c * 3 + j / 2) * kTile + i] |= id << (16 * (j & 1));
-            }
-        }
-    }
-    S.halo = std::max(S.halo, 1);
-    S.halo_id.assign((size_t)L.K * S.halo, 0);
-    for (int k = 0; k < L.K; ++k) std::copy(halo[k].begin(), halo[k].end(), S.halo_id.begin() + (size_t)k * S.halo);
-}
-
 size_t stream_smem(size_t stride, int nodes, int halo, int insts, int mixed) {
     return mixed ? StSmem<true>::bytes(stride, nodes, halo, insts) : StSmem<false>::bytes(stride, nodes, halo, insts);
 }

@@ -41,8 +41,8 @@ def _equil(r):
 
 
 # Resident: disk250, a handful of tiles; disk100, disk50, 128 threads; disk18k,
-# 256; disk15, 384.  Streamed: disk14, the smallest; disk7; disk6, near the
-# largest in FP64; disk5, mixed only; disk4, too large for both.
+# 256; disk15, 384.  Streamed: disk14, the smallest; disk7; disk6; disk5, near
+# the largest in both precisions; disk4, too large for both.
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("name", ["disk250", "disk100", "disk50", "disk18k", "disk15", "disk14", "disk7", "disk6", "disk5", "disk4"])
 def test_resident_equals_two_kernel_bitwise(workdir, name, precision):
