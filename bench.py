@@ -291,8 +291,14 @@ def workload_config(args, model):
 
 KERNEL_NAMES = {"cluster": ("k_cluster_step", "k_halo_update"), "two-kernel": ("k_tri_aos", "k_node_update"),
                 "tiles": ("k_tri_tiles", "k_node_update"), "node-tiles": ("k_node_tiles", None),
-                "node-pipe": ("k_node_pipe", None)}
+                "node-pipe": ("k_node_pipe", None), "many-step": ("k_resident or k_streamed (per step)", None)}
 PATH_IDS = {"cluster": 0, "two-kernel": 1, "tiles": 2, "node-tiles": 3, "node-pipe": 4}
+
+
+def many_steps_per_launch(model, precision):
+    """The default path takes whole calls in one cooperative launch where the
+    triangles' tables stay in L2 (the library's own line)."""
+    return model.num_tris * (160.0 if precision == "mixed" else 256.0) <= 88e6
 
 
 def timed_steps(model, info, bbar, precision, path, args, dials, local, dist, clock=None, setup=None):
@@ -310,6 +316,7 @@ def timed_steps(model, info, bbar, precision, path, args, dials, local, dist, cl
     g = GpuLoop(model, precision=prec, device=local)
     if setup is not None:
         setup["device_s"] = time.perf_counter() - t0
+    many = path == "auto" and many_steps_per_launch(model, precision)
     if path != "auto":
         g.set_step_path(PATH_IDS[path])
     path = {v: k for k, v in PATH_IDS.items()}[g.plan_info()["path"]]
@@ -342,6 +349,8 @@ def timed_steps(model, info, bbar, precision, path, args, dials, local, dist, cl
     x, v = g.download()
     t_tri, t_node = g.time_kernels(50, dial=float(dials[args.warmup]), dt=dt, damping=damp)
     g.upload(x, v)
+    if many:
+        path, t_tri = "many-step", ms_max / args.steps
     tri_name, node_name = KERNEL_NAMES[path]
     kernel_ms = {tri_name: t_tri} if node_name is None else {tri_name: t_tri, node_name: t_node}
     return g, ms_max, kernel_ms, path
@@ -369,6 +378,8 @@ def roofline(model, precision, path, workload, kernel_ms, step_ms):
 
 
 def launches(path, steps):
+    if path == "many-step":
+        return 1 + (max(0, steps - 128) + 8191) // 8192  # 128 steps, then up to 8,192
     per_step = 1 if KERNEL_NAMES[path][1] is None else 2
     return per_step * steps + (steps + 127) // 128  # + one chunk-end kernel per captured graph of 128 steps
 
@@ -606,7 +617,7 @@ def ensemble_measurement(n: int, precision: str, warmup: int, steps: int, local:
     peak, peak_kind = measured_peak_hbm()
     sizes = [p["num_tris"] for p in params]
     if sched["tri_block"] < 0:
-        kernels, per_step = "k_batch_pre + k_batch_node_tiles + k_batch_post (node-tiled schedule)", 3
+        kernels, per_step = "k_batch_node_tiles (node-tiled schedule, quiet stretches)", 1
     elif sched["tri_block"] == 0:
         kernels, per_step = "k_batch_pre + k_batch_tri_tiles + k_batch_node + k_batch_post (tiled schedule)", 4
     else:
