@@ -157,7 +157,7 @@ ms_status ms_advance_dynamics(ms_handle* h, double timestep, double damping_fact
  * ref_thickness, ref_shear_modulus T, abar and bbar 3T (all in the
  * ms_mesh_desc / row-major layouts above), dofs and forces 3N SoA.  Work
  * space is a static device array inside this library, sized for at most
- * 65,536 nodes and 65,536 triangles (about 13 MB that every GPU loading
+ * 65,536 nodes and 65,536 triangles (about 16 MB that every GPU loading
  * the library keeps until exit); larger meshes return
  * MS_ERR_INVALID_ARGUMENT with the reason in err.  Every call looks up that
  * array's device address in the current context (cudaGetSymbolAddress; the

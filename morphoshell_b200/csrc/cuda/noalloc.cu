@@ -12,22 +12,25 @@
 // device memory.
 //
 // Scratch: one file-scope __device__ array sized for meshes of up to
-// kMaxTris triangles and kMaxNodes nodes (about 13 MB, held by every GPU
+// kMaxTris triangles and kMaxNodes nodes (about 16 MB, held by every GPU
 // that loads the library until the process exits).  Larger meshes are
 // rejected.  Every call shares the array and it keeps the last call's
 // contents, so two calls that overlap on the GPU (different streams, or
 // different host threads on the same device) race and corrupt each other;
-// serialise them.  The chains' heads are cleared at the start of every call.
+// serialise them.  The nodes' counts are cleared at the start of every call.
 //
-// The node sums are deterministic: a node's entries are chained as they come
-// (one atomic exchange each), sorted by triangle when the node is summed, and
-// added in ascending triangle order, as in the main path.
+// The node sums are deterministic: a node's entries are listed as they come
+// (one atomic add each), sorted by triangle when the node is summed, and added
+// in ascending triangle order, as in the main path.
 //
-// Two kernels: k_na_tri (chains, and the triangles' contributions) and
-// k_na_gather (sort and sum).  What bounds them: a node's walk along its
-// chain, about 12 dependent trips to L2, and the tables' one trip from HBM.
-// Incidence lists built by counting, a one-block scan, filling and sorting
-// were five more launches; a call for 50,310 triangles took 114 us, now 53.
+// Two kernels: k_na_tri (lists, and the triangles' contributions) and
+// k_na_gather (sort and sum).  What bounds them: the tables' one trip from HBM,
+// and a node's three dependent trips to L2 (count, entries, contributions).
+// Per call for 50,310 triangles: incidence lists built by counting, a one-block
+// scan, filling and sorting in five more launches 114 us; entries chained, a
+// dozen dependent trips along a chain, 53; listed, and the triangles' weights
+// in flight together, 43.
+#include <climits>
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
@@ -39,14 +42,18 @@ namespace {
 
 constexpr int kMaxTris = 65536;
 constexpr int kMaxNodes = 65536;
+constexpr int kListed = 32;          // entries of a node listed, and sorted in shared memory, at most
+constexpr int kLists = 12 * 65536;   // room for the lists: kLists / N entries of a node (23 at T = 2 N = kMaxTris)
 
 struct Scratch {
     double contrib[kMaxTris * 18];  // per (triangle, slot) force contribution
-    int next[kMaxTris * 6];         // entry 6 t + slot: its chain's next entry + 1, or 0
-    int entries[kMaxTris * 6];      // sorted entries of the nodes with long chains
+    int list[kLists];               // [entry of the node][N] 6 t + slot, in the order of arrival
+    int next[kMaxTris * 6];         // entry 6 t + slot beyond a full list: its chain's next entry + 1, or 0
+    int entries[kMaxTris * 6];      // sorted entries of the nodes with chains
     int bad;                        // patch ids outside [0, num_nodes) seen this call
     int used;                       // of entries
-    int head[kMaxNodes];            // a node's first entry + 1, or 0 (bad, used and head are cleared every call)
+    int2 node[kMaxNodes];           // a node's entries, and its chain's first entry + 1, or 0 (bad, used and node are
+                                    // cleared every call)
 };
 
 static __device__ __align__(256) unsigned char ms_noalloc_scratch[sizeof(Scratch)];
@@ -64,7 +71,8 @@ cudaError_t scratch_address(Scratch** out) {
 
 constexpr int kTriBlock = 128;
 constexpr int kNodeBlock = 64;
-constexpr int kListed = 32;  // entries of a node sorted in shared memory
+
+__host__ __device__ inline int listed(int N) { return kListed < kLists / N ? kListed : kLists / N; }
 
 __global__ void __launch_bounds__(kTriBlock)
     k_na_tri(Scratch* s, int N, int T, const int* __restrict__ patch, const double* __restrict__ coef,
@@ -77,27 +85,47 @@ __global__ void __launch_bounds__(kTriBlock)
     __shared__ double rows[kTriBlock * 24];
     const int t0 = blockIdx.x * kTriBlock, i = threadIdx.x, t = t0 + i;
     const int live = min(kTriBlock, T - t0);
-    for (int e = i; e < 24 * live; e += kTriBlock) rows[e] = coef[24 * (size_t)t0 + e];
-    __syncthreads();
-    double c[24], f[18];
+    // All of them on their way at once (8 bytes each: the caller's array has a
+    // double's alignment), past the node lists and the positions.
+    for (int e = i; e < 24 * live; e += kTriBlock)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(rows + e)),
+                     "l"(coef + 24 * (size_t)t0 + e)
+                     : "memory");
+    double c[24], f[18], P[6][3];
+    TriMat<double> m;
     if (i < live) {
-        double P[6][3];
-#pragma unroll
-        for (int k = 0; k < 24; ++k) c[k] = rows[24 * i + k];
+        const int slots = listed(N);
+        m.abar0 = abar[3 * (size_t)t];
+        m.abar1 = abar[3 * (size_t)t + 1];
+        m.abar2 = abar[3 * (size_t)t + 2];
+        m.bbar0 = bbar[3 * (size_t)t];
+        m.bbar1 = bbar[3 * (size_t)t + 1];
+        m.bbar2 = bbar[3 * (size_t)t + 2];
+        m.h = thick[t];
+        m.mu = shear[t];
+        m.area = area[t];
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
             int id = patch[6 * (size_t)t + k];
             if (id < 0 || id >= N) {
-                // Reported; never read out of range, on no chain.
+                // Reported; never read out of range, on no list.
                 atomicAdd(&s->bad, 1);
                 id = 0;
             } else {
-                s->next[6 * t + k] = atomicExch(&s->head[id], 6 * t + k + 1);
+                const int at = atomicAdd(&s->node[id].x, 1);
+                if (at < slots) s->list[(size_t)at * N + id] = 6 * t + k;
+                else s->next[6 * t + k] = atomicExch(&s->node[id].y, 6 * t + k + 1);
             }
             P[k][0] = dofs[id];
             P[k][1] = dofs[(size_t)N + id];
             P[k][2] = dofs[2 * (size_t)N + id];
         }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (i < live) {
+#pragma unroll
+        for (int k = 0; k < 24; ++k) c[k] = rows[24 * i + k];
         double rx[3], ry[3], rxx[3], rxy[3], ryy[3];
         for (int d = 0; d < 3; ++d) {
             rx[d] = c[0] * P[0][d] + c[1] * P[1][d] + c[2] * P[2][d];
@@ -118,17 +146,7 @@ __global__ void __launch_bounds__(kTriBlock)
         q.rxx = {rxx[0], rxx[1], rxx[2]};
         q.rxy = {rxy[0], rxy[1], rxy[2]};
         q.ryy = {ryy[0], ryy[1], ryy[2]};
-        TriMat<double> m;
-        m.abar0 = abar[3 * (size_t)t];
-        m.abar1 = abar[3 * (size_t)t + 1];
-        m.abar2 = abar[3 * (size_t)t + 2];
-        m.bbar0 = bbar[3 * (size_t)t];
-        m.bbar1 = bbar[3 * (size_t)t + 1];
-        m.bbar2 = bbar[3 * (size_t)t + 2];
-        m.h = thick[t];
-        m.mu = shear[t];
         material_coefs(m.h, m.mu, nu, gamma, m.ks, m.kb, m.igmh);
-        m.area = area[t];
         CqGrad<double> g;
         energy_gradient<double>(q, m, nu, g);
 #pragma unroll
@@ -160,36 +178,76 @@ __global__ void __launch_bounds__(kNodeBlock) k_na_gather(Scratch* s, int N, dou
     __shared__ int list[kListed][kNodeBlock];
     const int n = blockIdx.x * kNodeBlock + threadIdx.x, i = threadIdx.x;
     if (n >= N) return;
-    // The chain in descending order, by insertion while it is walked (a chain
-    // starts with what came last, mostly the highest triangle).
-    int count = 0;
-    for (int e = s->head[n]; e != 0; e = s->next[e - 1]) {
-        if (count < kListed) {
-            int b = count;
-            while (b > 0 && list[b - 1][i] < e) {
-                list[b][i] = list[b - 1][i];
-                --b;
-            }
-            list[b][i] = e;
-        }
-        ++count;
-    }
+    const int2 node = s->node[n];
+    const int count = node.x, slots = listed(N);
     double fx = 0.0, fy = 0.0, fz = 0.0;
     auto add = [&](int e) {
-        const double* c = s->contrib + 3 * (size_t)(e - 1);
+        const double* c = s->contrib + 3 * (size_t)e;
         fx += c[0];
         fy += c[1];
         fz += c[2];
     };
-    if (count <= kListed) {
-#pragma unroll 4
-        for (int k = count - 1; k >= 0; --k) add(list[k][i]);
+    if (count <= slots) {
+        // Into ascending order.  Most nodes have at most kRanked entries: loaded
+        // together, their ranks counted in registers (independent compares;
+        // insertion's chain of shared-memory steps, as long as the warp's worst
+        // lane, took half of the kernel).
+        constexpr int kRanked = 16;
+        if (count <= kRanked) {
+            int e[kRanked], rank[kRanked];
+#pragma unroll
+            for (int u = 0; u < kRanked; ++u) {
+                e[u] = u < count && u < slots ? s->list[(size_t)u * N + n] : INT_MAX;
+                rank[u] = 0;
+            }
+#pragma unroll
+            for (int u = 1; u < kRanked; ++u)
+#pragma unroll
+                for (int w = 0; w < u; ++w) {
+                    const bool after = e[w] < e[u];
+                    rank[u] += after;
+                    rank[w] += !after;
+                }
+#pragma unroll
+            for (int u = 0; u < kRanked; ++u)
+                if (u < count) list[rank[u]][i] = e[u];
+        } else {
+            for (int k = 0; k < count; ++k) {
+                const int e = s->list[(size_t)k * N + n];
+                int b = k;
+                while (b > 0 && list[b - 1][i] > e) {
+                    list[b][i] = list[b - 1][i];
+                    --b;
+                }
+                list[b][i] = e;
+            }
+        }
+        // Several entries' contributions are under way together.
+        constexpr int kAhead = 8;
+        for (int k0 = 0; k0 < count; k0 += kAhead) {
+            double c[kAhead][3];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (k0 + u < count) {
+                    const double* from = s->contrib + 3 * (size_t)list[k0 + u][i];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) c[u][d] = from[d];
+                }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (k0 + u < count) {
+                    fx += c[u][0];
+                    fy += c[u][1];
+                    fz += c[u][2];
+                }
+        }
     } else {
-        // A longer chain: laid out from its end, which is nearly in order
-        // (blocks start in order), then insertion.
+        // The list, and the chain laid out from its end: nearly in order,
+        // then insertion.
         int* a = s->entries + atomicAdd(&s->used, count);
         int k = count;
-        for (int e = s->head[n]; e != 0; e = s->next[e - 1]) a[--k] = e;
+        for (int e = node.y; e != 0; e = s->next[e - 1]) a[--k] = e - 1;
+        while (--k >= 0) a[k] = s->list[(size_t)k * N + n];
         for (k = 1; k < count; ++k) {
             const int e = a[k];
             int b = k;
@@ -265,7 +323,7 @@ extern "C" ms_status ms_deformation_forces_noalloc(int32_t num_nodes, int32_t nu
         set_msg(err, err_len, buf);
         return false;
     };
-    e = cudaMemsetAsync(&s->bad, 0, offsetof(Scratch, head) - offsetof(Scratch, bad) + sizeof(int) * (size_t)N, st);
+    e = cudaMemsetAsync(&s->bad, 0, offsetof(Scratch, node) - offsetof(Scratch, bad) + sizeof(int2) * (size_t)N, st);
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_msg(err, err_len, cudaGetErrorString(e));

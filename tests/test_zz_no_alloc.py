@@ -78,9 +78,19 @@ def test_noalloc_matches_handle_path_on_two_calls(workdir):
 def test_noalloc_nodes_of_many_triangles(workdir, shared):
     """A node on more patches than a node's sorted list holds (32): `shared`
     triangles get it as their last patch node, besides its own."""
+    _shared_node(workdir, "disk50", shared)
+
+
+@pytest.mark.parametrize("shared", [29, 30, 31, 32])
+def test_noalloc_full_lists(workdir, shared):
+    """Around the longest list of a large mesh (30 entries at its node count)."""
+    _shared_node(workdir, "disk12", shared)
+
+
+def _shared_node(workdir, name, shared):
     import types
 
-    m = make_model(workdir, "disk50")
+    m = make_model(workdir, name)
     ids = m.tables()["patch_ids"].astype(np.int32)
     own = int((ids == 7).sum())
     free = [t for t in range(m.num_tris) if 7 not in ids[t]][:: max(1, m.num_tris // 1000)]
