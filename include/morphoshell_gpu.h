@@ -351,7 +351,8 @@ ms_status ms_batch_status(ms_batch* b, int32_t instance, ms_batch_inst_status* o
 /* Current (or final) positions and velocities of one instance, SoA; either may be NULL. */
 ms_status ms_batch_download_dofs(ms_batch* b, int32_t instance, double* dofs, double* velocities);
 /* Replaces one instance's positions (and velocities; NULL = zero), e.g. a
- * warm start, and restarts its state machine from dial_factor_to_start_from. */
+ * warm start, and restarts its state machine from dial_factor_to_start_from.
+ * The arrays, page-locked or not, have been read when the call returns. */
 ms_status ms_batch_upload_dofs(ms_batch* b, int32_t instance, const double* dofs, const double* velocities);
 /* Restarts one instance's state machine at dial_factor: dialling from there
  * (waiting = 0, as dial_factor_to_start_from), or waiting for equilibrium
