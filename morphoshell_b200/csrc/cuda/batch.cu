@@ -782,7 +782,7 @@ int batch_node_tile_blocks(int mixed, size_t smem) {
                           mixed ? (const void*)k_batch_node_tiles<true, QuietStep>
                                 : (const void*)k_batch_node_tiles<false, QuietStep>}) {
         int blocks = 0;
-        if (ea == cudaSuccess) ea = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (ea == cudaSuccess) ea = allow_shared(f, smem);
         if (ea == cudaSuccess) ea = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, f, kTile, smem);
         nb = std::min(nb, blocks);
     }
@@ -1512,8 +1512,6 @@ ms_status ms_batch_autotune(ms_batch* b, int32_t steps, ms_batch_schedule* chose
     // ms per step of schedule k from the saved state: one untimed pass
     // (graph instantiation, caches), then the timed one; < 0 on error (rc).
     auto time_sched = [&](int k) -> double {
-        if (kScheds[k].tri_block < 0)  // the launch's shared memory is the current plan's
-            batch_node_tile_blocks(mixed, node_tile_smem(b->ntp.stride, b->ntp.nodes, mixed));
         double t = -1.0;
         for (int rep = 0; rep < 2 && rc == MS_OK; ++rep) {
             if (copy_state(false) != cudaSuccess) {
@@ -1613,7 +1611,6 @@ ms_status ms_batch_autotune(ms_batch* b, int32_t steps, ms_batch_schedule* chose
                 for (void* x : al) cudaFree(x);
             }
         }
-        batch_node_tile_blocks(mixed, node_tile_smem(b->ntp.stride, b->ntp.nodes, mixed));
     }
     if (copy_state(false) != cudaSuccess && rc == MS_OK) rc = bcuda(b, cudaGetLastError(), "autotune restore");
     cudaStreamSynchronize(st);

@@ -472,6 +472,13 @@ int choose_cluster_size(int tpc, int threads, int mixed);
 size_t cluster_smem_bytes(int tpc, int mixed);
 // Threads per CTA of the cluster kernel.
 int cluster_threads();
+// Allows a kernel `need` bytes of dynamic shared memory per block; an error when
+// a block cannot have them.  The limit is a value of the function in the whole
+// process, not of a handle or a launch: were it a plan's size, another handle's
+// plan could lower it under this one's launches.  So it always goes to the most
+// that the device allows; occupancy and the split with L1 follow the size given
+// at the launch.
+cudaError_t allow_shared(const void* kernel, size_t need);
 // Raise the dynamic shared-memory limit of the cluster kernels (once, outside
 // any stream capture).
 cudaError_t prepare_cluster_kernels(int tpc);

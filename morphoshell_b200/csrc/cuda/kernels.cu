@@ -746,6 +746,18 @@ cudaError_t launch_energies(const DevMesh& m, const DevState& s, int parity, con
     return cudaGetLastError();
 }
 
+cudaError_t allow_shared(const void* kernel, size_t need) {
+    cudaFuncAttributes a{};
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+    if (e != cudaSuccess) return e;
+    most -= (int)a.sharedSizeBytes;
+    if (need > (size_t)most) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 void build_sell(int N, const int* off, const int* ent, std::vector<int>& sell_off, std::vector<int>& sell_ent) {
     const int W = (N + 31) / 32;
     sell_off.assign(W + 1, 0);

@@ -93,8 +93,7 @@ cudaError_t launch_one(const DevMesh& m, const ClusterPlan& p, const NodeTilePla
 
 template <int DIAL, bool MIXED>
 cudaError_t prepare_one(size_t smem, int& blocks) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_node_tiles<DIAL, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared((const void*)k_node_tiles<DIAL, MIXED>, smem);
     if (e != cudaSuccess) return e;
     int b = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_node_tiles<DIAL, MIXED>, kTile, smem);

@@ -39,3 +39,56 @@ def test_batch_upload_has_read_its_source(tmp_path, pinned, spacing):
             a[:] = -1.0
     for i, state in enumerate(want):
         assert all(np.array_equal(a, src) for a, src in zip(b.download(i), state))
+
+
+def _disk_loop(workdir, name, precision=0, path=None):
+    from morphoshell_b200 import GpuLoop
+    from conftest import make_model
+    m = make_model(workdir, name)
+    g = GpuLoop(m, precision=precision)
+    a, b = m.programmed()
+    g.set_programmed(3, a, b, m.scalars.dial_factors_to_hold_at_spacing)
+    if path is not None:
+        g.set_step_path(path)
+    g.upload(*deformed_state(m, seed=61, amp=0.02))
+    return m, g
+
+
+def _steps(m, g, n=20):
+    s = m.scalars
+    g.step_n(n, 0.2 + 1e-5 * np.arange(n), s.timestep, s.damping_factor_1)
+    g.do_dialling(0.3)
+    g.step_n(n, None, s.timestep, s.damping_factor_2)
+    return g.download()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("path", [3, 4])
+def test_larger_mesh_steps_after_a_smaller_one_is_created(workdir, monkeypatch, path, precision):
+    """A kernel's shared-memory limit belongs to the process: creating a handle
+    whose tiles need less must not take it from one whose tiles need more."""
+    if path == 4:
+        monkeypatch.setenv("MSB_NODE_TILE_PLAN", "4")
+    m, big = _disk_loop(workdir, "disk5", precision, path)
+    want = _steps(m, _disk_loop(workdir, "disk5", precision, 2)[1])
+    _, small = _disk_loop(workdir, "disk14", precision, path)
+    assert small.plan_info()["nodes_per_tile"] < big.plan_info()["nodes_per_tile"]
+    assert all(np.array_equal(a, b) for a, b in zip(_steps(m, big), want))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_larger_batch_steps_after_a_smaller_one_is_created(tmp_path, precision):
+    """The same for the batch's node-tiled schedule, in graphs (events) and in
+    quiet stretches."""
+    from morphoshell_b200 import Batch, ensemble
+    big_m, _ = ensemble.build_members([3, 5], str(tmp_path / "big"), spacing_range=(0.006, 0.0061), threads=4)
+    small_m, _ = ensemble.build_members([0, 1], str(tmp_path / "small"), spacing_range=(0.05, 0.1), threads=4)
+    big, ref = Batch(big_m, precision=precision), Batch(big_m, precision=precision)
+    big.set_schedule(-1, 0, 4)
+    ref.set_schedule(0, 256, 4)
+    small = Batch(small_m, precision=precision)
+    assert small.schedule()["nodes_per_tile"] < big.schedule()["nodes_per_tile"]
+    for steps in (4, 20):
+        assert big.run(steps) == ref.run(steps) == steps
+    for i in range(2):
+        assert all(np.array_equal(a, b) for a, b in zip(big.download(i), ref.download(i)))
