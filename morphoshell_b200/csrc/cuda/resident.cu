@@ -341,8 +341,7 @@ size_t smem_bytes(const ResidentPlan& q, int mixed) {
 template <int DIAL, bool MIXED, int TH>
 cudaError_t prepare_one(const ResidentPlan& q, int& blocks) {
     const size_t smem = smem_bytes(q, MIXED);
-    cudaError_t e = cudaFuncSetAttribute(k_resident<DIAL, MIXED, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_shared((const void*)k_resident<DIAL, MIXED, TH>, smem);
     if (e != cudaSuccess) return e;
     int b = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_resident<DIAL, MIXED, TH>, q.threads, smem);
@@ -360,16 +359,10 @@ cudaError_t prepare_th(const ResidentPlan& q, int& blocks) {
 template <int DIAL, bool MIXED, int TH>
 cudaError_t launch_one(const DevMesh& m, const ClusterPlan& p, const ResidentPlan& q, const DevState& s,
                        const StepScalars& sc, int steps, unsigned tag0, cudaStream_t st) {
-    const size_t smem = smem_bytes(q, MIXED);
-    // The limit belongs to the function, not to a handle: another handle's
-    // plan may have set it lower.
-    cudaError_t e = cudaFuncSetAttribute(k_resident<DIAL, MIXED, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(q.ntiles);
     cfg.blockDim = dim3(q.threads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = smem_bytes(q, MIXED);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

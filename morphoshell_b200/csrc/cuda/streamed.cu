@@ -430,8 +430,7 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
 template <int DIAL, bool MIXED, bool BATCH>
 cudaError_t prepare_one(const NodeTilePlan& q, const StreamPlan& sp, int insts, int& blocks) {
     const size_t smem = StSmem<MIXED>::bytes(q.stride, q.nodes, sp.halo, insts);
-    cudaError_t e = cudaFuncSetAttribute(k_streamed<DIAL, MIXED, BATCH>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared((const void*)k_streamed<DIAL, MIXED, BATCH>, smem);
     if (e != cudaSuccess) return e;
     int b = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_streamed<DIAL, MIXED, BATCH>, kTile, smem);
@@ -447,15 +446,10 @@ cudaError_t launch_one(const DevMesh& m, const NodeTilePlan& q, const StreamPlan
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    const size_t smem = StSmem<MIXED>::bytes(q.stride, q.nodes, sp.halo, bs.insts);
-    // The limit belongs to the function, not to a handle.
-    cudaError_t e = cudaFuncSetAttribute(k_streamed<DIAL, MIXED, BATCH>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(q.ntiles);
     cfg.blockDim = dim3(kTile);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = StSmem<MIXED>::bytes(q.stride, q.nodes, sp.halo, bs.insts);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

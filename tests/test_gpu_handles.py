@@ -92,3 +92,36 @@ def test_larger_batch_steps_after_a_smaller_one_is_created(tmp_path, precision):
         assert big.run(steps) == ref.run(steps) == steps
     for i in range(2):
         assert all(np.array_equal(a, b) for a, b in zip(big.download(i), ref.download(i)))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("big,small", [("disk15", "disk16"), ("disk6", "disk14")])
+def test_threads_step_meshes_of_different_size(workdir, big, small, precision):
+    """Host threads, a handle each, whose launches are of one kernel and need
+    different amounts of shared memory: the bits of each alone."""
+    import threading
+    got, errors = {}, []
+
+    def work(key, m, g):
+        s = m.scalars
+        lengths = np.random.default_rng(62).integers(2, 12, 3000)
+        try:
+            for n in lengths:
+                g.step_n(int(n), None, s.timestep, s.damping_factor_2)
+            got[key] = g.download()
+        except Exception as e:  # noqa: BLE001
+            errors.append((key, e))
+
+    for name in (big, small):
+        work(name, *_disk_loop(workdir, name, precision))
+    assert not errors, errors
+    loops = [(0, *_disk_loop(workdir, big, precision))]
+    loops += [(k, *_disk_loop(workdir, small, precision)) for k in (1, 2, 3)]
+    threads = [threading.Thread(target=work, args=x) for x in loops]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for k in range(4):
+        assert all(np.array_equal(a, b) for a, b in zip(got[k], got[small if k else big]))
