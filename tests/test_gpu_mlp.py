@@ -102,3 +102,51 @@ def test_new_rows_right_after_others():
         net.loss_grad(x[::-1], t)
         net.set_params(p * np.float32(1.0 + 0.01 * k))
         assert _rel(net.forward(x), mlp_ref.forward(net.params(), x, 22, 256, 2, 3, bf16_points=True)) < 1e-2
+
+
+def _activations(net, first=1.0):
+    """A network of one hidden layer whose first 16 hidden units are its
+    outputs, and whose hidden pre-activations are its inputs (the first one's
+    times `first`)."""
+    p = np.zeros(net.num_params(), dtype=np.float32)
+    (o0, n0, k0, _), (o1, n1, k1, _) = net.layers()
+    w0 = np.eye(n0, k0, dtype=np.float32)
+    w0[0, 0] = first
+    p[o0:o0 + n0 * k0] = w0.ravel()
+    p[o1:o1 + n1 * k1] = np.eye(n1, k1, dtype=np.float32).ravel()
+    net.set_params(p)
+
+
+def test_silu_of_every_bf16_value():
+    """Every finite BF16 pre-activation, beside others of every size (a
+    reciprocal serves two of them, one test sixteen), against SiLU in double,
+    rounded to BF16: rounding is monotone, so the result lies between the
+    rounded ends of an interval of FP32's errors around the value.  Those are
+    2^-22 of the exponential, of its argument's rounding 1.5 2^-24 times up to
+    89, and 2^-23 of the sum and the quotient: together under 2^-16.  Below
+    1e-36 the exponential overflows."""
+    import torch
+    rng = np.random.default_rng(70)
+    bits = np.arange(65536, dtype=np.uint32)
+    v = (bits[(bits & 0x7f80) != 0x7f80] << 16).view(np.float32)
+    x = np.stack([v] + [rng.permutation(v) for _ in range(127)], 1)
+    x[:, 64:] = rng.standard_normal((len(v), 64)).astype(np.float16)
+    net = _net(128, 128, 1, 16)
+    _activations(net)
+    z = torch.from_numpy(x[:, :16].astype(np.float64))
+    want = z / (1.0 + torch.exp(-z))
+    got = torch.from_numpy(net.forward(x)).double()
+    ends = [(want * (1.0 + e)).to(torch.float32).to(torch.bfloat16).double() for e in (-2.0 ** -16, 2.0 ** -16)]
+    ok = (got >= torch.minimum(*ends)) & (got <= torch.maximum(*ends)) | ((got - want).abs() <= 1e-36)
+    assert ok.all(), (z[~ok][:8], got[~ok][:8], want[~ok][:8])
+
+
+def test_silu_of_an_infinite_preactivation():
+    """A pre-activation beyond FP32 is infinite, and so is its SiLU."""
+    net = _net(128, 128, 1, 16)
+    _activations(net, first=4.0)
+    x = np.zeros((200, 128), dtype=np.float32)
+    x[::3, 0] = 3e38
+    y = net.forward(x)[:, 0]
+    assert (y[::3] == np.inf).all()
+    assert (np.delete(y, np.s_[::3]) == 0).all()
