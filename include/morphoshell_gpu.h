@@ -234,6 +234,13 @@ void* ms_stream(ms_handle* h);
  * until this call asks for a path by number.  All sum every node's contributions in ascending
  * triangle order, so they give the same bits. */
 ms_status ms_set_step_path(ms_handle* h, int path);
+/* Test hook: SM clocks a tile of the default path's many-step launches waits
+ * for a neighbour's positions before the launch is given up (2e9, about a
+ * second, unless set; 0: it is given up where a position is not there at the
+ * first look), in a call's launches from the from_launch-th on.  ms_step_n
+ * then runs the steps of that launch and the rest one by one, with the same
+ * result, and notes it in ms_last_error. */
+ms_status ms_set_wait_limit(ms_handle* h, int64_t clocks, int from_launch);
 /* Tiling of the cluster path: CTAs per cluster, triangles per CTA, number of
  * clusters, number of halo nodes (summed by the second kernel), and the
  * path in use. */
@@ -373,6 +380,8 @@ ms_status ms_batch_autotune(ms_batch* b, int32_t steps_per_trial, ms_batch_sched
  * node-tiled plan, ms per step): copies up to len - 1 bytes and a NUL into
  * buf, returns the full length (-1 for a null batch). */
 int32_t ms_batch_autotune_report(const ms_batch* b, char* buf, int32_t len);
+/* Test hook, as ms_set_wait_limit: the waits of the batch's many-step launches. */
+ms_status ms_batch_set_wait_limit(ms_batch* b, int64_t clocks);
 ms_status ms_batch_info(const ms_batch* b, int64_t* num_nodes, int64_t* num_tris, int32_t* n_instances);
 void* ms_batch_stream(ms_batch* b);
 

@@ -27,7 +27,8 @@ GPU_SYMBOLS = [
     "ms_download_programmed", "ms_surface_derivs", "ms_a_b_normals", "ms_deformation_forces",
     "ms_non_deformation_forces", "ms_impose_constraints", "ms_is_at_equilibrium", "ms_advance_dynamics",
     "ms_step_n", "ms_prepare_steps", "ms_output_quantities", "ms_device_info", "ms_stream", "ms_time_kernels",
-    "ms_deformation_forces_noalloc", "ms_set_step_path", "ms_plan_info", "ms_node_tile_layout", "ms_node_tile_plan",
+    "ms_deformation_forces_noalloc", "ms_set_step_path", "ms_set_wait_limit", "ms_batch_set_wait_limit",
+    "ms_plan_info", "ms_node_tile_layout", "ms_node_tile_plan",
     "ms_batch_create", "ms_batch_destroy", "ms_batch_last_error", "ms_batch_run", "ms_batch_status",
     "ms_batch_download_dofs", "ms_batch_upload_dofs", "ms_batch_set_schedule", "ms_batch_get_schedule",
     "ms_batch_autotune", "ms_batch_autotune_report", "ms_batch_info", "ms_batch_stream", "ms_batch_set_start",
@@ -169,6 +170,8 @@ def lib() -> C.CDLL:
                                                     C.c_double, C.c_void_p, C.c_void_p, C.c_void_p, C.c_char_p,
                                                     C.c_size_t]
         L.ms_set_step_path.argtypes = [C.c_void_p, C.c_int]
+        L.ms_set_wait_limit.argtypes = [C.c_void_p, C.c_int64, C.c_int]
+        L.ms_batch_set_wait_limit.argtypes = [C.c_void_p, C.c_int64]
         ip = C.POINTER(C.c_int)
         L.ms_plan_info.argtypes = [C.c_void_p, ip, ip, ip, ip, ip]
         L.ms_node_tile_plan.argtypes = [C.c_void_p, ip, ip, ip, ip]
@@ -462,6 +465,14 @@ class GpuLoop:
         on meshes with a node tile for every SM)."""
         self._chk(lib().ms_set_step_path(self._h, path), "set_step_path")
 
+    def set_wait_limit(self, clocks: int, from_launch: int = 0):
+        """Test hook: how long a tile of a many-step launch waits for its
+        neighbours (ms_set_wait_limit)."""
+        self._chk(lib().ms_set_wait_limit(self._h, clocks, from_launch), "set_wait_limit")
+
+    def last_error(self) -> str:
+        return lib().ms_last_error(self._h).decode()
+
     def plan_info(self) -> dict:
         v = [C.c_int() for _ in range(5)]
         self._chk(lib().ms_plan_info(self._h, *[C.byref(x) for x in v]), "plan_info")
@@ -596,6 +607,13 @@ class Batch:
         buf = C.create_string_buffer(max(n, 0) + 1)
         lib().ms_batch_autotune_report(self._h, buf, len(buf))
         return [ln for ln in buf.value.decode().splitlines() if ln]
+
+    def set_wait_limit(self, clocks: int):
+        """Test hook, as GpuLoop.set_wait_limit."""
+        self._chk(lib().ms_batch_set_wait_limit(self._h, clocks), "ms_batch_set_wait_limit")
+
+    def last_error(self) -> str:
+        return lib().ms_batch_last_error(self._h).decode()
 
     def info(self):
         N, T, n = C.c_int64(), C.c_int64(), C.c_int32()

@@ -856,11 +856,12 @@ ms_status build_stream(ms_batch* b, const std::vector<int>& patch6, const std::v
     sp.halo_id = d_ids;
     sp.local = d_local;
     sp.border = d_border;
-    b->stp = sp;
     b->bst.n_inst = b->n_inst;
     b->bst.insts = insts;
     b->bst.node_inst = b->d_node_inst;
-    b->bst.err = b->d_err;
+    sp.patience = kPacketPatience;
+    sp.wait = kPacketWait;
+    b->stp = sp;
     b->bst.trip = b->d_trip;
     b->have_stream = true;
     return MS_OK;
@@ -880,7 +881,7 @@ int64_t quiet_steps(const ms_batch* b, int64_t most) {
 }
 
 // One streamed stretch of `steps` steps; *stood says whether it counts (no
-// node tripped the guard).
+// node tripped the guard and no wait ran out; else its steps run one by one).
 ms_status run_stretch(ms_batch* b, int steps, bool* stood) {
     const int n = b->n_inst;
     cudaStream_t st = b->stream;
@@ -901,6 +902,8 @@ ms_status run_stretch(ms_batch* b, int steps, bool* stood) {
     b->is_stale = true;
     MB_TRY(fetch_states(b));
     *stood = trip == 0;
+    if (trip == MS_ERR_TIMEOUT)
+        b->last_error = "a tile waited too long for its neighbours' positions: a stretch's steps ran one by one";
     if (*stood) b->parity ^= 1;
     return MS_OK;
 }
@@ -1309,7 +1312,7 @@ ms_status ms_batch_run(ms_batch* b, int64_t max_steps, int64_t* steps_done) {
     // Unless streamed, in the node-tiled schedule.
     const bool quiet_nt = !stream && b->have_nt && kScheds[b->sched].tri_block < 0;
     const int64_t stretch = std::min<int64_t>(stream ? kStretchSteps : kQuietSteps, kStretchDials / b->n_inst);
-    int64_t by_step = 0;  // steps to take one by one: a stretch whose guard tripped
+    int64_t by_step = 0;  // steps to take one by one: a stretch that did not count
     while (done < max_steps && !all_frozen(b)) {
         int64_t most = b->chunk - done % b->chunk;  // a chunk, or to the end of this one after a stretch
         if (stream) {
@@ -1647,6 +1650,13 @@ ms_status ms_batch_info(const ms_batch* b, int64_t* num_nodes, int64_t* num_tris
     if (num_nodes) *num_nodes = b->m.N;
     if (num_tris) *num_tris = b->m.T;
     if (n_instances) *n_instances = b->n_inst;
+    return MS_OK;
+}
+
+ms_status ms_batch_set_wait_limit(ms_batch* b, int64_t clocks) {
+    if (!b || clocks < 0) return MS_ERR_INVALID_ARGUMENT;
+    b->stp.patience = clocks ? kPacketPatience : 0;
+    b->stp.wait = clocks;
     return MS_OK;
 }
 

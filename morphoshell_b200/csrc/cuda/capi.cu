@@ -102,6 +102,8 @@ struct ms_handle {
     ResidentPlan rsp{};
     StreamPlan stp{};
     unsigned pk_tag = 0;  // tag of the last step published in packets
+    long long wait = kPacketWait;  // ResidentPlan::wait of a call's launches from the wait_from-th on
+    int wait_from = 0;
 };
 
 namespace {
@@ -1209,11 +1211,18 @@ static bool use_resident(const ms_handle* h, int n, bool dialling, bool fuse_lce
     return dialling ? fuse_lce && h->plan.tri_aux && h->plan.lce_uniform : true;
 }
 
+ms_status ms_set_wait_limit(ms_handle* h, int64_t clocks, int from_launch) {
+    if (!h || clocks < 0 || from_launch < 0) return MS_ERR_INVALID_ARGUMENT;
+    h->wait = clocks;
+    h->wait_from = from_launch;
+    return MS_OK;
+}
+
 // Runs n steps from h->cur as resident or streamed launches and waits for them (the
 // error record is in *h->h_err then, the equilibrium record in *h->h_equil
 // with check_last).  *done receives the steps that stand: n with h->cur
-// holding their state, or, when a launch tripped the guard, the steps before
-// that launch with h->cur holding the state it started from.
+// holding their state, or, when a launch tripped the guard or was given up, the
+// steps before that launch with h->cur holding the state it started from.
 static ms_status run_resident(ms_handle* h, int n, const double* dials, int dial_mode, double dt, double damping,
                               int gd, int check_last, int* done) {
     cudaStream_t st = h->stream;
@@ -1225,6 +1234,8 @@ static ms_status run_resident(ms_handle* h, int n, const double* dials, int dial
         if (dials) MS_TRY(fill_dials(h, dials, at, at + len));
         starts.push_back(at);
         const bool last = at + len == n;
+        h->rsp.wait = h->stp.wait = k >= h->wait_from ? h->wait : kPacketWait;
+        h->rsp.patience = h->stp.patience = h->rsp.wait ? kPacketPatience : 0;
         StepScalars sc{at, p0 ^ (k & 1), dt, damping, h->rho_hh, h->force_limit, gd, check_last && last ? 1 : 0};
         if (h->have_resident)
             MS_CUDA(h, launch_resident(h->m, h->plan, h->rsp, h->s, sc, dial_mode, h->precision, len, h->pk_tag, st));
@@ -1236,18 +1247,17 @@ static ms_status run_resident(ms_handle* h, int n, const double* dials, int dial
     MS_CUDA(h, cudaMemcpyAsync(h->h_err, h->s.err, sizeof(DevError), cudaMemcpyDeviceToHost, st));
     if (check_last) MS_CUDA(h, cudaMemcpyAsync(h->h_equil, h->s.equil, sizeof(DevEquil), cudaMemcpyDeviceToHost, st));
     MS_CUDA(h, cudaStreamSynchronize(st));
-    if (h->h_err->flag == MS_ERR_TIMEOUT) {
-        // Blocks stopped at different steps; the buffer the first launch
-        // read is whole.
-        h->cur = p0;
-        return fail(h, MS_ERR_TIMEOUT, "a tile waited too long for its neighbours' positions");
-    }
     int launches = (int)starts.size();
     *done = n;
     if (h->h_err->flag) {
         const int step = (int)(h->h_err->guard_key >> 32);
         while (launches > 1 && starts[launches - 1] > step) --launches;
         *done = starts[--launches];
+        if (h->h_err->flag == MS_ERR_TIMEOUT) {
+            // Some blocks of a check step may have counted themselves.
+            MS_CUDA(h, cudaMemsetAsync(h->s.eq_counter, 0, sizeof(unsigned int), st));
+            h->last_error = "a tile waited too long for its neighbours' positions: a launch's steps ran one by one";
+        }
     }
     h->cur = p0 ^ (launches & 1);
     return MS_OK;
@@ -1278,7 +1288,8 @@ ms_status ms_step_n(ms_handle* h, int n, const double* dials, int dialling, doub
     if (resident) {
         MS_TRY(run_resident(h, n, dialling ? dials : nullptr, dial_mode, dt, damping, gd, check_last, &done));
         // After a guard trip the rest runs step by step, which stops at the
-        // tripping step with the state it started from.
+        // tripping step with the state it started from; so it does after a
+        // launch that was given up, and the call goes on as if it had not been.
         if (done < n) {
             DevError z{};
             z.base = done;

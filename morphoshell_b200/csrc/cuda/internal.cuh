@@ -236,6 +236,11 @@ void fill_node_tile_records(const NodeTileLayout& L, const int* patch_ids, const
 void fill_node_sections(const NodeTileLayout& L, size_t pitch, std::vector<unsigned char>& sections,
                         std::vector<int>& chunk_tri);
 
+// A tile's wait for another's packet: about a second of SM clock, which is read
+// once a few trips through L2 have not brought it.
+constexpr long long kPacketWait = 2000000000LL;
+constexpr int kPacketPatience = 64;
+
 // Resident step (resident.cu): many steps in one cooperative launch, one
 // block per node tile, one thread per triangle of the tile.
 struct ResidentPlan {
@@ -251,6 +256,8 @@ struct ResidentPlan {
     const unsigned char* border;   // [N] another tile reads this node
     const unsigned char* count;    // [N] entries of this node
     ulonglong2* packets;           // [2][3][N] positions in flight, each half of a double beside its step's tag
+    int patience;                  // looks at another tile's packet before the clock is read, ...
+    long long wait;                // ... and SM clocks after them before a tile gives up
 };
 struct ResidentLayout {
     int nodes = 0, ntiles = 0, halo = 0, threads = 0, width = 0;
@@ -274,6 +281,8 @@ struct StreamPlan {
     const unsigned char* border;   // [N] another tile reads this node
     double* metric;                // [nchunks][6][kTile] abar, bbar of a launch that reads them from the arrays
     ulonglong2* packets;           // as ResidentPlan::packets
+    int patience;                  // as ResidentPlan::patience, wait
+    long long wait;
 };
 struct StreamLayout {
     int halo = 0;
@@ -344,8 +353,8 @@ struct BatchStream {
     const InstParams* ip;
     const InstState* is;
     const double2* dials;       // [steps][n_inst] lambda, lambda^(-2 nu_ot)
-    int* err;                   // 5 (MS_ERR_TIMEOUT) when a wait ran out
-    int* trip;                  // 1 when a node tripped the force guard: the stretch does not count
+    int* trip;                  // when a node tripped the force guard (1) or a wait ran out (5, MS_ERR_TIMEOUT): the
+                                // stretch does not count
 };
 
 struct DevState {

@@ -25,6 +25,14 @@ __device__ __forceinline__ bool packet_is(unsigned long long lo, unsigned long l
     return (unsigned)(lo >> 32) == tag && (unsigned)(hi >> 32) == tag;
 }
 
+// Whether a wait that missed its packet for the `spin`-th time (from 0) is over.
+// The clock is read, first into t0, from the `patience`-th miss on.
+__device__ __forceinline__ bool wait_is_over(int spin, int patience, long long& t0, long long limit) {
+    if (spin < patience) return false;
+    if (spin == patience) t0 = clock64();
+    return clock64() - t0 >= limit;
+}
+
 __device__ __forceinline__ double packet_value(unsigned long long lo, unsigned long long hi) {
     return __longlong_as_double((long long)((lo & 0xffffffffULL) | (hi << 32)));
 }

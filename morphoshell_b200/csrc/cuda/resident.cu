@@ -36,11 +36,12 @@
 // step-s packet has read step s + 1 of every tile that could still want it.
 //
 // The launch is cooperative, so its blocks are resident together.  Every
-// poll is bounded (about a second of SM clock); a block that gives up
-// records MS_ERR_TIMEOUT and returns, and so do its neighbours in turn.
-// The state the launch starts from stays untouched in its buffer (only the
-// last step writes the other one), so a step that trips the force guard is
-// found and reported by running the launch's steps again one by one.
+// wait is bounded (about a second of SM clock); a block that gives up
+// records it and returns, and so do its neighbours in turn.  The state the
+// launch starts from stays untouched in its buffer (only the last step writes
+// the other one), so the steps of a launch that tripped the force guard or
+// was given up run again one by one: the call gives the same result, and finds
+// and reports the step that trips.
 #include <algorithm>
 #include <climits>
 
@@ -77,8 +78,8 @@ __global__ void __launch_bounds__(TH, 1)
                int steps, unsigned tag0) {
     using R = typename Real<MIXED>::T;
     const int g0 = global_step(s.err, sc.step);
-    // An earlier launch tripped the guard or timed out: uniform over the grid.
-    if (stale(s.err, g0) || *((volatile const int*)&s.err->flag) == 5) return;
+    // An earlier launch tripped the guard or was given up: uniform over the grid.
+    if (stale(s.err, g0)) return;
     extern __shared__ __align__(16) unsigned char rs_smem[];
     constexpr int S = TH;
     const int NT = q.nodes, N = m.N;
@@ -306,15 +307,14 @@ __global__ void __launch_bounds__(TH, 1)
                         }
                     }
                 if (!wait) break;
-                if (spin == 64) t0 = clock64();
-                if (spin > 64 && clock64() - t0 > 2000000000LL) {
+                if (wait_is_over(spin, q.patience, t0, q.wait)) {
                     ok = 0;
                     break;
                 }
             }
         }
         if (!__syncthreads_and(ok)) {
-            if (i == 0) atomicCAS(&s.err->flag, 0, 5);  // MS_ERR_TIMEOUT
+            if (i == 0) record_timeout(s, g0);
             return;
         }
     }

@@ -32,6 +32,15 @@ __device__ __forceinline__ void record_guard(const DevState& s, int gstep, long 
     atomicExch(&s.err->flag, 3);  // MS_ERR_IMPLAUSIBLE_FORCE
 }
 
+// A many-step launch from step g0 whose wait ran out did not finish: it counts
+// as one that tripped the guard, after every node of its first step.  Later
+// launches do nothing, the state it started from survives, and its steps run
+// again one by one.
+__device__ __forceinline__ void record_timeout(const DevState& s, int g0) {
+    atomicMin(&s.err->guard_key, ((unsigned long long)(unsigned)g0 << 32) | 0xffffffffULL);
+    atomicCAS(&s.err->flag, 0, 5);  // MS_ERR_TIMEOUT
+}
+
 // Larger value wins; on equal values the smaller node id wins
 // (std::max_element returns the first maximum).  NaN never wins a
 // comparison, as in std::max_element.

@@ -22,8 +22,8 @@
 // the adds, was slower (15.9 us): three times the entries' loads.
 //
 // The launch is cooperative; every wait is bounded; the state a launch starts
-// from stays untouched, and a step that trips the force guard is found by
-// running the launch's steps again one by one, as for the resident step.
+// from stays untouched, and the steps of one that tripped the force guard or was
+// given up run again one by one, as for the resident step.
 //
 // The batch runs stretches of steps in which no instance changes its status or
 // checks for equilibrium the same way (BATCH): the union is the mesh, a tile
@@ -136,10 +136,13 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
     int g0 = 0;
     if constexpr (!BATCH) {
         g0 = global_step(s.err, sc.step);
-        // An earlier launch tripped the guard or timed out: uniform over the grid.
-        if (stale(s.err, g0) || *((volatile const int*)&s.err->flag) == 5) return;
+        // An earlier launch tripped the guard or was given up: uniform over the grid.
+        if (stale(s.err, g0)) return;
     }
-    int* err_flag = BATCH ? bs.err : &s.err->flag;
+    auto give_up = [&]() {
+        if constexpr (BATCH) atomicExch(bs.trip, 5);
+        else record_timeout(s, g0);
+    };
     extern __shared__ __align__(128) unsigned char st_smem[];
     __shared__ uint64_t bar;
     const int NT = q.nodes, N = m.N, ld = NT + sp.halo;
@@ -245,7 +248,7 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
             const int ok = __syncthreads_and(bar_wait(&bar, phase) ? 1 : 0);
             phase ^= 1u;
             if (!ok) {
-                if (i == 0) atomicCAS(err_flag, 0, 5);  // MS_ERR_TIMEOUT; no other copy is in flight
+                if (i == 0) give_up();  // no other copy is in flight
                 return;
             }
             if (i == 0 && nc >= 0) fetch(nc, slot ^ 1);
@@ -406,8 +409,7 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
                         }
                     }
                 if (!wait) break;
-                if (++spin == 64) t0 = clock64();
-                if (spin > 64 && clock64() - t0 > 2000000000LL) {
+                if (wait_is_over(spin++, sp.patience, t0, sp.wait)) {
                     ok = 0;
                     break;
                 }
@@ -415,8 +417,8 @@ __global__ void __launch_bounds__(kTile, MIXED ? 4 : 3)
         }
         if (!__syncthreads_and(ok)) {
             if (i == 0) {
-                atomicCAS(err_flag, 0, 5);  // MS_ERR_TIMEOUT
-                bar_wait(&bar, phase);          // the next step's first node section is on its way
+                give_up();
+                bar_wait(&bar, phase);  // the next step's first node section is on its way
             }
             return;
         }

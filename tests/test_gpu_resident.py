@@ -239,3 +239,45 @@ def test_batch_steps_reported_when_the_last_instance_fails(tmp_path, sched):
         assert all(g.status(i).status == MS_INST_FAILED for i in range(2))
         out.append((done, _batch_state(g)))
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("name", ["disk100", "disk18k", "disk15", "disk14"])
+@pytest.mark.parametrize("launch", [0, 1, 2])
+def test_wait_that_runs_out(workdir, name, launch, precision):
+    """A launch given up because a tile's wait ran out -- the first of a call,
+    the second, which writes the buffer the call began from, or the third, with
+    the check -- leaves no trace: the bits and the report of the two-kernel
+    step, and so the next call's with waits as they were."""
+    m = make_model(workdir, name)
+    s = m.scalars
+    x, v = deformed_state(m, seed=45, amp=0.02)
+    n = 128 + 8192 + 160
+    out = []
+    for g in _pair(m, precision):
+        g.upload(x, v)
+        g.set_wait_limit(0, launch)
+        r = [_equil(g.step_n(n, 0.2 + 1e-6 * np.arange(n), s.timestep, s.damping_factor_1, check_last=True))]
+        noted = g.last_error()
+        state = g.download()
+        metric = g.programmed()
+        g.set_wait_limit(2_000_000_000)
+        r.append(_equil(g.step_n(200, None, s.timestep, s.damping_factor_2, check_last=True)))
+        out.append((noted, r, [bytes(a) for a in (*state, *metric, *g.download())]))
+    assert "waited too long" in out[0][0] and not out[1][0]
+    assert out[0][1:] == out[1][1:]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batch_wait_that_runs_out(tmp_path, precision):
+    """The same for a batch's stretches: step by step instead, from the states
+    and counters before."""
+    from morphoshell_b200 import Batch
+    models = _batch_members(tmp_path, [12, 13, 14, 15, 16, 17], spacing_range=(0.03, 0.05))
+    a, b = Batch(models, precision=precision), Batch(models, precision=precision)
+    b.set_schedule(0, 256, 64)
+    for steps, clocks in [(100, 2_000_000_000), (300, 0), (300, 2_000_000_000), (3000, 0)]:
+        a.set_wait_limit(clocks)
+        assert a.run(steps) == b.run(steps)
+        assert _batch_state(a) == _batch_state(b)
+        assert ("waited too long" in a.last_error()) == (steps > 100)
