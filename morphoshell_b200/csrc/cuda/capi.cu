@@ -459,14 +459,15 @@ ms_status room_for_partials(ms_handle* h, int n) {
     return MS_OK;
 }
 
-// Plan of the resident step, where the mesh is small enough for it.
+// Plan of the resident step, where the mesh is small enough for it and of one
+// material, as that step needs.
 ms_status build_resident(ms_handle* h, const ms_mesh_desc* d, const std::vector<int>& off,
                          const std::vector<int>& ent) {
     int sms = 0, coop = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device);
     ResidentLayout L;
-    if (!coop || !resident_layout(d->patch_ids, d->num_nodes, d->num_tris, sms, off, ent, L)) return MS_OK;
+    if (!coop || !h->m.uniform_hmu || !resident_layout(d->patch_ids, d->num_nodes, d->num_tris, sms, off, ent, L)) return MS_OK;
     ResidentPlan q{};
     q.nodes = L.nodes;
     q.ntiles = L.ntiles;
@@ -498,12 +499,13 @@ ms_status build_resident(ms_handle* h, const ms_mesh_desc* d, const std::vector<
     return MS_OK;
 }
 
-// Meshes the streamed step is for: tables (of the mesh's triangles; border
-// ones come once per tile, about a quarter more) that stay in L2.
+// Meshes the streamed step is for: one material, and tables (of the mesh's
+// triangles; border ones come once per tile, about a quarter more) that stay
+// in L2.
 bool stream_range(const ms_handle* h, int N, int T) {
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device);
-    return coop && N >= 8192 && stream_bytes(h->precision == MS_PRECISION_MIXED, T) <= kStreamBytes;
+    return coop && h->m.uniform_hmu && N >= 8192 && stream_bytes(h->precision == MS_PRECISION_MIXED, T) <= kStreamBytes;
 }
 
 ms_status build_streamed(ms_handle* h, const StreamLayout& S) {

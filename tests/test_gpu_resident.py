@@ -281,3 +281,28 @@ def test_batch_wait_that_runs_out(tmp_path, precision):
         assert a.run(steps) == b.run(steps)
         assert _batch_state(a) == _batch_state(b)
         assert ("waited too long" in a.last_error()) == (steps > 100)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_varied_materials_keep_the_node_tiled_plan(workdir, tmp_path, precision):
+    """A mid-size mesh with a material per triangle, which the many-step
+    kernels do not take: node tiles of at least 256 nodes as without those
+    kernels, and the two-kernel step's bits on them."""
+    from morphoshell_b200 import Model, meshgen
+    mesh = meshgen.disk_mesh(0.013, seed=5)
+    info = meshgen.lce_abar_info(mesh, meshgen.azimuthal_director, 0.9)
+    st = os.path.join(str(tmp_path), "s.txt")
+    meshgen.write_settings(st, protocol=3, ref_shear_modulus_if_uniform=-1.0)
+    shear = 1 + 0.3 * np.random.default_rng(7).random(mesh.num_tris)
+    m = Model.from_arrays(st, mesh.nodes, mesh.tris, info, np.zeros((mesh.num_tris, 3)), shear_modulus=shear)
+    assert np.ptp(m.tables()["ref_shear_modulus"]) > 0.2
+    s = m.scalars
+    ga, gb = _pair(m, precision)
+    assert ga.plan_info()["nodes_per_tile"] >= 256
+    ga.set_step_path(3)
+    for g in (ga, gb):
+        g.upload(*deformed_state(m, seed=46, amp=0.02))
+        g.step_n(40, 0.2 + 1e-5 * np.arange(40), s.timestep, s.damping_factor_1)
+        g.do_dialling(0.3)
+        g.step_n(40, None, s.timestep, s.damping_factor_2)
+    assert _same(ga, gb)
