@@ -480,6 +480,8 @@ ms_status build_resident(ms_handle* h, const ms_mesh_desc* d, const std::vector<
         return MS_OK;  // the other paths remain
     }
     TableBlob blob;
+    blob.bytes.reserve(4 * (L.head.size() + L.tri.size() + L.halo_id.size()) + 2 * (L.local.size() + L.entries.size()) +
+                       L.border.size() + L.count.size() + 7 * 16);
     const size_t head = blob.put(L.head), tri = blob.put(L.tri), halo_id = blob.put(L.halo_id),
                  local = blob.put(L.local), entries = blob.put(L.entries), border = blob.put(L.border),
                  count = blob.put(L.count);
@@ -510,6 +512,7 @@ bool stream_range(const ms_handle* h, int N, int T) {
 
 ms_status build_streamed(ms_handle* h, const StreamLayout& S) {
     TableBlob blob;
+    blob.bytes.reserve(4 * (S.halo_count.size() + S.halo_id.size() + S.local.size()) + S.border.size() + 4 * 16);
     const size_t count = blob.put(S.halo_count), ids = blob.put(S.halo_id), local = blob.put(S.local),
                  border = blob.put(S.border);
     unsigned char* base;
