@@ -292,8 +292,13 @@ ms_status ms_time_kernels(ms_handle* h, int reps, int dialling, double dial_fact
  * thresholds and programmed field.  An instance that trips the guard is
  * marked failed and keeps the state from before that step; one that reaches
  * equilibrium at dial factor 1 (with stop_at_final_equilibrium) is done;
- * either way it stops while the others go on.  Steps run in chunks captured
- * as CUDA graphs; the host looks at the instance states between chunks. */
+ * either way it stops while the others go on.  The steps in which no instance
+ * ends a dial phase or checks run in stretches: on unions whose tables stay in
+ * L2 (up to 80 MB at 256 bytes a triangle, 160 mixed; one material per
+ * instance) in one cooperative launch a stretch, with the node-tiled schedule
+ * one launch a step.  The others run in chunks captured as CUDA graphs.  The
+ * host looks at the instance states between stretches and chunks.  However a
+ * step is run, it gives the same bits. */
 typedef struct ms_batch ms_batch;
 
 enum ms_inst_status {
@@ -339,7 +344,10 @@ typedef struct ms_batch_inst_status {
  * per-node kernel, steps per captured graph (even).  nodes_per_tile and
  * blocks_per_sm describe the node-tiled plan in use (read by
  * ms_batch_get_schedule, chosen by ms_batch_autotune; ignored by
- * ms_batch_set_schedule). */
+ * ms_batch_set_schedule).  After ms_batch_set_schedule every step runs in that
+ * schedule, those of whole stretches too; by default, and after
+ * ms_batch_autotune where that found it faster, whole stretches run in one
+ * launch and the schedule is that of the steps between them. */
 typedef struct ms_batch_schedule {
     int32_t tri_block, node_block, chunk_steps;
     int32_t nodes_per_tile, blocks_per_sm;
@@ -373,7 +381,10 @@ ms_status ms_batch_get_schedule(const ms_batch* b, ms_batch_schedule* s);
  * CUDA events) from the current state, puts the state back after each trial,
  * and keeps the fastest; then rebuilds the node-tiled plan at other tile
  * sizes and resident blocks per SM, times each the same way and keeps the
- * fastest plan.  All schedules and plans give the same bits. */
+ * fastest plan; last, where the batch has them, times whole stretches in one
+ * launch (at least 256 steps, if no instance ends a dial phase or checks before)
+ * and turns them on or off.  best_ms_per_step is the fastest of all.  All
+ * schedules and plans give the same bits. */
 ms_status ms_batch_autotune(ms_batch* b, int32_t steps_per_trial, ms_batch_schedule* chosen,
                             double* best_ms_per_step);
 /* The last ms_batch_autotune's trials as text, one per line (schedule or

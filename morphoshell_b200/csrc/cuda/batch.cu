@@ -808,6 +808,7 @@ ms_status fetch_states(ms_batch* b) {
 constexpr int kStretchSteps = 4096;
 constexpr int kQuietSteps = 256;  // the same in separate launches: the host looks at the states between
 constexpr int kStretchMin = 8;
+constexpr int kTuneStretch = 256;  // the autotuner times at least these many steps of one, if no event comes before
 constexpr int kStretchDials = 1 << 18;  // dial table entries (instances x steps)
 
 // The streamed plan of the union, where it is in that kernel's range.
@@ -880,21 +881,32 @@ int64_t quiet_steps(const ms_batch* b, int64_t most) {
     return std::max<int64_t>(most, 0);
 }
 
-// One streamed stretch of `steps` steps; *stood says whether it counts (no
-// node tripped the guard and no wait ran out; else its steps run one by one).
-ms_status run_stretch(ms_batch* b, int steps, bool* stood) {
+// The kernel of a streamed stretch of `steps` steps, after the tables it reads.
+ms_status prepare_stretch(ms_batch* b, int steps) {
     const int n = b->n_inst;
-    cudaStream_t st = b->stream;
-    MB_CUDA(b, cudaMemsetAsync(b->d_trip, 0, sizeof(int), st));
-    k_batch_dials<<<(n * steps + 127) / 128, 128, 0, st>>>(b->d_ip, b->d_is, n, steps, b->d_dials, nullptr);
+    MB_CUDA(b, cudaMemsetAsync(b->d_trip, 0, sizeof(int), b->stream));
+    k_batch_dials<<<(n * steps + 127) / 128, 128, 0, b->stream>>>(b->d_ip, b->d_is, n, steps, b->d_dials, nullptr);
     MB_CUDA(b, cudaGetLastError());
+    return MS_OK;
+}
+ms_status launch_stretch(ms_batch* b, int steps) {
     BatchStream bs = b->bst;
     bs.dials = b->d_dials;
     bs.ip = b->d_ip;
     bs.is = b->d_is;
     MB_CUDA(b, launch_batch_streamed(b->m, b->st_ntp, b->stp, bs, b->s, b->parity, b->precision, steps, b->pk_tag,
-                                     st));
+                                     b->stream));
     b->pk_tag += (unsigned)steps;
+    return MS_OK;
+}
+
+// One streamed stretch of `steps` steps; *stood says whether it counts (no
+// node tripped the guard and no wait ran out; else its steps run one by one).
+ms_status run_stretch(ms_batch* b, int steps, bool* stood) {
+    const int n = b->n_inst;
+    cudaStream_t st = b->stream;
+    MB_TRY(prepare_stretch(b, steps));
+    MB_TRY(launch_stretch(b, steps));
     k_batch_advance<<<(n + 127) / 128, 128, 0, st>>>(b->d_ip, b->d_is, n, steps, b->d_dials, b->d_trip, nullptr, 0);
     MB_CUDA(b, cudaGetLastError());
     int trip = 0;
@@ -1615,6 +1627,39 @@ ms_status ms_batch_autotune(ms_batch* b, int32_t steps, ms_batch_schedule* chose
             }
         }
     }
+    // The streamed kernel, which a run takes between events: on where it beats
+    // the fastest schedule, off where not; as it was where an event comes so
+    // soon that there is nothing to time, or the stretch would not count.
+    bool stream_on = b->stream_on;
+    auto time_stretch = [&]() -> ms_status {
+        int64_t most = std::min<int64_t>(std::max(steps, kTuneStretch), kStretchDials / b->n_inst);
+        for (int rep = 0; rep < 2; ++rep) {
+            if (copy_state(false) != cudaSuccess) return bcuda(b, cudaGetLastError(), "autotune restore");
+            b->parity = p0;
+            b->is_stale = true;
+            MB_TRY(fetch_states(b));
+            most = quiet_steps(b, most);
+            if (most < kStretchMin) return MS_OK;
+            MB_TRY(prepare_stretch(b, (int)most));
+            cudaEventRecord(ev0, st);
+            MB_TRY(launch_stretch(b, (int)most));
+            cudaEventRecord(ev1, st);
+            int trip = 0;
+            MB_CUDA(b, cudaMemcpyAsync(&trip, b->d_trip, sizeof(int), cudaMemcpyDeviceToHost, st));
+            MB_CUDA(b, cudaStreamSynchronize(st));
+            if (trip) return MS_OK;  // the steps would be taken one by one
+        }
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ev0, ev1);
+        const double t = ms / (double)most;
+        char line[160];
+        std::snprintf(line, sizeof line, "streamed stretches: %.4f ms/step\n", t);
+        report += line;
+        stream_on = t < best;
+        best = std::min(best, t);
+        return MS_OK;
+    };
+    if (rc == MS_OK && b->have_stream) rc = time_stretch();
     if (copy_state(false) != cudaSuccess && rc == MS_OK) rc = bcuda(b, cudaGetLastError(), "autotune restore");
     cudaStreamSynchronize(st);
     cudaEventDestroy(ev0);
@@ -1628,6 +1673,7 @@ ms_status ms_batch_autotune(ms_batch* b, int32_t steps, ms_batch_schedule* chose
         return rc;
     }
     b->sched = best_k;
+    b->stream_on = stream_on;
     b->tune_report = report;
     if (chosen) ms_batch_get_schedule(b, chosen);
     if (best_ms) *best_ms = best;

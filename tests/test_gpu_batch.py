@@ -217,3 +217,30 @@ def test_batch_members_against_oracle(tmp_path):
         bx, bv = b.download(i)
         assert np.abs(bx - ox).max() <= 1e-9 * np.abs(ox).max(), i
         assert np.abs(bx - m.dofs(1)).max() > 0
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_autotune_weighs_whole_stretches_too(tmp_path, precision):
+    """The autotuner times a stretch in one launch beside the schedules, turns
+    it on after a schedule by number had turned it off (and only where it is
+    the fastest), reports the time that a run then takes, and leaves the state
+    and the bits alone."""
+    from morphoshell_b200 import Batch
+    models, _ = _members(tmp_path, [6, 7])
+    a, b = Batch(models, precision=precision), Batch(models, precision=precision)
+    for g in (a, b):
+        g.set_schedule(0, 256, 64)
+        g.set_wait_limit(0)  # a stretch in one launch notes that it was given up
+        assert g.run(100) == 100 and not g.last_error()
+    a.set_wait_limit(2_000_000_000)
+    sched, ms = a.autotune(steps_per_trial=10)
+    a.set_wait_limit(0)
+    trials = {line.split(":")[0]: float(line.split(":")[1].split()[0]) for line in a.autotune_report()}
+    assert "streamed stretches" in trials
+    assert abs(ms - min(trials.values())) < 1e-4  # printed to four places
+    assert all(a.status(i).stepcount == 100 for i in range(2))
+    assert a.run(100) == b.run(100) == 100
+    assert ("waited too long" in a.last_error()) == (trials["streamed stretches"] <= ms + 1e-4)
+    assert not b.last_error()
+    for i in range(2):
+        assert all(np.array_equal(x, y) for x, y in zip(a.download(i), b.download(i)))
