@@ -295,17 +295,11 @@ KERNEL_NAMES = {"cluster": ("k_cluster_step", "k_halo_update"), "two-kernel": ("
 PATH_IDS = {"cluster": 0, "two-kernel": 1, "tiles": 2, "node-tiles": 3, "node-pipe": 4}
 
 
-def many_steps_per_launch(model, precision):
-    """The default path takes whole calls in one cooperative launch where the
-    triangles' tables stay in L2 (the library's own line)."""
-    return model.num_tris * (160.0 if precision == "mixed" else 256.0) <= 88e6
-
-
 def timed_steps(model, info, bbar, precision, path, args, dials, local, dist, clock=None, setup=None):
     """One handle at `precision`: W warm-up steps, then K fused steps timed
     with CUDA events on the library's stream (barrier + synchronize on both
     sides, max over ranks), then the per-launch kernel times for the
-    roofline.  Returns (handle, ms of the K steps, kernel ms, path name)."""
+    roofline.  Returns (handle, ms of the K steps, kernel ms, path name, launches of the K steps)."""
     import contextlib
 
     import torch
@@ -316,11 +310,11 @@ def timed_steps(model, info, bbar, precision, path, args, dials, local, dist, cl
     g = GpuLoop(model, precision=prec, device=local)
     if setup is not None:
         setup["device_s"] = time.perf_counter() - t0
-    many = path == "auto" and many_steps_per_launch(model, precision)
     if path != "auto":
         g.set_step_path(PATH_IDS[path])
     path = {v: k for k, v in PATH_IDS.items()}[g.plan_info()["path"]]
     g.set_programmed(3, info, bbar, s.dial_factors_to_hold_at_spacing)
+    many = g.many_step_launches(args.steps)
     g.upload(model.dofs(1))
     dt, damp = s.timestep, s.damping_factor_1
     g.step_n(args.warmup, dials[:args.warmup], dt, damp)
@@ -353,7 +347,7 @@ def timed_steps(model, info, bbar, precision, path, args, dials, local, dist, cl
         path, t_tri = "many-step", ms_max / args.steps
     tri_name, node_name = KERNEL_NAMES[path]
     kernel_ms = {tri_name: t_tri} if node_name is None else {tri_name: t_tri, node_name: t_node}
-    return g, ms_max, kernel_ms, path
+    return g, ms_max, kernel_ms, path, many or launches(path, args.steps)
 
 
 def roofline(model, precision, path, workload, kernel_ms, step_ms):
@@ -378,8 +372,7 @@ def roofline(model, precision, path, workload, kernel_ms, step_ms):
 
 
 def launches(path, steps):
-    if path == "many-step":
-        return 1 + (max(0, steps - 128) + 8191) // 8192  # 128 steps, then up to 8,192
+    """Kernel launches of `steps` steps taken one by one."""
     per_step = 1 if KERNEL_NAMES[path][1] is None else 2
     return per_step * steps + (steps + 127) // 128  # + one chunk-end kernel per captured graph of 128 steps
 
@@ -423,8 +416,8 @@ def run_ours(args):
     dt, damp = s.timestep, s.damping_factor_1
     clk = ClockSampler(local)
     setup = {}
-    g, ms_max, kernel_ms, path = timed_steps(model, info, bbar, args.precision, args.path, args, dials, local, dist,
-                                             clock=clk, setup=setup)
+    g, ms_max, kernel_ms, path, n_launch = timed_steps(model, info, bbar, args.precision, args.path, args, dials, local,
+                                                       dist, clock=clk, setup=setup)
     value = T * args.steps * world / (ms_max / 1e3)
 
     # End to end through the C ABI with the state on the host every step.
@@ -457,7 +450,6 @@ def run_ours(args):
     if dist:
         dist.all_reduce(t2, op=dist.ReduceOp.MAX)
     e2e_value = T * e2e_steps * world / (float(t2.item()) / 1e3)
-    n_launch = launches(path, args.steps)
 
     line = {
         "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
@@ -481,8 +473,8 @@ def run_ours(args):
     # the FP64 run ended in.
     if args.precision == "fp64" and not args.no_mixed:
         clk_m = ClockSampler(local)
-        gm, ms_m, kernel_m, path_m = timed_steps(model, info, bbar, "mixed", args.path, args, dials, local, dist,
-                                                 clock=clk_m)
+        gm, ms_m, kernel_m, path_m, launches_m = timed_steps(model, info, bbar, "mixed", args.path, args, dials, local,
+                                                             dist, clock=clk_m)
         xm, _ = gm.download()
         x64, v64 = g.download()
         dial_last = float(dials[args.warmup + args.steps - 1])
@@ -497,7 +489,7 @@ def run_ours(args):
             "force_err_state": "the FP64 run's final state, dial factor of its last step; forces from one "
                                "undamped velocity update of each path",
             "clocks": clk_m.summary()}
-        line["gpu_launches"] = n_launch + launches(path_m, args.steps)
+        line["gpu_launches"] = n_launch + launches_m
         gm.close()
     if rank == 0 and world == 1 and not args.no_cpu:
         line["cpu_baseline"] = cpu_baseline(model, info, bbar)

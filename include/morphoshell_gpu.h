@@ -234,6 +234,9 @@ void* ms_stream(ms_handle* h);
  * until this call asks for a path by number.  All sum every node's contributions in ascending
  * triangle order, so they give the same bits. */
 ms_status ms_set_step_path(ms_handle* h, int path);
+/* Launches in which ms_step_n(h, n, ...) would run, dialling or not, when whole
+ * stretches of steps go in one launch; 0 when it runs step by step. */
+ms_status ms_many_step_launches(ms_handle* h, int n, int dialling, int* launches);
 /* Test hook: SM clocks a tile of the default path's many-step launches waits
  * for a neighbour's positions before the launch is given up (2e9, about a
  * second, unless set; 0: it is given up where a position is not there at the

@@ -28,6 +28,7 @@ GPU_SYMBOLS = [
     "ms_non_deformation_forces", "ms_impose_constraints", "ms_is_at_equilibrium", "ms_advance_dynamics",
     "ms_step_n", "ms_prepare_steps", "ms_output_quantities", "ms_device_info", "ms_stream", "ms_time_kernels",
     "ms_deformation_forces_noalloc", "ms_set_step_path", "ms_set_wait_limit", "ms_batch_set_wait_limit",
+    "ms_many_step_launches",
     "ms_plan_info", "ms_node_tile_layout", "ms_node_tile_plan",
     "ms_batch_create", "ms_batch_destroy", "ms_batch_last_error", "ms_batch_run", "ms_batch_status",
     "ms_batch_download_dofs", "ms_batch_upload_dofs", "ms_batch_set_schedule", "ms_batch_get_schedule",
@@ -171,6 +172,7 @@ def lib() -> C.CDLL:
                                                     C.c_size_t]
         L.ms_set_step_path.argtypes = [C.c_void_p, C.c_int]
         L.ms_set_wait_limit.argtypes = [C.c_void_p, C.c_int64, C.c_int]
+        L.ms_many_step_launches.argtypes = [C.c_void_p, C.c_int, C.c_int, P(C.c_int)]
         L.ms_batch_set_wait_limit.argtypes = [C.c_void_p, C.c_int64]
         ip = C.POINTER(C.c_int)
         L.ms_plan_info.argtypes = [C.c_void_p, ip, ip, ip, ip, ip]
@@ -464,6 +466,12 @@ class GpuLoop:
         compute triangles while a third sums and updates nodes; the default
         on meshes with a node tile for every SM)."""
         self._chk(lib().ms_set_step_path(self._h, path), "set_step_path")
+
+    def many_step_launches(self, n: int, dialling: bool = True) -> int:
+        """Launches of whole stretches in which step_n(n) would run; 0: step by step."""
+        k = C.c_int()
+        self._chk(lib().ms_many_step_launches(self._h, n, int(dialling), C.byref(k)), "many_step_launches")
+        return k.value
 
     def set_wait_limit(self, clocks: int, from_launch: int = 0):
         """Test hook: how long a tile of a many-step launch waits for its

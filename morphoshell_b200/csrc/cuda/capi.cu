@@ -1216,6 +1216,20 @@ static bool use_resident(const ms_handle* h, int n, bool dialling, bool fuse_lce
     return dialling ? fuse_lce && h->plan.tri_aux && h->plan.lce_uniform : true;
 }
 
+// Steps of the k-th launch (from 0) of a call, `left` steps from its end.
+static int launch_steps(int k, int left, bool dialling) {
+    const int len = std::min(dialling && k == 0 ? kResidentFirst : kResidentSteps, left);
+    return left - len < kResidentFirst ? left : len;
+}
+
+ms_status ms_many_step_launches(ms_handle* h, int n, int dialling, int* launches) {
+    if (!h || n < 0 || !launches) return MS_ERR_INVALID_ARGUMENT;
+    *launches = 0;
+    if (!use_resident(h, n, dialling != 0, dialling && lce_fusable(h))) return MS_OK;
+    for (int at = 0; at < n; ++*launches) at += launch_steps(*launches, n - at, dialling != 0);
+    return MS_OK;
+}
+
 ms_status ms_set_wait_limit(ms_handle* h, int64_t clocks, int from_launch) {
     if (!h || clocks < 0 || from_launch < 0) return MS_ERR_INVALID_ARGUMENT;
     h->wait = clocks;
@@ -1234,8 +1248,7 @@ static ms_status run_resident(ms_handle* h, int n, const double* dials, int dial
     const int p0 = h->cur;
     std::vector<int> starts;
     for (int at = 0, k = 0; at < n; ++k) {
-        int len = std::min(dials && k == 0 ? kResidentFirst : kResidentSteps, n - at);
-        if (n - at - len < kResidentFirst) len = n - at;
+        const int len = launch_steps(k, n - at, dials != nullptr);
         if (dials) MS_TRY(fill_dials(h, dials, at, at + len));
         starts.push_back(at);
         const bool last = at + len == n;

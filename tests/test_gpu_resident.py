@@ -306,3 +306,19 @@ def test_varied_materials_keep_the_node_tiled_plan(workdir, tmp_path, precision)
         g.do_dialling(0.3)
         g.step_n(40, None, s.timestep, s.damping_factor_2)
     assert _same(ga, gb)
+
+
+@pytest.mark.parametrize("name,precision,first", [("disk100", 0, 128), ("disk18k", 1, 128), ("disk5", 0, 128),
+                                                  ("disk4", 0, 0), ("disk4", 1, 128)])
+def test_many_step_launches(workdir, name, precision, first):
+    """The library's own answer whether and in how many launches whole
+    stretches run: none on meshes too large for them, with a path by number,
+    or for single steps."""
+    g = _pair(make_model(workdir, name), precision)[0]
+    assert g.many_step_launches(1) == 0
+    for n, launches in [(2, 1), (128, 1), (255, 1), (256, 2), (128 + 8192, 2), (128 + 8192 + 128, 3)]:
+        assert g.many_step_launches(n) == (launches if first else 0)
+    assert g.many_step_launches(8192 + 127, dialling=False) == (1 if first else 0)
+    assert g.many_step_launches(8192 + 128, dialling=False) == (2 if first else 0)
+    g.set_step_path(2)
+    assert g.many_step_launches(1000) == 0
