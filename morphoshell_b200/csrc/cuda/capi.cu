@@ -292,6 +292,19 @@ constexpr int kNtNodesMin = 256;
 #define MSB_PIPE_NODES 1600
 #endif
 
+// Equilibrium partials for n blocks.
+ms_status room_for_partials(ms_handle* h, int n) {
+    if (n <= h->s.eq_blocks) return MS_OK;
+    EqPartial* ep;
+    MS_TRY(dalloc(h, &ep, n));
+    h->s.eq_part = ep;
+    h->s.eq_blocks = n;
+    return MS_OK;
+}
+
+bool stream_range(const ms_handle* h, int N, int T);
+ms_status build_streamed(ms_handle* h, const StreamLayout& S);
+
 // Plan of the node-tiled step: the chunk records, area in the trigonometry
 // block (cos^2 = 1, the rest 0) until prepare_lce_tables writes the
 // director's values.  A block walks its tiles in turn, so the step takes as
@@ -299,10 +312,6 @@ constexpr int kNtNodesMin = 256;
 // tile count is a multiple of the resident blocks (SMs x blocks per SM), at
 // the largest size that keeps those blocks resident.  Leaves the other paths
 // in place when the kernel cannot be set up.
-// (forward: the streamed step's part of that plan)
-bool stream_range(const ms_handle* h, int N, int T);
-ms_status build_streamed(ms_handle* h, const StreamLayout& S);
-
 ms_status build_node_tiles(ms_handle* h, const ms_mesh_desc* d, const std::vector<int>& off,
                            const std::vector<int>& ent) {
     const int mixed = h->precision == MS_PRECISION_MIXED;
@@ -411,13 +420,7 @@ ms_status build_node_tiles(ms_handle* h, const ms_mesh_desc* d, const std::vecto
     q.chunk_tag = nullptr;
     h->d_nt_rec = d_rec;
     // One equilibrium partial per block.
-    const int parts = std::min(K, std::max(q.grid, q.grid_pipe));
-    if (parts > h->s.eq_blocks) {
-        EqPartial* ep;
-        MS_TRY(dalloc(h, &ep, parts));
-        h->s.eq_part = ep;
-        h->s.eq_blocks = parts;
-    }
+    MS_TRY(room_for_partials(h, std::min(K, std::max(q.grid, q.grid_pipe))));
     h->have_ntiles = q.grid > 0;
     h->have_pipe = q.grid_pipe > 0;
     if (stream) MS_TRY(build_streamed(h, S));
@@ -446,16 +449,6 @@ ms_status make_packets(ms_handle* h, ulonglong2** p) {
     const size_t n = 6ULL * h->m.N;
     MS_TRY(dalloc(h, p, n));
     MS_CUDA(h, cudaMemsetAsync(*p, 0, n * sizeof(ulonglong2), h->stream));
-    return MS_OK;
-}
-
-// Equilibrium partials for n blocks.
-ms_status room_for_partials(ms_handle* h, int n) {
-    if (n <= h->s.eq_blocks) return MS_OK;
-    EqPartial* ep;
-    MS_TRY(dalloc(h, &ep, n));
-    h->s.eq_part = ep;
-    h->s.eq_blocks = n;
     return MS_OK;
 }
 
@@ -613,13 +606,7 @@ ms_status build_cluster_plan(ms_handle* h, const ms_mesh_desc* d, const std::vec
     p.n_halo = (int)halo_nodes.size();
     // Equilibrium partials: one per cluster-kernel CTA plus one per halo block.
     h->halo_parts = p.n_halo > 0 ? (p.n_halo + 255) / 256 : 1;
-    const int parts = p.nclusters * p.cs + h->halo_parts;
-    if (parts > h->s.eq_blocks) {
-        EqPartial* ep;
-        MS_TRY(dalloc(h, &ep, parts));
-        h->s.eq_part = ep;
-        h->s.eq_blocks = parts;
-    }
+    MS_TRY(room_for_partials(h, p.nclusters * p.cs + h->halo_parts));
     h->have_plan = true;
     MS_TRY(build_tiles(h, d));
     MS_TRY(build_resident(h, d, off, ent));

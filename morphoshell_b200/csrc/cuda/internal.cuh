@@ -290,7 +290,6 @@ struct StreamLayout {
     std::vector<unsigned> local;
     std::vector<unsigned char> border;
 };
-struct NodeTileLayout;
 void stream_layout(const NodeTileLayout& L, const int* patch_ids, int N, int NT, StreamLayout& S);
 
 // Layout of the per-(triangle, slot) force contributions: x, y, z doubles;
@@ -470,8 +469,8 @@ cudaError_t launch_batch_streamed(const DevMesh& m, const NodeTilePlan& q, const
 // node-tiled step in graphs: FP64 268,146 triangles (69 MB) 24.8 (23.7) against
 // 26.9 (26.6), 342,658 (88 MB) 30.4 (28.9) against 32.7 (32.6), but 374,412
 // (96 MB) 42.0 against 33.7; mixed 342,658 (55 MB) 22.6 against 28.6, 411,150
-// (66 MB) 29.6 (30.6) against 31.2 (32.4); the mixed blocks of larger meshes do
-// not fit.
+// (66 MB) 29.6 (30.6) against 31.2 (32.4), 476,735 (76 MB) 34.4 (35.7) against
+// 36.0 (37.2); the mixed blocks of meshes of 500,000 and more do not fit.
 constexpr double kStreamBytes = 88e6;
 constexpr double stream_bytes(int mixed, double tris) { return (mixed ? 160.0 : 256.0) * tris; }
 // Largest cluster size (8, 4, 2, 1) whose clusters fill the most SMs, and the
