@@ -128,7 +128,10 @@ ms_status ms_set_zero_dial_state(ms_handle* h, const double* a0 /*3T or NULL*/, 
 ms_status ms_do_dialling(ms_handle* h, double dial_factor);
 ms_status ms_download_programmed(ms_handle* h, double* abar /*3T*/, double* bbar /*3T*/);
 
-/* ---- the reference's per-step sequence, one call each ------------------ */
+/* ---- the reference's per-step sequence, one call each ------------------
+ * Calls that return no values (ms_do_dialling among them) are in order on the
+ * handle's stream and do not wait for the device; a CUDA error of theirs shows
+ * at the next call that does. */
 /* calc_surface_derivs.cpp:27-34: cq = D * dofs.  cq may be NULL (kept on device). */
 ms_status ms_surface_derivs(ms_handle* h, double* cq /*15T or NULL*/);
 /* calc_a_comps_and_b_comps_and_normals.cpp:27-62, from the last cq. */
@@ -179,7 +182,8 @@ ms_status ms_deformation_forces_noalloc(int32_t num_nodes, int32_t num_tris, con
 /* ---- fused stepper: the whole main.cpp:308-488 body per step ----------
  * Runs n steps of: surface derivs -> (dialling) -> deformation forces ->
  * damping -> constraints -> (equilibrium check on the last step if
- * check_last) -> force guard -> symplectic Euler, as one kernel per step on
+ * check_last) -> force guard -> symplectic Euler: whole stretches of steps in
+ * one launch where ms_many_step_launches says so, else one kernel per step on
  * the node-tiled path (two on the others, ms_set_step_path) captured in CUDA
  * graphs.  Fused protocol-3 steps dial inside the force kernel; the abar and
  * bbar arrays are brought to the last step's dial factor only when a later
@@ -194,7 +198,8 @@ ms_status ms_step_n(ms_handle* h, int n, const double* dial_factors, int diallin
 /* Builds (captures and instantiates) the CUDA graphs that ms_step_n with
  * the same n, dialling, timestep, damping, gradient-descent and check_last
  * arguments would use from the current state buffer, launching nothing, so
- * that the first such call does not pay for them.  No reference counterpart
+ * that the first such call does not pay for them; nothing is to be built where
+ * ms_many_step_launches is not 0.  No reference counterpart
  * (it only moves set-up work out of the timed loop). */
 ms_status ms_prepare_steps(ms_handle* h, int n, int dialling, double timestep, double damping_factor,
                            int using_gradient_descent, int check_last);
@@ -226,12 +231,13 @@ void* ms_stream(ms_handle* h);
  * step -- one kernel: each block takes tiles of consecutive nodes, computes
  * every triangle that touches the tile (border triangles once per tile),
  * sums the tile's forces in shared memory and updates its nodes, so no
- * contribution goes through HBM.  The default is 3 on meshes with at least
- * one node tile per resident block, else 2; on meshes small enough for one
- * thread per triangle (about 35,000 on B200), and on mid-size ones whose tables
- * stay in L2 (about 230,000 triangles, 370,000 mixed), the default runs whole
- * calls of ms_step_n in one cooperative launch each (resident.cu, streamed.cu),
- * until this call asks for a path by number.  All sum every node's contributions in ascending
+ * contribution goes through HBM.  The default is 3 on meshes with a node tile
+ * for nine tenths of the resident blocks or more, else 2.  On meshes of one
+ * material that are small enough for one thread per triangle (about 35,000 on
+ * B200), and on mid-size ones whose tables stay in L2 and whose tiles fit
+ * (about 343,000 triangles, 477,000 mixed), the default runs whole calls of
+ * ms_step_n in a cooperative launch (resident.cu, streamed.cu), until this call
+ * asks for a path by number.  All sum every node's contributions in ascending
  * triangle order, so they give the same bits. */
 ms_status ms_set_step_path(ms_handle* h, int path);
 /* Launches in which ms_step_n(h, n, ...) would run, dialling or not, when whole
