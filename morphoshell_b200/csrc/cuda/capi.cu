@@ -1258,11 +1258,12 @@ static ms_status run_resident(ms_handle* h, int n, const double* dials, int dial
         const int step = (int)(h->h_err->guard_key >> 32);
         while (launches > 1 && starts[launches - 1] > step) --launches;
         *done = starts[--launches];
-        if (h->h_err->flag == MS_ERR_TIMEOUT) {
-            // Some blocks of a check step may have counted themselves.
-            MS_CUDA(h, cudaMemsetAsync(h->s.eq_counter, 0, sizeof(unsigned int), st));
+        // Of a check step's blocks some may have counted themselves and others,
+        // whose wait ran out, not (whatever the flag says: a trip in the same
+        // launch takes it over).
+        MS_CUDA(h, cudaMemsetAsync(h->s.eq_counter, 0, sizeof(unsigned int), st));
+        if (h->h_err->flag == MS_ERR_TIMEOUT)
             h->last_error = "a tile waited too long for its neighbours' positions: a launch's steps ran one by one";
-        }
     }
     h->cur = p0 ^ (launches & 1);
     return MS_OK;

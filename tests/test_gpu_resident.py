@@ -322,3 +322,56 @@ def test_many_step_launches(workdir, name, precision, first):
     assert g.many_step_launches(8192 + 128, dialling=False) == (2 if first else 0)
     g.set_step_path(2)
     assert g.many_step_launches(1000) == 0
+
+
+def _without_neighbours(m, first):
+    """The model with its first nodes cut off from the rest: triangles on both
+    stand for another triangle once more, with no area."""
+    import ctypes as C
+    import types
+    t = m.tables()
+    ids, w, area = (t[k].copy() for k in ("patch_ids", "deriv_coeffs", "ref_area"))
+    ids = ids.astype(np.int32)
+    both = ((ids < first).any(1)) & ((ids >= first).any(1))
+    other = np.flatnonzero((ids >= first).all(1))[0]
+    ids[both], w[both], area[both] = ids[other], w[other], 0.0
+    desc = type(m.desc)()
+    C.memmove(C.byref(desc), C.byref(m.desc), C.sizeof(desc))
+    desc.patch_ids = ids.ctypes.data_as(C.POINTER(C.c_int32))
+    desc.deriv_coeffs = w.ctypes.data_as(C.POINTER(C.c_double))
+    desc.ref_area = area.ctypes.data_as(C.POINTER(C.c_double))
+    return types.SimpleNamespace(desc=desc, params=m.params, scalars=m.scalars, num_nodes=m.num_nodes,
+                                 num_tris=m.num_tris, programmed=m.programmed, dofs=m.dofs, keep=(ids, w, area))
+
+
+# Nodes cut off: as many as a tile of the mesh without them as neighbours has.
+# The meshes have under 256 nodes, so that the check by itself is one block.
+@pytest.mark.parametrize("name,first", [("disk125", 32), ("disk135", 37), ("disk145", 36)])
+def test_guard_and_wait_in_one_launch(workdir, name, first):
+    """A launch in which a node trips the guard, the waits of tiles run out and
+    the first, which waits for nobody, reaches the check on its last step:
+    reported as the two-kernel step reports it, and the checks after it are of
+    the state then."""
+    from morphoshell_b200 import MsError
+    m = _without_neighbours(make_model(workdir, name), first)
+    s = m.scalars
+    x, v = deformed_state(m, seed=47, amp=0.02)
+    bad = x.copy()
+    bad[-3] += 1e6
+    out = []
+    for g in _pair(m):
+        got = []
+        for k in range(3):
+            g.upload(x, (1.0 + k) * v)
+            got.append(_equil(g.step_n(3, None, s.timestep, s.damping_factor_2, check_last=True)))
+            g.upload(bad, v)
+            g.set_wait_limit(0)
+            with pytest.raises(MsError) as ei:
+                g.step_n(2, None, s.timestep, s.damping_factor_2, check_last=True)
+            r = ei.value.report
+            got.append((r.error_step, r.offending_dof, r.offending_force, r.steps_done))
+            g.set_wait_limit(2_000_000_000)
+            e = g.is_at_equilibrium()
+            got.append((e.max_force, e.max_speed, e.max_force_node, e.max_speed_node))
+        out.append(got)
+    assert out[0] == out[1]
